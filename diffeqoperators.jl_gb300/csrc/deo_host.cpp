@@ -2393,7 +2393,8 @@ extern "C" deo_status deo_batch_create(int n, const deo_instance* in, int adjoin
         CUDA_TRY(cudaMemcpy(b->d_inst, b->inst.data(), n * sizeof(deo::InstDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(instances)");
     }
-    CUDA_TRY(cudaMalloc(&b->d_counter, sizeof(unsigned int)), "cudaMalloc(counter)");
+    CUDA_TRY(cudaMalloc(&b->d_counter, 2 * sizeof(unsigned int)), "cudaMalloc(counters)");
+    CUDA_TRY(cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned int)), "cudaMemset(counters)");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
@@ -2446,7 +2447,8 @@ extern "C" deo_status deo_stage_batch_create(int n, const deo_stage* in, int til
         CUDA_TRY(cudaMemcpy(b->d_stages, b->stages.data(), n * sizeof(deo::StageDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(stages)");
     }
-    CUDA_TRY(cudaMalloc(&b->d_counter, sizeof(unsigned int)), "cudaMalloc(counter)");
+    CUDA_TRY(cudaMalloc(&b->d_counter, 2 * sizeof(unsigned int)), "cudaMalloc(counters)");
+    CUDA_TRY(cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned int)), "cudaMemset(counters)");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
