@@ -20,6 +20,7 @@ SOURCES = {
     "deo_kernels.o": ("nvcc", "deo_kernels.cu"),
     "deo_tma.o": ("nvcc", "deo_tma.cu"),
     "deo_vec.o": ("nvcc", "deo_vec.cu"),
+    "deo_march.o": ("nvcc", "deo_march.cu"),
     "deo_concretize.o": ("nvcc", "deo_concretize.cu"),
     "deo_shell.o": ("nvcc", "deo_shell.cu"),
     "deo_static.o": ("nvcc", "deo_static.cu"),
@@ -49,7 +50,7 @@ def _stale(obj: str, src: str) -> bool:
         return True
     deps = [src, os.path.join(CSRC, "deo_internal.h"), os.path.join(CSRC, "deo_eval.cuh"),
             os.path.join(CSRC, "deo_rows.cuh"), os.path.join(CSRC, "deo_ptx.cuh"), os.path.join(CSRC, "deo_fx.cuh"),
-            os.path.join(CSRC, "deo_bfx.cuh"), os.path.join(CSRC, "deo_lap.cuh"),
+            os.path.join(CSRC, "deo_bfx.cuh"), os.path.join(CSRC, "deo_bfp.cuh"), os.path.join(CSRC, "deo_lap.cuh"),
             os.path.join(HERE, "..", "include", "deo.h"),
             os.path.abspath(__file__)]
     t = os.path.getmtime(obj)

@@ -813,6 +813,8 @@ constexpr int kFxFp64Rows = 2;
 struct deo_plan {
     PlanDev dev{};
     deo::UniPlan uni{};
+    deo::BfpMarch march{};      // 3-D Float64: the marching block fixed-point interior (ok = 0: not this plan)
+    int fx_rows_set = 0;        // DEO_OPT_FX_FP64_ROWS was set: the caller wants the per-point kernel's rows
     deo::ShellPlan shell{};
     int fast_path = 1;   // DEO_OPT_FAST_PATH
     int use_tma = 1;     // DEO_OPT_TMA
@@ -1063,6 +1065,50 @@ static bool bfx_weights(const double* w, int H, deo::UniPlan& U) {
     U.bfx_cneg = cneg ? 1 : 0;
     U.bfx_f = fmin;
     U.bfx_tshift = 53 + G0 - 1 - Tc;
+    return true;
+}
+
+// The weights of the marching block fixed-point interior (deo_march.cu) for the
+// band w[a][0..2H] of each axis: W = round(w * 2^s) with the sum of |W| below
+// 2^60, split at bit 30, and the acceptance thresholds: a point is within 2 ulp
+// of its sum |w u| when that sum is at least 1.05 * 2^52 units times the sum of
+// |W|, which one tap alone shows when its high limb (2^30 units, half a unit of
+// rounding) reaches that over its own |W|.
+static void split_limbs(long long W, int& h, int& l) {
+    h = (int)((W + (1LL << 29)) >> 30);
+    l = (int)(W - ((long long)h << 30));
+}
+static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
+    const int K = 2 * H + 1;
+    double sum = 0.0;
+    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < K; ++k) {
+            if (!std::isfinite(w[a][k])) return false;
+            sum += std::fabs(w[a][k]);
+        }
+    if (!(sum > 0.0) || std::fpclassify(sum) != FP_NORMAL) return false;
+    const int s = 59 - std::ilogb(sum) - 1;  // (one bit for the sum's own rounding)
+    long long c0 = 0;
+    double total = 0.0;
+    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < K; ++k) {
+            const long long W = std::llrint(std::ldexp(w[a][k], s));
+            total += std::fabs((double)W);
+            if (k == H) c0 += W;
+            split_limbs(W, B.wh[a][k], B.wl[a][k]);
+        }
+    split_limbs(c0, B.c0h, B.c0l);
+    B.shared = std::memcmp(w[0], w[1], K * sizeof(double)) == 0 && std::memcmp(w[0], w[2], K * sizeof(double)) == 0;
+    auto threshold = [&](double W, double slack) {
+        const double t = std::fabs(W) > 0.0 ? std::ldexp(1.05 * total / std::fabs(W), 22) + slack : 4e9;
+        return t < 2147483647.0 ? (int)std::ceil(t) : INT_MAX;
+    };
+    auto limb = [&](int a, int k) { return (double)(((long long)B.wh[a][k] << 30) + B.wl[a][k]); };
+    B.t0 = threshold((double)c0, 1.0);
+    const int t1 = threshold(limb(0, H + 1), 2.0);
+    B.sh1 = 0;
+    while (B.sh1 < 31 && ((long long)B.t0 << B.sh1) < t1) ++B.sh1;  // |n1| >> sh1 >= t0 implies |n1| >= t1
+    B.kbase = 57 - s - 1075 - 6;
     return true;
 }
 
@@ -1388,6 +1434,14 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
                 U.bfx = std::memcmp(U.t[t].w, U.t[0].w, sizeof(double) * (2 * H + 1)) == 0;
             if (U.bfx) U.bfx = bfx_weights(U.t[0].w, H, U);
             for (int k = 0; k < 3; ++k) U.n[k] = k < ndims ? sizes[k] : 1;
+            if (U.lap && dtype == DEO_F64 && D.nterms == 3 && H <= 3 && (int64_t)sizes[0] * sizes[1] < (1LL << 28)) {
+                const double* const w[3] = {U.t[0].w, U.t[1].w, U.t[2].w};
+                P->march.ok = march_weights(w, H, P->march) ? 1 : 0;
+                for (int a = 0; a < 3; ++a) {
+                    P->march.lo[a] = U.t[a].flo - 1;
+                    P->march.hi[a] = U.t[a].fhi - 1;
+                }
+            }
         } else {
             U.enabled = 0;
         }
@@ -1457,9 +1511,63 @@ static void mark(const deo_plan* p, int k, void* stream) {
 // a device counter (zeroed on the stream before each launch), so they balance
 // around the shell's CTAs.  Launch timing with a concurrent shell: ms[0] =
 // fork to the end of the interior kernel, ms[1] = the wait for the shell after it.
+//
+// 3-D Float64 plans take the marching block fixed-point interior
+// (deo_march.cu) by default, whatever the alignment; the options that ask for
+// another variant, the FP64 rows of the per-point kernel or the TMA kernels'
+// wait test keep theirs.
+static bool use_march(const deo_plan* p) {
+    return p->march.ok && p->exact_sums == 1 && p->fast_path && p->use_tma && !p->fx_rows_set &&
+           !p->uni.test_withhold;
+}
+static unsigned int* next_sched(const deo_plan* p) {
+    return p->d_sched ? p->d_sched + (p->sched_slot.fetch_add(1) % kSchedSlots) : nullptr;
+}
+
+// The interior first, then the shell with its full grid, which fills the SMs as
+// the interior's CTAs leave them (the face kernel where TMA can read the array,
+// else one thread per point): 188 us at 256^3, against 213 with the line
+// kernel, 231-256 with the face kernel's one-CTA-per-SM form and 220 with the
+// shell after the interior (interior alone 164, shell alone 55).
+static int launch_march(const deo_plan* p, const void* u, void* du, int overwrite, void* stream) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    deo::UniPlan us = p->uni;
+    if (us.shell_kernel == 0) us.shell_kernel = 1;
+    const bool conc = p->concurrent && p->side && p->d_shell;
+    const deo::ShellPlan* sp = p->d_shell ? &p->shell : nullptr;
+    const char* k2 = "";
+    std::unique_lock<std::mutex> lk(p->apply_mu, std::defer_lock);
+    if (conc) {
+        lk.lock();
+        const cudaError_t c = cudaEventRecord(p->ev_fork, st);
+        if (c != cudaSuccess) return (int)c;
+    }
+    int e = deo_k_apply_march(&p->uni, &p->march, next_sched(p), u, du, overwrite, stream);
+    if (e) return e;
+    mark(p, 1, stream);
+    if (conc) {
+        const cudaError_t c = cudaStreamWaitEvent(p->side, p->ev_fork, 0);
+        if (c != cudaSuccess) return (int)c;
+    }
+    e = deo_k_apply_shell(&us, sp, p->d_shell, DEO_SHELL_ALONE, p->d_plan, p->dev.dtype, u, du, overwrite,
+                          conc ? static_cast<void*>(p->side) : stream, &k2);
+    if (e) return e;
+    if (conc) {
+        cudaError_t c = cudaEventRecord(p->ev_join, p->side);
+        if (c == cudaSuccess) c = cudaStreamWaitEvent(st, p->ev_join, 0);
+        if (c != cudaSuccess) return (int)c;
+    }
+    p->last_kernel = "k_lap_fx";
+    p->last_kernel2 = k2;
+    p->ev_launches = 2;
+    mark(p, 2, stream);
+    return 0;
+}
+
 static int launch_forward(const deo_plan* p, const void* u, void* du, int overwrite, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     mark(p, 0, stream);
+    if (use_march(p)) return launch_march(p, u, du, overwrite, stream);
     if (p->uni.enabled && p->fast_path) {
         if (p->uni.lap && p->use_tma && deo_k_tma_ok(&p->uni, p->dev.dtype, u)) {
             // overlap only pays beside an interior kernel that leaves the FP64 pipe free: the fixed-point
@@ -1473,7 +1581,7 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
             const char* k = "";
             const char* k2 = "";
             // a counter of its own for this launch (applies of one plan may run on several streams at once)
-            unsigned int* sched = p->d_sched ? p->d_sched + (p->sched_slot.fetch_add(1) % kSchedSlots) : nullptr;
+            unsigned int* sched = next_sched(p);
             if (conc) {
                 // the interior first, on the caller's stream: its persistent grid takes its CTAs' places
                 // on every SM at once; then the shell on the side stream, whose CTAs fill the place left
@@ -1535,6 +1643,7 @@ extern "C" deo_status deo_plan_set_option(deo_plan* p, int option, int value) {
         case DEO_OPT_FX_FP64_ROWS:
             if (value < 0 || value > 8) return fail(DEO_ERR_BAD_ARG, "FP64 rows %d not in 0..8", value);
             p->uni.fx_rows = value;
+            p->fx_rows_set = 1;
             return DEO_OK;
         case DEO_OPT_F32_VECTOR: p->uni.f32_vec = value ? 1 : 0; return DEO_OK;
         case DEO_OPT_F32_TILE:
@@ -1576,7 +1685,7 @@ extern "C" int deo_plan_get_option(const deo_plan* p, int option) {
             return (p->dev.dtype == DEO_F64 && p->uni.enabled && p->uni.lap &&
                     (p->exact_sums == 1 || p->exact_sums == 4 || (p->exact_sums == 5 && !p->uni.bfx)) &&
                     p->uni.fx &&
-                    p->uni.radius <= 3)
+                    p->uni.radius <= 3 && !use_march(p))
                        ? p->uni.fx_rows
                        : 0;
         case DEO_OPT_CONCURRENT_SHELL:
@@ -1637,6 +1746,26 @@ static void reverse_taps(E* w, int n) {
 }
 
 static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwrite, void* stream) {
+    if (p->adj_ok && use_march(p)) {
+        deo::UniPlan ua = p->uni;
+        deo::BfpMarch B = p->march;
+        const int K = 2 * ua.radius + 1;
+        for (int a = 0; a < 3; ++a) {
+            ua.t[a].flo = p->adj_lo[a];
+            ua.t[a].fhi = p->adj_hi[a];
+            B.lo[a] = p->adj_lo[a] - 1;
+            B.hi[a] = p->adj_hi[a] - 1;
+            reverse_taps(ua.t[a].w, K);
+            reverse_taps(B.wh[a], K);
+            reverse_taps(B.wl[a], K);
+        }
+        int e = deo_k_apply_march(&ua, &B, next_sched(p), d, ub, overwrite, stream);
+        if (!e) e = deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, stream);
+        if (e) return e;
+        p->last_kernel = "k_lap_fx";
+        p->last_kernel2 = "k_shell_adj";
+        return 0;
+    }
     if (p->adj_ok && p->uni.enabled && p->uni.lap && p->fast_path && p->use_tma &&
         deo_k_tma_ok(&p->uni, p->dev.dtype, d)) {
         deo::UniPlan ua = p->uni;

@@ -169,6 +169,20 @@ struct UniPlan {
     int shell_kernel;
 };
 
+// Weights of a 3-D Laplacian-type plan for the block fixed-point interior
+// (deo_bfp.cuh, deo_march.cu): W = round(w * 2^s) = wh * 2^30 + wl, |wl| <= 2^29,
+// with the sum of |W| over all taps below 2^60.  [k] is the offset k - H; c0 the
+// centre weights of the three axes added.
+struct BfpMarch {
+    int ok;
+    int shared;           // the three axes share one band: neighbours are added before the product
+    int lo[3], hi[3];     // interior box, 0-based inclusive
+    int c0h, c0l;
+    int wh[3][9], wl[3][9];
+    int t0, sh1;          // a point is accepted when its centre's high limb, or its +1 neighbours' >> sh1, reaches t0
+    int kbase;            // the sum in units of 2^57 times 2^(kbase + E) is the result
+};
+
 // Boundary rows of the terms of a Laplacian-type plan (the rows outside each
 // term's interior range [flo, fhi]) with their weights and ghost maps; the
 // plan keeps a device copy that the boundary-shell kernel stages into shared
@@ -331,6 +345,9 @@ extern "C" int deo_k_apply_shell_adj(const deo::UniPlan* up, const deo::PlanDev*
 // plan or the buffers do not fit it (the caller then runs k_lap_q)
 extern "C" int deo_k_apply_vec(const deo::UniPlan* up, unsigned int* sched, const void* u, void* du, int ow,
                                void* stream);
+// Float64 interior in block fixed point, marching along axis 3 (deo_march.cu)
+extern "C" int deo_k_apply_march(const deo::UniPlan* up, const deo::BfpMarch* B, unsigned int* sched, const void* u,
+                                 void* du, int overwrite, void* stream);
 extern "C" int deo_k_read_vec_status(unsigned int* status);
 // Device concretisation from the plan's tables (deo_concretize.cu): mode 0
 // dense, 1 banded (l, u; *flag set for an entry outside), 2 bandwidths into lu

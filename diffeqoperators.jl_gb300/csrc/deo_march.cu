@@ -1,0 +1,372 @@
+// deo_march.cu -- Float64 interior of a 3-D Laplacian-type plan in block fixed
+// point (deo_bfp.cuh), marching along axis 3.
+//
+// CTA = 32 x TYT threads over a 64 x TYT*RY tile; a thread owns 2 consecutive x
+// points on RY rows and marches through a chunk of planes.  Each plane of the
+// tile plus its halo is loaded to registers two planes ahead (plain 8-byte
+// loads, so any size and alignment; a halo position outside the array reads the
+// nearest value inside, which no evaluated point uses), its largest exponent
+// found on the way (one plane ahead), converted once to limbs on the block's
+// exponent and put in a shared-memory ring of 2H + 2 planes, from which every
+// tap is read, two points to a 16-byte load.  One barrier per plane: a slot is
+// rewritten only after a barrier that follows its last reader.  When a plane
+// exceeds the block's exponent, or the planes in use have all fallen two below
+// it, the resident planes are converted again from global memory (rare, and
+// uniform over the CTA).
+//
+// A point whose error bound fails (BfpMarch::t0) is queued by its warp and
+// evaluated in the reference's order, from global memory, 32 at a time at the
+// end of the unit (draining as the queue passed 32 held every other warp at the
+// plane's barrier: 8 us more at 256^3).  A plane with Inf/NaN, or with an exponent
+// outside the range the scaled result needs, sends all its points there.
+//
+// What bounds it (256^3, d2 a4, smooth field; start: the per-point fixed point,
+// 270 us beside its shell): 164 us for the interior, 139 us of them without the 2.8 %
+// of points in the reference's order.  139 instructions per point -- 20 32 x 32 ->
+// 64-bit multiply-adds, about 35 to load and convert 1.6 values (halo and fill
+// planes included), 16 to add neighbours and test, 12 to round -- at 45-59 % issue:
+// with 12-24 warps per SM the multiply-add chains and the per-plane barrier show.
+// Tiles of 64 x 16 with 4, 2 or 1 rows a thread (128, 256, 512 threads) measured
+// 172-210 us, this 64 x 8 with 2 rows 164; a second rounding in integer arithmetic
+// instead of the conversion and scale costs 17 us more.
+#include <cuda_runtime.h>
+#include <limits.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "deo_bfp.cuh"
+#include "deo_eval.cuh"
+#include "deo_lap.cuh"
+
+namespace deo {
+namespace march {
+
+template <int H, int TYT, int RY>
+struct Cfg {
+    static constexpr int TXT = 32, NTHR = TXT * TYT;
+    static constexpr int TX = 64, TY = TYT * RY;
+    static constexpr int HP = (H + 1) / 2 * 2;  // x halo in whole pairs (16-byte shared loads)
+    static constexpr int BX = TX + 2 * HP, BY = TY + 2 * H;
+    static constexpr int PLANE = BX * BY;
+    static constexpr int NLD = (PLANE + NTHR - 1) / NTHR;  // values a thread loads per plane
+    static constexpr int SLOTS = 2 * H + 2;
+    static constexpr int QCAP = 1024 / TYT * 4;  // fallback points a warp can hold (>= 2 * 64 * RY)
+    static constexpr int SLOT = PLANE;
+    static constexpr int SMEM = SLOTS * SLOT * 8 + TYT * QCAP * 2;
+    static_assert(RY <= 4 && QCAP >= 2 * 64 * RY, "a queued point is 8 bits of plane, 2 of row, 6 of x");
+};
+
+// One point in the reference's order, from global memory.
+template <int H>
+__device__ __forceinline__ double ref_point(const UniPlan& U, const double* __restrict__ u, int64_t idx, int64_t nx,
+                                            int64_t sxy) {
+    const int64_t st[3] = {1, nx, sxy};
+    double total = 0.0;
+#pragma unroll
+    for (int t = 0; t < 3; ++t) {
+        double acc = 0.0;
+#pragma unroll
+        for (int k = 0; k < 2 * H + 1; ++k) acc = fma(U.t[t].w[k], u[idx + (k - H) * st[t]], acc);
+        total = t == 0 ? acc : total + acc;
+    }
+    return zero_fix(total);
+}
+
+template <int H, bool SH, bool OW, int TYT, int RY>
+__global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __grid_constant__ UniPlan U,
+                                                             const __grid_constant__ BfpMarch B, const LapGrid g,
+                                                             const double* __restrict__ u, double* __restrict__ du, int pairs) {
+    using C = Cfg<H, TYT, RY>;
+    constexpr int NQ = 2 * H + 1, HL = C::HP / 2, S = C::SLOTS;
+    extern __shared__ __align__(16) unsigned char smem[];
+    Limbs* ring = reinterpret_cast<Limbs*>(smem);
+    unsigned short* queue = reinterpret_cast<unsigned short*>(smem + S * C::SLOT * 8) + threadIdx.y * C::QCAP;
+    __shared__ unsigned s_max[16], s_min[16];  // of plane p at p & 15
+    __shared__ int s_next;
+    const int nx = (int)U.n[0], ny = (int)U.n[1];
+    const int64_t sxy = (int64_t)nx * ny;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+    const int own = (ty * RY + H) * C::BX + C::HP + 2 * tx;  // the first own row's pair inside a slot
+    int nq = 0;                                              // this warp's queued points
+
+    auto drain = [&](int keep, int x0, int y0, int z0) {
+        while (nq > keep) {
+            const int n = min(nq, 32);
+            nq -= n;
+            if (tx < n) {
+                const unsigned e = queue[nq + tx];
+                const int64_t idx = (int64_t)(z0 + (int)(e >> 8)) * sxy +
+                                    (int64_t)(y0 + ty * RY + (int)((e >> 6) & 3u)) * nx + x0 + (int)(e & 63u);
+                const double r = ref_point<H>(U, u, idx, nx, sxy);
+                du[idx] = OW ? r : r + du[idx];
+            }
+            __syncwarp();
+        }
+    };
+
+    for (int k = claim_unit(g, s_next, blockIdx.x); k < g.units; k = claim_unit(g, s_next, k + gridDim.x)) {
+        const int unit = (int)(((long long)k * g.perm) % g.units);
+        const int txi = unit % g.tiles_x, rest = unit / g.tiles_x;
+        const int tyi = rest % g.tiles_y, ci = rest / g.tiles_y;
+        const int x0 = txi * C::TX, y0 = tyi * C::TY;
+        const int z0 = B.lo[2] + ci * g.zc, z1 = min(z0 + g.zc, B.hi[2] + 1);  // interior planes of this unit
+        const int npl = z1 - z0 + 2 * H;
+        unsigned off[C::NLD];  // byte offsets in a plane of the values this thread loads
+#pragma unroll
+        for (int j = 0; j < C::NLD; ++j) {
+            const int q = min(tid + j * C::NTHR, C::PLANE - 1);
+            const int r = q / C::BX, c = q - r * C::BX;
+            off[j] = 8u * (unsigned)(min(max(y0 + r - H, 0), ny - 1) * nx + min(max(x0 + c - C::HP, 0), nx - 1));
+        }
+        unsigned live = 0;  // own points (row j, lane v: bit 2j + v) inside the box
+#pragma unroll
+        for (int j = 0; j < RY; ++j)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                const int x = x0 + 2 * tx + v, y = y0 + ty * RY + j;
+                if (x >= B.lo[0] && x <= B.hi[0] && y >= B.lo[1] && y <= B.hi[1]) live |= 1u << (2 * j + v);
+            }
+        const bool all_live = live == (1u << (2 * RY)) - 1u;
+        const char* up = reinterpret_cast<const char*>(u + (int64_t)(z0 - H) * sxy);
+        char* dp = reinterpret_cast<char*>(du + (int64_t)(z0 - 2 * H) * sxy);  // plane p finishes plane p of this
+        const unsigned dof = 8u * (unsigned)((y0 + ty * RY) * nx + x0 + 2 * tx);
+        double raw[C::NLD];
+        auto load = [&](int p) {
+            const char* s = up + (int64_t)p * (sxy * 8);
+#pragma unroll
+            for (int j = 0; j < C::NLD; ++j) raw[j] = __ldg(reinterpret_cast<const double*>(s + off[j]));
+        };
+        // the loaded plane on exponent E into a slot; its largest and smallest nonzero key
+        auto put = [&](Limbs* w, int E, unsigned& mx, unsigned& mn) {
+            mx = 0;
+            mn = 0xffffffffu;
+#pragma unroll
+            for (int j = 0; j < C::NLD; ++j) {
+                const unsigned key = bfp_key(raw[j]);
+                mx = max(mx, key);
+                mn = min(mn, key - 1u);  // (a zero wraps to the largest value)
+                if (j + 1 < C::NLD || tid + j * C::NTHR < C::PLANE) w[tid + j * C::NTHR] = bfp_convert(raw[j], key, E);
+            }
+        };
+        if (tid < 16) {
+            s_max[tid] = 0;
+            s_min[tid] = 0xffffffffu;
+        }
+        load(0);
+        __syncthreads();
+        int E = 64;
+        int low = 0;           // planes since one last reached E
+        unsigned inexact = 0;  // planes in use (bit 0 the newest) of which some value may have lost bits
+        int sl = 0;            // ring slot of plane p
+        for (int p = 0; p < npl; ++p) {
+            {
+                unsigned mx, mn;
+                put(ring + sl * C::SLOT, E, mx, mn);
+                if (p + 1 < npl) load(p + 1);
+                mx = __reduce_max_sync(0xffffffffu, mx);
+                mn = __reduce_min_sync(0xffffffffu, mn);
+                if (tx == 0) {
+                    atomicMax(&s_max[p & 15], mx);
+                    atomicMin(&s_min[p & 15], mn);
+                }
+                if (tid == 0) {
+                    s_max[(p + 2) & 15] = 0;
+                    s_min[(p + 2) & 15] = 0xffffffffu;
+                }
+            }
+            __syncthreads();
+            const int ep = (int)(s_max[p & 15] >> 20);
+            low = ep < E ? low + 1 : 0;
+            if (ep > E || low > NQ + 2) {
+                // a new exponent: the planes in use (this one included) again
+                int ew = 64;
+                for (int b = 0; b < NQ && b <= p; ++b) ew = max(ew, (int)(s_max[(p - b) & 15] >> 20));
+                low = 0;
+                if (ew != E) {
+                    E = ew;
+                    inexact = ~0u;
+                    for (int b = min(NQ - 1, p); b >= 0; --b) {
+                        unsigned mx, mn;
+                        load(p - b);
+                        put(ring + (sl - b < 0 ? sl - b + S : sl - b) * C::SLOT, E, mx, mn);
+                    }
+                    if (p + 1 < npl) load(p + 1);
+                    __syncthreads();
+                }
+            }
+            inexact = inexact << 1 | (unsigned)(E - (int)(s_min[p & 15] >> 20) > BFP_G);  // (key - 1: at most one binade below)
+            const int cur = sl;
+            sl = sl + 1 == S ? 0 : sl + 1;
+            if (p < 2 * H) continue;
+            const int kexp = B.kbase + E;
+            // thresholds of this plane: none when no value in use lost a bit, out of reach when the
+            // exponent rules fixed point out
+            const bool special = E >= 2047 || !bfp_range_ok(kexp);
+            const bool exact = !(inexact & ((1u << NQ) - 1u));
+            const int t0 = special ? INT_MAX : (exact ? 0 : B.t0);
+            const double scale = special ? 1.0 : bfp_pow2(kexp);
+            const int4* pl[NQ];  // own pair of the first row in the planes z - H .. z + H
+#pragma unroll
+            for (int m = 0; m < NQ; ++m) {
+                const int i = cur - (NQ - 1 - m);
+                pl[m] = reinterpret_cast<const int4*>(ring + (i < 0 ? i + S : i) * C::SLOT + own);
+            }
+            int4 yc[RY + 2 * H];  // the centre plane's pair at rows -H .. RY - 1 + H
+#pragma unroll
+            for (int m = 0; m < RY + 2 * H; ++m) yc[m] = pl[H][(m - H) * (C::BX / 2)];
+            char* dz = dp + (int64_t)p * (sxy * 8);
+            double r[RY][2];
+            int far[RY][2];  // distance of each point from its fallback, against t0
+#pragma unroll
+            for (int j = 0; j < RY; ++j) {
+                int4 xs[2 * HL + 1], zs[NQ];
+#pragma unroll
+                for (int m = 0; m < 2 * HL + 1; ++m) xs[m] = m == HL ? yc[H + j] : pl[H][j * (C::BX / 2) + m - HL];
+#pragma unroll
+                for (int m = 0; m < NQ; ++m) zs[m] = m == H ? yc[H + j] : pl[m][j * (C::BX / 2)];
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    auto hl = [&](const int4& t, int w) { return w ? Limbs{t.z, t.w} : Limbs{t.x, t.y}; };
+                    const Limbs c = hl(yc[H + j], v);
+                    BfpAcc a{0, 0, 0};
+                    bfp_mad(a, B.c0h, B.c0l, c.h, c.l);
+                    int n1 = 0;  // the neighbours at +1
+#pragma unroll
+                    for (int o = 1; o <= H; ++o)
+#pragma unroll
+                        for (int sd = 0; sd < 2; ++sd) {
+                            const int so = sd ? o : -o, xi = 2 * HL + v + so;
+                            const Limbs X = hl(xs[xi >> 1], xi & 1), Y = hl(yc[H + j + so], v), Z = hl(zs[H + so], v);
+                            if constexpr (SH) {
+                                const int sh = X.h + Y.h + Z.h, sl3 = X.l + Y.l + Z.l;
+                                bfp_mad(a, B.wh[0][H + so], B.wl[0][H + so], sh, sl3);
+                                if (so == 1) n1 = sh;
+                            } else {
+                                bfp_mad(a, B.wh[0][H + so], B.wl[0][H + so], X.h, X.l);
+                                bfp_mad(a, B.wh[1][H + so], B.wl[1][H + so], Y.h, Y.l);
+                                bfp_mad(a, B.wh[2][H + so], B.wl[2][H + so], Z.h, Z.l);
+                                if (so == 1) n1 = X.h;
+                            }
+                        }
+                    r[j][v] = bfp_double(bfp_total(a), scale);
+                    far[j][v] = max(abs(c.h), abs(n1) >> B.sh1);
+                }
+            }
+            int nearest = INT_MAX;
+#pragma unroll
+            for (int j = 0; j < RY; ++j) nearest = min(nearest, min(far[j][0], far[j][1]));
+            if (__all_sync(0xffffffffu, all_live && nearest >= t0)) {
+#pragma unroll
+                for (int j = 0; j < RY; ++j) {
+                    double* d = reinterpret_cast<double*>(dz + (dof + 8u * (unsigned)(j * nx)));
+                    if (pairs) {
+                        double2* d2 = reinterpret_cast<double2*>(d);
+                        if constexpr (OW) *d2 = make_double2(r[j][0], r[j][1]);
+                        else *d2 = make_double2(r[j][0] + d2->x, r[j][1] + d2->y);
+                    } else {
+                        d[0] = OW ? r[j][0] : r[j][0] + d[0];
+                        d[1] = OW ? r[j][1] : r[j][1] + d[1];
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int b = 0; b < 2 * RY; ++b) {
+                    const bool on = (live >> b) & 1u, ok = far[b / 2][b % 2] >= t0;
+                    if (on && ok) {
+                        double* d = reinterpret_cast<double*>(dz + (dof + 8u * (unsigned)((b / 2) * nx + b % 2)));
+                        *d = OW ? r[b / 2][b % 2] : r[b / 2][b % 2] + *d;
+                    }
+                    const unsigned bal = __ballot_sync(0xffffffffu, on && !ok);
+                    if (on && !ok)
+                        queue[nq + __popc(bal & ((1u << tx) - 1u))] =
+                            (unsigned short)((unsigned)(p - 2 * H) << 8 | (unsigned)(b / 2) << 6 | (unsigned)(2 * tx + b % 2));
+                    nq += __popc(bal);
+                }
+                __syncwarp();
+                if (nq > C::QCAP - 64 * RY) drain(31, x0, y0, z0);
+            }
+        }
+        drain(0, x0, y0, z0);
+        __syncthreads();  // the next unit reuses the ring and the exponents
+    }
+}
+
+}  // namespace march
+}  // namespace deo
+
+using namespace deo;
+
+namespace {
+
+// Units of (tile, chunk of interior planes) for G resident CTAs that claim them
+// from a counter.  A unit of zc planes costs about zc + 0.4 * 2H + 3 planes (the
+// planes that only fill the ring are converted, not evaluated), and the last
+// round leaves about a third of a unit idle.  A queued point holds its plane in 8
+// bits, so zc <= 256.
+LapGrid chunks_of(const UniPlan* up, const BfpMarch* B, int tx, int ty, int H, int64_t G) {
+    const int nzi = B->hi[2] - B->lo[2] + 1;
+    LapGrid g{};
+    g.tiles_x = (int)((up->n[0] + tx - 1) / tx);
+    g.tiles_y = (int)((up->n[1] + ty - 1) / ty);
+    const int64_t tiles = (int64_t)g.tiles_x * g.tiles_y;
+    double best = 1e300;
+    for (int c = (nzi + 255) / 256; c <= nzi; ++c) {
+        const int zc = (nzi + c - 1) / c;
+        const double rounds = std::max(1.0, (double)(tiles * ((nzi + zc - 1) / zc)) / (double)G + 0.35);
+        const double t = rounds * (zc + 0.8 * H + 3.0);
+        if (t < best) {
+            best = t;
+            g.zc = zc;
+        }
+        if (zc <= 4) break;
+    }
+    g.chunks = (nzi + g.zc - 1) / g.zc;
+    g.units = (int)(tiles * g.chunks);
+    g.perm = 1;
+    return g;
+}
+
+template <int H, bool SH, int TYT, int RY>
+int launch(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du, int ow,
+           cudaStream_t st) {
+    using C = march::Cfg<H, TYT, RY>;
+    static int64_t G = 0;
+    if (!G) {
+        int e = occupancy_grid(march::k_lap_fx<H, SH, true, TYT, RY>, C::NTHR, C::SMEM, G);
+        if (!e) e = occupancy_grid(march::k_lap_fx<H, SH, false, TYT, RY>, C::NTHR, C::SMEM, G);
+        if (e) return e;
+    }
+    LapGrid g = chunks_of(up, B, C::TX, C::TY, H, G);
+    g.sched = sched;
+    if (sched) {
+        const cudaError_t e = cudaMemsetAsync(sched, 0, sizeof(unsigned int), st);
+        if (e != cudaSuccess) return (int)e;
+    }
+    const int grid = (int)std::min<int64_t>(G, g.units);
+    const int pairs = up->n[0] % 2 == 0 && (uintptr_t)du % 16 == 0;  // 16-byte stores
+    auto go = [&](auto kernel) {
+        kernel<<<grid, dim3(32, TYT), C::SMEM, st>>>(*up, *B, g, (const double*)u, (double*)du, pairs);
+    };
+    if (ow) go(march::k_lap_fx<H, SH, true, TYT, RY>);
+    else go(march::k_lap_fx<H, SH, false, TYT, RY>);
+    return (int)cudaGetLastError();
+}
+
+}  // namespace
+
+extern "C" int deo_k_apply_march(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du,
+                                 int overwrite, void* stream) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    for (int a = 0; a < 3; ++a)
+        if (B->lo[a] > B->hi[a]) return 0;  // no interior point
+    switch (up->radius) {
+        case 1: return B->shared ? launch<1, true, 4, 2>(up, B, sched, u, du, overwrite, st)
+                                 : launch<1, false, 4, 2>(up, B, sched, u, du, overwrite, st);
+        case 2: return B->shared ? launch<2, true, 4, 2>(up, B, sched, u, du, overwrite, st)
+                                 : launch<2, false, 4, 2>(up, B, sched, u, du, overwrite, st);
+        case 3: return B->shared ? launch<3, true, 4, 2>(up, B, sched, u, du, overwrite, st)
+                                 : launch<3, false, 4, 2>(up, B, sched, u, du, overwrite, st);
+    }
+    return (int)cudaErrorNotSupported;
+}

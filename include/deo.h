@@ -229,9 +229,11 @@ int deo_plan_star_taps(const deo_plan* plan);
  *   DEO_OPT_EXACT_SUMS: Float64 Laplacian-type plans whose terms share one
  *     band evaluate interior points in integer arithmetic and round once
  *     (result within a few ulp of sum|c_k u_k| of the reference's order):
- *       1 the best variant that applies (default): the per-point
- *         fixed-point kernel (variant 4) when the band's weights allow it,
- *         else variant 3;
+ *       1 the best variant that applies (default): for three axes with band
+ *         radius <= 3 the marching block fixed-point kernel (any alignment and
+ *         any bands; within 2 ulp of sum|c_k u_k| of the exact sum); else the
+ *         per-point fixed-point kernel (variant 4) when the band's weights
+ *         allow it, else variant 3;
  *       5 for three axes the block fixed-point kernel (values aligned once
  *         per plane to one exponent per plane tile, no FP64 instruction per
  *         point; points near a zero of u, where that alignment cannot bound
@@ -262,8 +264,8 @@ int deo_plan_star_taps(const deo_plan* plan);
  *     plane; whole warps) are evaluated in the reference's per-term tap order
  *     on the FP64 pipe, bit-identical to the generic kernel, while the others
  *     use the integer pipes; 0 evaluates every interior point in fixed point.
- *     deo_plan_get_option returns the value when the fixed-point kernel
- *     applies, else 0.
+ *     Setting it keeps a plan on the per-point kernel.  deo_plan_get_option
+ *     returns the value when that kernel applies, else 0.
  *   DEO_OPT_TEST_WITHHOLD: 0 (default) or k in 1..64, for tests of the
  *     bounded waits only: the TMA kernels (interior and shell) withhold the
  *     copy of plane k of each CTA's first unit (the shell: each CTA's first
