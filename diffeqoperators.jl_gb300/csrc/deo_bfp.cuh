@@ -70,6 +70,13 @@ __device__ __forceinline__ long long bfp_total(const BfpAcc& a) {
 }
 // t * 2^k (scale = 2^k; no nonzero t leaves the normal range, see bfp_range_ok).
 __device__ __forceinline__ double bfp_double(long long t, double scale) { return __ll2double_rn(t) * scale; }
+// The same by the exponent field, without FP64: k20 = k * 2^20.
+__device__ __forceinline__ double bfp_double(long long t, int k20) {
+    const double r = __ll2double_rn(t);
+    int hi = __double2hiint(r);
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.s32 p, %0, 0;\n\t@p add.s32 %0, %0, %1;\n\t}" : "+r"(hi) : "r"(k20));
+    return __hiloint2double(hi, __double2loint(r));
+}
 // 2^k, k in the normal range
 __device__ __forceinline__ double bfp_pow2(int k) { return __hiloint2double((1023 + k) << 20, 0); }
 __host__ __device__ __forceinline__ bool bfp_range_ok(int k) { return 1023 + k >= 1 && 1023 + 62 + k <= 2046; }

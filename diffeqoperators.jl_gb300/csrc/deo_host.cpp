@@ -810,6 +810,21 @@ constexpr unsigned int kSchedSlots = 1024;
 // integer-pipe rows
 constexpr int kFxFp64Rows = 2;
 
+// Rotating claim counters of the marching kernels: two words each, zeroed here
+// once and left zero by every launch (claims_done in deo_lap.cuh).
+struct ClaimSlots {
+    unsigned int* d = nullptr;
+    std::atomic<unsigned int> slot{0};
+    ~ClaimSlots() {
+        if (d) cudaFree(d);
+    }
+    cudaError_t init() {
+        cudaError_t e = cudaMalloc(&d, 2 * kSchedSlots * sizeof(unsigned int));
+        return e == cudaSuccess ? cudaMemset(d, 0, 2 * kSchedSlots * sizeof(unsigned int)) : e;
+    }
+    unsigned int* next() { return d + 2 * (slot.fetch_add(1) % kSchedSlots); }
+};
+
 struct deo_plan {
     PlanDev dev{};
     deo::UniPlan uni{};
@@ -831,6 +846,7 @@ struct deo_plan {
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     unsigned int* d_sched = nullptr;  // kSchedSlots unit counters, one per apply in rotation
     mutable std::atomic<unsigned int> sched_slot{0};
+    mutable ClaimSlots claims;  // of the marching interior
     mutable std::mutex apply_mu;  // one fork/join sequence at a time per plan
     std::vector<void*> allocs;
     size_t table_bytes = 0;
@@ -1078,16 +1094,36 @@ static void split_limbs(long long W, int& h, int& l) {
     h = (int)((W + (1LL << 29)) >> 30);
     l = (int)(W - ((long long)h << 30));
 }
+static int bfp_threshold(double total, double W, double slack) {
+    const double t = std::fabs(W) > 0.0 ? std::ldexp(1.05 * total / std::fabs(W), 22) + slack : 4e9;
+    return t < 2147483647.0 ? (int)std::ceil(t) : INT_MAX;
+}
+// s such that the sum of |w| * 2^s stays below 2^60 (one bit for the sum's own rounding)
+static bool bfp_scale(double sum, int& s) {
+    if (!(sum > 0.0) || std::fpclassify(sum) != FP_NORMAL) return false;
+    s = 59 - std::ilogb(sum) - 1;
+    return true;
+}
+// The limbs of one row's K weights on a scale of their own; total = the sum of |W|.
+static bool bfp_band(const double* w, int K, int& s, double& total, int* wh, int* wl) {
+    double sum = 0.0;
+    for (int k = 0; k < K; ++k) sum += std::fabs(w[k]);
+    if (!bfp_scale(sum, s)) return false;
+    total = 0.0;
+    for (int k = 0; k < K; ++k) {
+        const long long W = std::llrint(std::ldexp(w[k], s));
+        total += std::fabs((double)W);
+        split_limbs(W, wh[k], wl[k]);
+    }
+    return true;
+}
 static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
     const int K = 2 * H + 1;
     double sum = 0.0;
     for (int a = 0; a < 3; ++a)
-        for (int k = 0; k < K; ++k) {
-            if (!std::isfinite(w[a][k])) return false;
-            sum += std::fabs(w[a][k]);
-        }
-    if (!(sum > 0.0) || std::fpclassify(sum) != FP_NORMAL) return false;
-    const int s = 59 - std::ilogb(sum) - 1;  // (one bit for the sum's own rounding)
+        for (int k = 0; k < K; ++k) sum += std::fabs(w[a][k]);
+    int s = 0;
+    if (!bfp_scale(sum, s)) return false;
     long long c0 = 0;
     double total = 0.0;
     for (int a = 0; a < 3; ++a)
@@ -1099,13 +1135,8 @@ static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
         }
     split_limbs(c0, B.c0h, B.c0l);
     B.shared = std::memcmp(w[0], w[1], K * sizeof(double)) == 0 && std::memcmp(w[0], w[2], K * sizeof(double)) == 0;
-    auto threshold = [&](double W, double slack) {
-        const double t = std::fabs(W) > 0.0 ? std::ldexp(1.05 * total / std::fabs(W), 22) + slack : 4e9;
-        return t < 2147483647.0 ? (int)std::ceil(t) : INT_MAX;
-    };
-    auto limb = [&](int a, int k) { return (double)(((long long)B.wh[a][k] << 30) + B.wl[a][k]); };
-    B.t0 = threshold((double)c0, 1.0);
-    const int t1 = threshold(limb(0, H + 1), 2.0);
+    B.t0 = bfp_threshold(total, (double)c0, 1.0);
+    const int t1 = bfp_threshold(total, std::ldexp(w[0][H + 1], s), 2.0);
     B.sh1 = 0;
     while (B.sh1 < 31 && ((long long)B.t0 << B.sh1) < t1) ++B.sh1;  // |n1| >> sh1 >= t0 implies |n1| >= t1
     B.kbase = 57 - s - 1075 - 6;
@@ -1448,6 +1479,7 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
     }
     CUDA_TRY(cudaMalloc(&P->d_plan, sizeof(PlanDev)), "cudaMalloc(plan)");
     CUDA_TRY(cudaMemcpy(P->d_plan, &P->dev, sizeof(PlanDev), cudaMemcpyHostToDevice), "cudaMemcpy(plan)");
+    if (P->march.ok) CUDA_TRY(P->claims.init(), "cudaMalloc(claim counters)");
     if (P->shell.ok && P->uni.enabled && P->uni.lap) {
         CUDA_TRY(cudaMalloc(&P->d_shell, sizeof(deo::ShellPlan)), "cudaMalloc(shell rows)");
         CUDA_TRY(cudaMemcpy(P->d_shell, &P->shell, sizeof(deo::ShellPlan), cudaMemcpyHostToDevice),
@@ -1542,7 +1574,7 @@ static int launch_march(const deo_plan* p, const void* u, void* du, int overwrit
         const cudaError_t c = cudaEventRecord(p->ev_fork, st);
         if (c != cudaSuccess) return (int)c;
     }
-    int e = deo_k_apply_march(&p->uni, &p->march, next_sched(p), u, du, overwrite, stream);
+    int e = deo_k_apply_march(&p->uni, &p->march, p->claims.next(), u, du, overwrite, stream);
     if (e) return e;
     mark(p, 1, stream);
     if (conc) {
@@ -1759,7 +1791,7 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
             reverse_taps(B.wh[a], K);
             reverse_taps(B.wl[a], K);
         }
-        int e = deo_k_apply_march(&ua, &B, next_sched(p), d, ub, overwrite, stream);
+        int e = deo_k_apply_march(&ua, &B, p->claims.next(), d, ub, overwrite, stream);
         if (!e) e = deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, stream);
         if (e) return e;
         p->last_kernel = "k_lap_fx";
@@ -1929,6 +1961,8 @@ extern "C" void deo_nonlinear_diffusion_destroy(deo_nld* nl) { delete nl; }
 struct deo_vc {
     deo_plan tabs;  // owns the uploaded tables (no kernels of its own)
     deo::VcDev dev{};
+    deo::VcBfp bfp{};  // 3-D Float64 with a uniform band: block fixed point (ok = 0: not this plan)
+    mutable ClaimSlots claims;
     int dtype = 0;
     int ncomp_in = 1, ncomp_out = 1;
 };
@@ -1997,6 +2031,30 @@ extern "C" deo_status deo_vector_calculus_plan(int kind, int ndims, const deo_op
             bnk = 0;
     }
     D.band_nk = (bnk == 3 || bnk == 5 || bnk == 7 || bnk == 9) ? bnk : 0;
+    if (D.band_nk && ndims == 3 && dtype == DEO_F64 && D.pstride[2] < (1LL << 28)) {
+        V->bfp.ok = 1;
+        for (int a = 0; a < 3; ++a) {
+            const double* w = D.t[a].tab[0].wband;
+            double total = 0.0;
+            int s = 0, wh[DEO_MAX_NW], wl[DEO_MAX_NW];
+            const int mid = bnk / 2;
+            if (!bfp_band(w, bnk, s, total, wh, wl)) V->bfp.ok = 0;
+            auto W = [&](int k) { return ((long long)wh[k] << 30) + wl[k]; };
+            // antisymmetric up to a few units: W(+o) (x(+o) - x(-o)) + d x(-o), d = W(+o) + W(-o), and the centre
+            for (int o = 1; o <= mid && V->bfp.ok; ++o) {
+                const long long d = W(mid + o) + W(mid - o);
+                if (std::llabs(d) >= (1 << 20) || (bnk < 7 && d != 0)) V->bfp.ok = 0;
+                V->bfp.wh[a][o] = wh[mid + o];
+                V->bfp.wl[a][o] = wl[mid + o];
+                V->bfp.wd[a][o] = (int)d;
+            }
+            if (V->bfp.ok && std::llabs(W(mid)) >= (1 << 20)) V->bfp.ok = 0;
+            V->bfp.wd[a][0] = V->bfp.ok ? (int)W(mid) : 0;
+            V->bfp.t0 = std::max(V->bfp.t0, bfp_threshold(total, (double)W(mid + 1), 1.0));
+            V->bfp.kbase[a] = 57 - s - 1075 - 6;
+        }
+        if (V->bfp.ok) CUDA_TRY(V->claims.init(), "cudaMalloc(claim counters)");
+    }
     V->dtype = dtype;
     V->ncomp_in = kind == DEO_VC_GRADIENT ? 1 : (kind == DEO_VC_CURL ? 3 : ndims);
     V->ncomp_out = kind == DEO_VC_DIVERGENCE ? 1 : (kind == DEO_VC_CURL ? 3 : ndims);
@@ -2028,7 +2086,7 @@ extern "C" deo_status deo_vector_calculus_apply(const deo_vc* vc, const void* M,
     const size_t es = vc->dtype == DEO_F64 ? 8 : 4;
     if (overlaps(M, (size_t)(vc->dev.pvol * vc->ncomp_in) * es, out, (size_t)(vc->dev.ovol * vc->ncomp_out) * es))
         return fail(DEO_ERR_BAD_ARG, "the output must not overlap the input");
-    const int e = deo_k_vector_calculus(&vc->dev, vc->dtype, M, out, overwrite ? 1 : 0, stream);
+    const int e = deo_k_vector_calculus(&vc->dev, &vc->bfp, vc->bfp.ok ? vc->claims.next() : nullptr, vc->dtype, M, out, overwrite ? 1 : 0, stream);
     if (e) return cuda_fail((cudaError_t)e, "deo_vector_calculus_apply launch");
     return DEO_OK;
 }

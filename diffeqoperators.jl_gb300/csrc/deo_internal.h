@@ -265,12 +265,24 @@ struct VcDev {
     TermDev tn[3];
 };
 
+// The first-derivative band of each axis in block fixed point (deo_bfp.cuh), its
+// own scale per axis: a derivative in units of 2^57 times 2^(kbase[a] + E) is the
+// result.  The band is antisymmetric up to a few units: the limbs [o] multiply
+// x(+o) - x(-o); wd[o] units (wd[0]: the centre's weight) multiply x(-o), and the
+// kernels for up to 5 taps have wd[o > 0] = 0.
+struct VcBfp {
+    int ok;
+    int wh[3][5], wl[3][5], wd[3][5];
+    int t0;  // a derivative is accepted when the larger of its two nearest taps' high limbs reaches this
+    int kbase[3];
+};
+
 }  // namespace deo
 
 // Launchers implemented in deo_vector.cu.  kind/nd/quirk come from V; out may
 // not overlap M.  overwrite = 1 writes A*M, 0 adds it to out (mul!).
-extern "C" int deo_k_vector_calculus(const deo::VcDev* V, int dtype, const void* M, void* out, int overwrite,
-                                     void* stream);
+extern "C" int deo_k_vector_calculus(const deo::VcDev* V, const deo::VcBfp* B, unsigned int* claims, int dtype,
+                                     const void* M, void* out, int overwrite, void* stream);
 // L*M on a padded array: V.t[0] is the operator's table (generic methods),
 // V.len the output size, V.pstride M's strides; coff the offset of the
 // stripped edge planes of M's other axes.

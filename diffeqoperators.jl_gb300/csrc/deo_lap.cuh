@@ -34,6 +34,23 @@ __device__ __forceinline__ int claim_unit(const LapGrid& g, int& s_next, int k_s
     return s_next;
 }
 
+// The marching kernels' claims: counter[0] the next unit, counter[1] the CTAs
+// that have left; the last to leave zeroes both, so a launch needs no memset
+// before it (a memset node costs about 2 us of a short apply).
+__device__ __forceinline__ int claim_next(unsigned int* counter, int& s_next) {
+    if (threadIdx.x == 0 && threadIdx.y == 0) s_next = (int)atomicAdd(counter, 1u);
+    __syncthreads();
+    return s_next;
+}
+__device__ __forceinline__ void claims_done(unsigned int* counter) {
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        __threadfence();
+        if (atomicAdd(counter + 1, 1u) == gridDim.x - 1) {
+            counter[0] = 0u;
+            counter[1] = 0u;
+        }
+    }
+}
 
 // Units and z chunk for a persistent grid of G CTAs (see LapGrid).
 static inline LapGrid make_grid(const UniPlan* up, int tx, int ty, int H, int nt, int64_t G) {
@@ -74,6 +91,33 @@ static inline LapGrid make_grid(const UniPlan* up, int tx, int ty, int H, int nt
             break;
         }
     }
+    return g;
+}
+
+// Units of (tile, chunk of nz planes) for the marching block fixed-point kernels
+// with G resident CTAs that share them out.  A unit of zc planes costs about
+// zc + 0.4 * 2H + 3 planes (the planes that only fill the ring are converted, not
+// evaluated), and the last round leaves about a third of a unit idle.  A queued
+// point holds its plane in 8 bits, so zc <= 256.
+static inline LapGrid march_chunks(int64_t nx, int64_t ny, int nz, int tx, int ty, int H, int64_t G) {
+    LapGrid g{};
+    g.tiles_x = (int)((nx + tx - 1) / tx);
+    g.tiles_y = (int)((ny + ty - 1) / ty);
+    const int64_t tiles = (int64_t)g.tiles_x * g.tiles_y;
+    double best = 1e300;
+    for (int c = (nz + 255) / 256; c <= nz; ++c) {
+        const int zc = (nz + c - 1) / c;
+        const double rounds = std::max(1.0, (double)(tiles * ((nz + zc - 1) / zc)) / (double)G + 0.35);
+        const double t = rounds * (zc + 0.8 * H + 3.0);
+        if (t < best) {
+            best = t;
+            g.zc = zc;
+        }
+        if (zc <= 4) break;
+    }
+    g.chunks = (nz + g.zc - 1) / g.zc;
+    g.units = (int)(tiles * g.chunks);
+    g.perm = 1;
     return g;
 }
 

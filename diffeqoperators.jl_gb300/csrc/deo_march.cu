@@ -88,25 +88,24 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
     const int64_t sxy = (int64_t)nx * ny;
     const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
     const int own = (ty * RY + H) * C::BX + C::HP + 2 * tx;  // the first own row's pair inside a slot
-    int nq = 0;                                              // this warp's queued points
-
-    auto drain = [&](int keep, int x0, int y0, int z0) {
+    int nq = 0;  // this warp's queued points
+    __shared__ int s_nq[TYT];
+    auto point = [&](int w, unsigned e, int x0, int y0, int z0) {  // a queued point of warp w
+        const int64_t idx = (int64_t)(z0 + (int)(e >> 8)) * sxy + (int64_t)(y0 + w * RY + (int)((e >> 6) & 3u)) * nx + x0 +
+                            (int)(e & 63u);
+        const double r = ref_point<H>(U, u, idx, nx, sxy);
+        du[idx] = OW ? r : r + du[idx];
+    };
+    auto drain = [&](int keep, int x0, int y0, int z0) {  // this warp's own, when its queue is nearly full
         while (nq > keep) {
             const int n = min(nq, 32);
             nq -= n;
-            if (tx < n) {
-                const unsigned e = queue[nq + tx];
-                const int64_t idx = (int64_t)(z0 + (int)(e >> 8)) * sxy +
-                                    (int64_t)(y0 + ty * RY + (int)((e >> 6) & 3u)) * nx + x0 + (int)(e & 63u);
-                const double r = ref_point<H>(U, u, idx, nx, sxy);
-                du[idx] = OW ? r : r + du[idx];
-            }
+            if (tx < n) point(ty, queue[nq + tx], x0, y0, z0);
             __syncwarp();
         }
     };
 
-    for (int k = claim_unit(g, s_next, blockIdx.x); k < g.units; k = claim_unit(g, s_next, k + gridDim.x)) {
-        const int unit = (int)(((long long)k * g.perm) % g.units);
+    for (int unit = claim_next(g.sched, s_next); unit < g.units; unit = claim_next(g.sched, s_next)) {
         const int txi = unit % g.tiles_x, rest = unit / g.tiles_x;
         const int tyi = rest % g.tiles_y, ci = rest / g.tiles_y;
         const int x0 = txi * C::TX, y0 = tyi * C::TY;
@@ -287,9 +286,17 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                 if (nq > C::QCAP - 64 * RY) drain(31, x0, y0, z0);
             }
         }
-        drain(0, x0, y0, z0);
-        __syncthreads();  // the next unit reuses the ring and the exponents
+        // the queues, shared out over the CTA
+        if (tx == 0) s_nq[ty] = nq;
+        __syncthreads();
+        nq = 0;
+        for (int w = 0, i = tid; w < TYT; ++w) {
+            for (; i < s_nq[w]; i += C::NTHR) point(w, (queue + (w - ty) * C::QCAP)[i], x0, y0, z0);
+            i -= s_nq[w];
+        }
+        __syncthreads();  // the next unit reuses the ring, the queues and the exponents
     }
+    claims_done(g.sched);
 }
 
 }  // namespace march
@@ -298,34 +305,6 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
 using namespace deo;
 
 namespace {
-
-// Units of (tile, chunk of interior planes) for G resident CTAs that claim them
-// from a counter.  A unit of zc planes costs about zc + 0.4 * 2H + 3 planes (the
-// planes that only fill the ring are converted, not evaluated), and the last
-// round leaves about a third of a unit idle.  A queued point holds its plane in 8
-// bits, so zc <= 256.
-LapGrid chunks_of(const UniPlan* up, const BfpMarch* B, int tx, int ty, int H, int64_t G) {
-    const int nzi = B->hi[2] - B->lo[2] + 1;
-    LapGrid g{};
-    g.tiles_x = (int)((up->n[0] + tx - 1) / tx);
-    g.tiles_y = (int)((up->n[1] + ty - 1) / ty);
-    const int64_t tiles = (int64_t)g.tiles_x * g.tiles_y;
-    double best = 1e300;
-    for (int c = (nzi + 255) / 256; c <= nzi; ++c) {
-        const int zc = (nzi + c - 1) / c;
-        const double rounds = std::max(1.0, (double)(tiles * ((nzi + zc - 1) / zc)) / (double)G + 0.35);
-        const double t = rounds * (zc + 0.8 * H + 3.0);
-        if (t < best) {
-            best = t;
-            g.zc = zc;
-        }
-        if (zc <= 4) break;
-    }
-    g.chunks = (nzi + g.zc - 1) / g.zc;
-    g.units = (int)(tiles * g.chunks);
-    g.perm = 1;
-    return g;
-}
 
 template <int H, bool SH, int TYT, int RY>
 int launch(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du, int ow,
@@ -337,12 +316,8 @@ int launch(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void
         if (!e) e = occupancy_grid(march::k_lap_fx<H, SH, false, TYT, RY>, C::NTHR, C::SMEM, G);
         if (e) return e;
     }
-    LapGrid g = chunks_of(up, B, C::TX, C::TY, H, G);
+    LapGrid g = march_chunks(up->n[0], up->n[1], B->hi[2] - B->lo[2] + 1, C::TX, C::TY, H, G);
     g.sched = sched;
-    if (sched) {
-        const cudaError_t e = cudaMemsetAsync(sched, 0, sizeof(unsigned int), st);
-        if (e != cudaSuccess) return (int)e;
-    }
     const int grid = (int)std::min<int64_t>(G, g.units);
     const int pairs = up->n[0] % 2 == 0 && (uintptr_t)du % 16 == 0;  // 16-byte stores
     auto go = [&](auto kernel) {

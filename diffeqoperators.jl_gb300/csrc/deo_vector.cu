@@ -10,12 +10,15 @@
 // fused multiply-adds in the same order.  The reference's per-point additions
 // into the output are replayed in its order (see VcDev).
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include <algorithm>
 #include <type_traits>
 
+#include "deo_bfp.cuh"
 #include "deo_eval.cuh"
+#include "deo_lap.cuh"
 
 namespace deo {
 namespace {
@@ -44,73 +47,75 @@ __device__ __forceinline__ T vc_deriv(const TermDev& t, const T* __restrict__ M,
     return eval_row_padded<T>(t.tab[0], M + ia - (oa + 1) * s, s, (int)oa + 1);  // the line's left ghost
 }
 
-// The 2-D / 3-D methods (vector_calculus_convolutions.jl:174-838, curl :844-1067).
-// Blocks of 32 x 8 points of one (x, y) plane; blockIdx.z walks the planes.
-// Used for Float64, for operators without a uniform interior band, and where
-// the marching kernel's grid would not fit; launched with NK = 0 (every row
-// from the row tables).  NK > 0 would give a derivative along an axis on which
-// the point is an interior row the unrolled band loop.
-template <typename T, int KIND, int ND, int NK>
+// One output point of the 2-D / 3-D methods (vector_calculus_convolutions.jl:174-838,
+// curl :844-1067), every row from the row table (NK = 0), or an interior point
+// of a uniform band of NK taps.
+template <typename T, int KIND, int ND, int NK = 0>
+__device__ __forceinline__ void vc_point(const VcDev& V, const T* __restrict__ M, T* __restrict__ out, int overwrite,
+                                         int64_t o0, int64_t o1, int64_t o2) {
+    const int64_t n = o0 + V.len[0] * (o1 + (ND == 3 ? V.len[1] : 1) * o2);
+    const int64_t o[3] = {o0, o1, o2};
+    // other axes at the padded index equal to the output index; +1 along the differentiated axis
+    int64_t q = 0;
+#pragma unroll
+    for (int b = 0; b < ND; ++b) q += o[b] * V.pstride[b];
+    int ph[ND];
+#pragma unroll
+    for (int a = 0; a < ND; ++a) ph[a] = vc_phase(o[a], V.len[a], V.bpc);
+    auto D = [&](const TermDev& t, const T* x, int a) { return vc_deriv<T, NK>(t, x, q + V.pstride[a], o[a]); };
+    if (KIND == DEO_VC_GRADIENT) {
+#pragma unroll
+        for (int a = 0; a < ND; ++a) {
+            const T d = D(V.t[a], M, a);
+            T* y = out + n + a * V.ovol;
+            *y = overwrite ? zero_fix(d) : *y + d;
+        }
+    } else if (KIND == DEO_VC_DIVERGENCE) {
+        T d[ND];
+#pragma unroll
+        for (int a = 0; a < ND; ++a) d[a] = D(V.t[a], M + a * V.pvol, a);
+        T acc = overwrite ? T(0) : out[n];
+        bool first = overwrite != 0;  // 0 + x is x up to the sign of zero
+#pragma unroll
+        for (int p = 0; p < 3; ++p)
+#pragma unroll
+            for (int a = 0; a < ND; ++a)
+                if (ph[a] == p) {
+                    acc = first ? zero_fix(d[a]) : acc + d[a];
+                    first = false;
+                }
+        out[n] = acc;
+    } else {
+        // curl component c = (D_{a1} u[c1]) sign1 + (D_{a2} u[c2]) sign2, a1 < a2:
+        //   x1: +D2 u3, -D3 u2;  x2: -D1 u3, +D3 u1;  x3: +D1 u2, -D2 u1
+        constexpr int A1[3] = {1, 0, 0}, A2[3] = {2, 2, 1};
+        constexpr int C1[3] = {2, 2, 1}, C2[3] = {1, 0, 0};
+        constexpr bool N1[3] = {false, true, false}, N2[3] = {true, false, true};
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const int a1 = A1[c], a2 = A2[c];
+            const T e1 = D(N1[c] ? V.tn[a1] : V.t[a1], M + C1[c] * V.pvol, a1);
+            const T e2 = D(N2[c] ? V.tn[a2] : V.t[a2], M + C2[c] * V.pvol, a2);
+            T* y = out + n + c * V.ovol;
+            const T f = ph[a1] <= ph[a2] ? e1 : e2, g = ph[a1] <= ph[a2] ? e2 : e1;
+            *y = (overwrite ? zero_fix(f) : *y + f) + g;
+        }
+    }
+}
+
+// The 2-D / 3-D methods point by point: blocks of 32 x 8 points of one (x, y)
+// plane; blockIdx.z walks the planes.  Used where neither marching kernel
+// applies (2-D Float64, operators without a uniform interior band, grids
+// beyond the launch limits).
+template <typename T, int KIND, int ND>
 __global__ void __launch_bounds__(256) k_vc(const VcDev V, const T* __restrict__ M, T* __restrict__ out,
                                             int overwrite) {
     const int64_t n0 = V.len[0], n1 = V.len[1], n2 = ND == 3 ? V.len[2] : 1;
     const int64_t o0 = (int64_t)blockIdx.x * 32 + threadIdx.x % 32;
     if (o0 >= n0) return;
-    for (int64_t o1 = (int64_t)blockIdx.y * 8 + threadIdx.x / 32; o1 < n1; o1 += (int64_t)gridDim.y * 8) {
-        for (int64_t o2 = blockIdx.z; o2 < n2; o2 += gridDim.z) {
-            const int64_t o[3] = {o0, o1, o2};
-            const int64_t n = o0 + n0 * (o1 + n1 * o2);
-            // other axes at the padded index equal to the output index; +1 along the differentiated axis
-            int64_t q = 0;
-#pragma unroll
-            for (int b = 0; b < ND; ++b) q += o[b] * V.pstride[b];
-            int ph[ND];
-#pragma unroll
-            for (int a = 0; a < ND; ++a) ph[a] = vc_phase(o[a], V.len[a], V.bpc);
-            auto D = [&](const TermDev& t, const T* x, int a) {
-                return (NK > 0 && ph[a] == 1) ? vc_deriv<T, NK>(t, x, q + V.pstride[a], o[a])
-                                              : vc_deriv<T, 0>(t, x, q + V.pstride[a], o[a]);
-            };
-            if (KIND == DEO_VC_GRADIENT) {
-#pragma unroll
-                for (int a = 0; a < ND; ++a) {
-                    const T d = D(V.t[a], M, a);
-                    T* y = out + n + a * V.ovol;
-                    *y = overwrite ? zero_fix(d) : *y + d;
-                }
-            } else if (KIND == DEO_VC_DIVERGENCE) {
-                T d[ND];
-#pragma unroll
-                for (int a = 0; a < ND; ++a) d[a] = D(V.t[a], M + a * V.pvol, a);
-                T acc = overwrite ? T(0) : out[n];
-                bool first = overwrite != 0;  // 0 + x is x up to the sign of zero
-#pragma unroll
-                for (int p = 0; p < 3; ++p)
-#pragma unroll
-                    for (int a = 0; a < ND; ++a)
-                        if (ph[a] == p) {
-                            acc = first ? zero_fix(d[a]) : acc + d[a];
-                            first = false;
-                        }
-                out[n] = acc;
-            } else {
-                // curl component c = (D_{a1} u[c1]) sign1 + (D_{a2} u[c2]) sign2, a1 < a2:
-                //   x1: +D2 u3, -D3 u2;  x2: -D1 u3, +D3 u1;  x3: +D1 u2, -D2 u1
-                constexpr int A1[3] = {1, 0, 0}, A2[3] = {2, 2, 1};
-                constexpr int C1[3] = {2, 2, 1}, C2[3] = {1, 0, 0};
-                constexpr bool N1[3] = {false, true, false}, N2[3] = {true, false, true};
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const int a1 = A1[c], a2 = A2[c];
-                    const T e1 = D(N1[c] ? V.tn[a1] : V.t[a1], M + C1[c] * V.pvol, a1);
-                    const T e2 = D(N2[c] ? V.tn[a2] : V.t[a2], M + C2[c] * V.pvol, a2);
-                    T* y = out + n + c * V.ovol;
-                    const T f = ph[a1] <= ph[a2] ? e1 : e2, g = ph[a1] <= ph[a2] ? e2 : e1;
-                    *y = (overwrite ? zero_fix(f) : *y + f) + g;
-                }
-            }
-        }
-    }
+    for (int64_t o1 = (int64_t)blockIdx.y * 8 + threadIdx.x / 32; o1 < n1; o1 += (int64_t)gridDim.y * 8)
+        for (int64_t o2 = blockIdx.z; o2 < n2; o2 += gridDim.z)
+            vc_point<T, KIND, ND>(V, M, out, overwrite, o0, o1, o2);
 }
 
 // The same methods for operators with a uniform interior band of NK taps.
@@ -236,6 +241,367 @@ __global__ void __launch_bounds__(256) k_vc_march(const VcDev V, const T* __rest
     }
 }
 
+// The same methods for Float64 on a 3-D array whose operators share a uniform
+// interior band of NK taps, in block fixed point (deo_bfp.cuh), marching along
+// axis 3 as deo_march.cu does: CTA = 32 x 4 threads over 64 x 8 outputs, a
+// thread 2 x 2 of them; each input component's plane (with the halo its own
+// derivatives need) is converted once and read from a shared-memory ring -- NK +
+// 1 planes for a component differentiated along axis 3, 2 for the others.  Points
+// whose bound fails in some derivative (the larger of the two nearest taps below
+// the threshold while the block has lost bits) are queued and evaluated by
+// vc_point at the end of the unit; points on boundary rows are units of their own.
+//
+// What bounds it: instruction issue, 253 a gradient point (39 multiply-adds, 45 to
+// load and convert 2.1 values, 39 to round and test three derivatives, the rest
+// addressing and control) at 48 %.  256^3, 4th order, against the per-point
+// FP64 kernel (15, 17 and 33 FP64 instructions a point at 2 per clock per SM):
+// gradient 546 -> 257 us, divergence 553 -> 446, curl 1086 -> 888.  1 or 4 rows a
+// thread 259 / 289 us; boundary points through the warps' queues instead of
+// units of their own 376 (one warp drains a tile's whole boundary row).
+template <int KIND, int NK>
+struct VfCfg {
+    static constexpr int NC = KIND == DEO_VC_GRADIENT ? 1 : 3;
+    static constexpr int MID = NK / 2, LH = MID - 1, RH = MID + 1;  // taps o + 1 - MID .. o + 1 + MID
+    static constexpr int PL = (LH + 1) / 2 * 2, PR = (RH + 1) / 2 * 2;  // x halo in whole pairs
+    static constexpr int TYT = 4, RY = 2, NTHR = 32 * TYT, TY = TYT * RY;
+    // does component c have a derivative along axis a
+    __host__ __device__ static constexpr bool has(int c, int a) {
+        return KIND == DEO_VC_GRADIENT ? true : (KIND == DEO_VC_DIVERGENCE ? c == a : c != a);
+    }
+    __host__ __device__ static constexpr int bx(int c) { return 64 + (has(c, 0) ? PL + PR : 0); }
+    __host__ __device__ static constexpr int by(int c) { return TY + (has(c, 1) ? LH + RH : 0); }
+    __host__ __device__ static constexpr int plane(int c) { return bx(c) * by(c); }
+    __host__ __device__ static constexpr int nld(int c) { return (plane(c) + NTHR - 1) / NTHR; }
+    __host__ __device__ static constexpr int slots(int c) { return has(c, 2) ? NK + 1 : 2; }
+    __host__ __device__ static constexpr int base(int c) { return c == 0 ? 0 : base(c - 1) + slots(c - 1) * plane(c - 1); }
+    static constexpr int QCAP = 1024;  // fallback points a warp can hold
+    static constexpr int SMEM = base(NC) * 8 + TYT * QCAP * 2;
+};
+
+template <int C>
+using Comp = std::integral_constant<int, C>;
+
+template <int KIND, int NK, bool OW>
+__global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
+    k_vc_fx(const __grid_constant__ VcDev V, const __grid_constant__ VcBfp B, const LapGrid g,
+            const double* __restrict__ M, double* __restrict__ out) {
+    using C = VfCfg<KIND, NK>;
+    constexpr int MID = C::MID, RY = C::RY, NC = C::NC;
+    extern __shared__ __align__(16) unsigned char smem[];
+    Limbs* ring = reinterpret_cast<Limbs*>(smem);
+    unsigned short* queue = reinterpret_cast<unsigned short*>(smem + C::base(NC) * 8) + threadIdx.y * C::QCAP;
+    __shared__ unsigned s_max[NC][16], s_min[NC][16];
+    __shared__ int s_next;
+    const int n0 = (int)V.len[0], n1 = (int)V.len[1], n2 = (int)V.len[2];
+    const int px = n0 + 2, py = n1 + 2, bpc = V.bpc;
+    const int64_t psz = (int64_t)px * py, osz = (int64_t)n0 * n1;
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * 32 + tx;
+    int nq = 0;
+    __shared__ int s_nq[C::TYT];
+    auto point = [&](int w, unsigned e, int x0, int y0, int z0) {  // a queued point of warp w
+        vc_point<double, KIND, 3, NK>(V, M, out, OW, x0 + (int)(e & 63u), y0 + w * RY + (int)((e >> 6) & 3u),
+                                      z0 + (int)(e >> 8));
+    };
+    auto drain = [&](int keep, int x0, int y0, int z0) {  // this warp's own, when its queue is nearly full
+        while (nq > keep) {
+            const int n = min(nq, 32);
+            nq -= n;
+            if (tx < n) point(ty, queue[nq + tx], x0, y0, z0);
+            __syncwarp();
+        }
+    };
+    // points with a boundary row: 1024 to a unit, before the others (axis 3's planes, then axis 2's rows and
+    // axis 1's columns between them)
+    const int iy = n1 - 2 * bpc, iz = n2 - 2 * bpc;
+    const int64_t ez = (int64_t)2 * bpc * n0 * n1, ey = (int64_t)2 * bpc * n0 * iz, ex = (int64_t)2 * bpc * iy * iz;
+    const int64_t etot = ez + ey + ex;
+    auto out_of = [&](int i, int n) { return i < bpc ? i : n - 2 * bpc + i; };  // the i-th boundary row of n
+    const int edge = (int)((etot + 1023) / 1024);
+    for (int k = claim_next(g.sched, s_next); k < g.units + edge; k = claim_next(g.sched, s_next)) {
+        if (k < edge) {
+            for (int64_t i = (int64_t)k * 1024 + tid; i < min((int64_t)(k + 1) * 1024, etot); i += C::NTHR) {
+                int64_t r = i;
+                int x, y, z;
+                if (r < ez) {
+                    z = (int)(r / osz);
+                    r -= z * osz;
+                    y = (int)(r / n0);
+                    x = (int)(r - (int64_t)y * n0);
+                    z = out_of(z, n2);
+                } else if ((r -= ez) < ey) {
+                    const int64_t l = r / n0;
+                    x = (int)(r - l * n0);
+                    z = bpc + (int)(l / (2 * bpc));
+                    y = out_of((int)(l % (2 * bpc)), n1);
+                } else {
+                    r -= ey;
+                    const int64_t l = r / iy;
+                    y = bpc + (int)(r - l * iy);
+                    z = bpc + (int)(l / (2 * bpc));
+                    x = out_of((int)(l % (2 * bpc)), n0);
+                }
+                vc_point<double, KIND, 3>(V, M, out, OW, x, y, z);
+            }
+            __syncthreads();  // s_next has been read by every thread
+            continue;
+        }
+        const int unit = k - edge;
+        const int txi = unit % g.tiles_x, rest = unit / g.tiles_x;
+        const int tyi = rest % g.tiles_y, ci = rest / g.tiles_y;
+        const int x0 = txi * 64, y0 = tyi * C::TY;
+        const int z0 = bpc + ci * g.zc, z1 = min(z0 + g.zc, n2 - bpc);
+        const int npl = z1 - z0 + 2 * MID;
+        // the component's values this thread loads: byte offsets in a plane
+        unsigned off[NC][C::nld(KIND == DEO_VC_DIVERGENCE ? 1 : NC - 1)];
+        double raw[NC][C::nld(KIND == DEO_VC_DIVERGENCE ? 1 : NC - 1)];
+        auto offsets = [&](auto cc) {
+            constexpr int c = decltype(cc)::value, BX = C::bx(c);
+#pragma unroll
+            for (int j = 0; j < C::nld(c); ++j) {
+                const int q = min(tid + j * C::NTHR, C::plane(c) - 1);
+                const int r = q / BX, x = x0 + (q - r * BX) - (C::has(c, 0) ? C::PL : 0);
+                const int y = y0 + r - (C::has(c, 1) ? C::LH : 0);
+                off[c][j] = 8u * (unsigned)(min(max(y, 0), py - 1) * px + min(max(x, 0), px - 1));
+            }
+        };
+        // the plane of component c that step p brings: o + 1 + MID for axis 3's window, else o itself
+        auto load = [&](auto cc, int p) {
+            constexpr int c = decltype(cc)::value;
+            const char* s = reinterpret_cast<const char*>(M + c * V.pvol) +
+                            (int64_t)(C::has(c, 2) ? z0 + 1 - MID + p : z0 + p - 2 * MID) * (psz * 8);
+#pragma unroll
+            for (int j = 0; j < C::nld(c); ++j) raw[c][j] = __ldg(reinterpret_cast<const double*>(s + off[c][j]));
+        };
+        int r6 = 0;  // p mod (NK + 1)
+        auto slot = [&](auto cc, int p, int back) {  // of step p - back, back <= NK
+            constexpr int c = decltype(cc)::value;
+            const int i = C::has(c, 2) ? (r6 - back < 0 ? r6 - back + NK + 1 : r6 - back) : ((p - back) & 1);
+            return ring + C::base(c) + i * C::plane(c);
+        };
+        auto put = [&](auto cc, int p, int back, int E, unsigned& mx, unsigned& mn) {
+            constexpr int c = decltype(cc)::value;
+            Limbs* w = slot(cc, p, back);
+            mx = 0;
+            mn = 0xffffffffu;
+#pragma unroll
+            for (int j = 0; j < C::nld(c); ++j) {
+                const unsigned key = bfp_key(raw[c][j]);
+                mx = max(mx, key);
+                mn = min(mn, key - 1u);
+                if (j + 1 < C::nld(c) || tid + j * C::NTHR < C::plane(c))
+                    w[tid + j * C::NTHR] = bfp_convert(raw[c][j], key, E);
+            }
+        };
+        auto each = [&](auto f) {
+            f(Comp<0>{});
+            if constexpr (NC == 3) {
+                f(Comp<1>{});
+                f(Comp<2>{});
+            }
+        };
+        unsigned live = 0;  // own points: interior rows on both axes
+#pragma unroll
+        for (int b = 0; b < 2 * RY; ++b) {
+            const int x = x0 + 2 * tx + (b & 1), y = y0 + ty * RY + b / 2;
+            if (x >= bpc && x < n0 - bpc && y >= bpc && y < n1 - bpc) live |= 1u << b;
+        }
+        const bool all_live = live == (1u << (2 * RY)) - 1u;
+        if (tid < 16)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+                s_max[c][tid] = 0;
+                s_min[c][tid] = 0xffffffffu;
+            }
+        each([&](auto cc) {
+            offsets(cc);
+            if constexpr (C::has(decltype(cc)::value, 2)) load(cc, 0);
+        });
+        __syncthreads();
+        int E[NC], low[NC];
+        unsigned inexact[NC];
+#pragma unroll
+        for (int c = 0; c < NC; ++c) E[c] = 64, low[c] = 0, inexact[c] = 0;
+        for (int p = 0; p < npl; ++p, r6 = r6 == NK ? 0 : r6 + 1) {
+            each([&](auto cc) {
+                constexpr int c = decltype(cc)::value;
+                if (C::has(c, 2) || p >= 2 * MID) {
+                    unsigned mx, mn;
+                    put(cc, p, 0, E[c], mx, mn);
+                    mx = __reduce_max_sync(0xffffffffu, mx);
+                    mn = __reduce_min_sync(0xffffffffu, mn);
+                    if (tx == 0) {
+                        atomicMax(&s_max[c][p & 15], mx);
+                        atomicMin(&s_min[c][p & 15], mn);
+                    }
+                }
+                if (p + 1 < npl && (C::has(c, 2) || p + 1 >= 2 * MID)) load(cc, p + 1);
+                if (tid == 0) {
+                    s_max[c][(p + 2) & 15] = 0;
+                    s_min[c][(p + 2) & 15] = 0xffffffffu;
+                }
+            });
+            __syncthreads();
+            each([&](auto cc) {  // a new exponent: the planes in use again (as in deo_march.cu)
+                constexpr int c = decltype(cc)::value, W = C::has(c, 2) ? NK : 1;
+                if (!C::has(c, 2) && p < 2 * MID) return;
+                const int ep = (int)(s_max[c][p & 15] >> 20);
+                low[c] = ep < E[c] ? low[c] + 1 : 0;
+                if (ep > E[c] || low[c] > W + 2) {
+                    int ew = 64;
+                    for (int b = 0; b < W && b <= p; ++b) ew = max(ew, (int)(s_max[c][(p - b) & 15] >> 20));
+                    low[c] = 0;
+                    if (ew != E[c]) {
+                        E[c] = ew;
+                        inexact[c] = ~0u;
+                        for (int b = min(W - 1, p); b >= 0; --b) {
+                            unsigned mx, mn;
+                            load(cc, p - b);
+                            put(cc, p, b, E[c], mx, mn);
+                        }
+                        if (p + 1 < npl) load(cc, p + 1);
+                        __syncthreads();
+                    }
+                }
+                inexact[c] = inexact[c] << 1 | (unsigned)(E[c] - (int)(s_min[c][p & 15] >> 20) > BFP_G);
+            });
+            if (p < 2 * MID) continue;
+            const int z = z0 + p - 2 * MID;
+            // a derivative of component c along axis a at the own points: its value and its distance
+            // from its fallback
+            auto taps = [&](auto cc, int a, const Limbs* t, double& d, int& far) {
+                constexpr int c = decltype(cc)::value;
+                BfpAcc s{0, 0, 0};
+                s.cr = (long long)B.wd[a][0] * t[MID].h;
+#pragma unroll
+                for (int o = 1; o <= MID; ++o) {
+                    bfp_mad(s, B.wh[a][o], B.wl[a][o], t[MID + o].h - t[MID - o].h, t[MID + o].l - t[MID - o].l);
+                    if (NK >= 7) s.cr += (long long)B.wd[a][o] * t[MID - o].h;
+                }
+                d = bfp_double(bfp_total(s), (B.kbase[a] + E[c]) * (1 << 20));
+                far = min(far, max(abs(t[MID - 1].h), abs(t[MID + 1].h)));
+            };
+            auto hl = [&](const int4& t, int w) { return w ? Limbs{t.z, t.w} : Limbs{t.x, t.y}; };
+            double d[2 * RY][3 * (KIND == DEO_VC_CURL ? 2 : 1)];  // GRADIENT, DIVERGENCE: [a]; CURL: [2 c + (first, second)]
+            int margin[2 * RY];  // below 0: some derivative's bound fails
+#pragma unroll
+            for (int b = 0; b < 2 * RY; ++b) margin[b] = INT_MAX;
+            each([&](auto cc) {
+                constexpr int c = decltype(cc)::value, BX = C::bx(c);
+                const Limbs* pc = slot(cc, p, C::has(c, 2) ? MID + 1 : 0);
+                const int own = (ty * RY + (C::has(c, 1) ? C::LH : 0)) * BX + (C::has(c, 0) ? C::PL : 0) + 2 * tx;
+                bool special = E[c] >= 2047, exact = !(inexact[c] & ((1u << (C::has(c, 2) ? NK : 1)) - 1u));
+#pragma unroll
+                for (int a = 0; a < 3; ++a) special |= C::has(c, a) && !bfp_range_ok(B.kbase[a] + E[c]);
+                const int t0 = special ? INT_MAX : (exact ? 0 : B.t0);
+                // where the derivative along axis a of this component goes
+                auto place = [&](int a) {
+                    // curl x1 = D2 u3 - D3 u2, x2 = -D1 u3 + D3 u1, x3 = D1 u2 - D2 u1
+                    return KIND == DEO_VC_CURL ? (c == 2 ? (a == 1 ? 0 : 2) : (c == 1 ? (a == 2 ? 1 : 4) : (a == 2 ? 3 : 5)))
+                                               : a;
+                };
+                int far[2 * RY];
+#pragma unroll
+                for (int b = 0; b < 2 * RY; ++b) far[b] = INT_MAX;
+                if constexpr (C::has(c, 0)) {
+#pragma unroll
+                    for (int j = 0; j < RY; ++j) {
+                        constexpr int NP = (C::PL + 2 + C::PR) / 2;
+                        int4 xs[NP];
+#pragma unroll
+                        for (int m = 0; m < NP; ++m)
+                            xs[m] = *reinterpret_cast<const int4*>(pc + own + j * BX - C::PL + 2 * m);
+#pragma unroll
+                        for (int v = 0; v < 2; ++v) {
+                            Limbs t[NK];
+#pragma unroll
+                            for (int m = 0; m < NK; ++m) {
+                                const int i = C::PL + v + 1 - MID + m;
+                                t[m] = hl(xs[i >> 1], i & 1);
+                            }
+                            taps(cc, 0, t, d[2 * j + v][place(0)], far[2 * j + v]);
+                        }
+                    }
+                }
+                if constexpr (C::has(c, 1)) {
+                    int4 yc[RY + 2 * MID];
+#pragma unroll
+                    for (int m = 0; m < RY + 2 * MID; ++m)
+                        yc[m] = *reinterpret_cast<const int4*>(pc + own + (m + 1 - MID) * BX);
+#pragma unroll
+                    for (int b = 0; b < 2 * RY; ++b) {
+                        Limbs t[NK];
+#pragma unroll
+                        for (int m = 0; m < NK; ++m) t[m] = hl(yc[b / 2 + m], b & 1);
+                        taps(cc, 1, t, d[b][place(1)], far[b]);
+                    }
+                }
+                if constexpr (C::has(c, 2)) {
+#pragma unroll
+                    for (int j = 0; j < RY; ++j) {
+                        int4 zs[NK];
+#pragma unroll
+                        for (int m = 0; m < NK; ++m)
+                            zs[m] = *reinterpret_cast<const int4*>(slot(cc, p, 2 * MID - m) + own + j * BX);
+#pragma unroll
+                        for (int v = 0; v < 2; ++v) {
+                            Limbs t[NK];
+#pragma unroll
+                            for (int m = 0; m < NK; ++m) t[m] = hl(zs[m], v);
+                            taps(cc, 2, t, d[2 * j + v][place(2)], far[2 * j + v]);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int b = 0; b < 2 * RY; ++b) margin[b] = min(margin[b], far[b] - t0);
+            });
+            const int64_t n = (int64_t)z * osz + (int64_t)(y0 + ty * RY) * n0 + x0 + 2 * tx;
+            auto store = [&](int b) {
+                double* y = out + n + (int64_t)(b / 2) * n0 + b % 2;
+                if constexpr (KIND == DEO_VC_GRADIENT) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) y[a * V.ovol] = OW ? d[b][a] : y[a * V.ovol] + d[b][a];
+                } else if constexpr (KIND == DEO_VC_DIVERGENCE) {
+                    *y = ((OW ? d[b][0] : *y + d[b][0]) + d[b][1]) + d[b][2];
+                } else {
+                    y[0] = (OW ? d[b][0] : y[0] + d[b][0]) - d[b][1];
+                    y[V.ovol] = (OW ? -d[b][2] : y[V.ovol] - d[b][2]) + d[b][3];
+                    y[2 * V.ovol] = (OW ? d[b][4] : y[2 * V.ovol] + d[b][4]) - d[b][5];
+                }
+            };
+            int least = all_live ? 0 : -1;
+#pragma unroll
+            for (int b = 0; b < 2 * RY; ++b) least = min(least, margin[b]);
+            if (__all_sync(0xffffffffu, least >= 0)) {
+#pragma unroll
+                for (int b = 0; b < 2 * RY; ++b) store(b);
+            } else {
+#pragma unroll
+                for (int b = 0; b < 2 * RY; ++b) {
+                    const bool on = (live >> b) & 1u, later = on && margin[b] < 0;
+                    if (on && !later) store(b);
+                    const unsigned bal = __ballot_sync(0xffffffffu, later);
+                    if (later)
+                        queue[nq + __popc(bal & ((1u << tx) - 1u))] =
+                            (unsigned short)((unsigned)(p - 2 * MID) << 8 | (unsigned)(b / 2) << 6 | (unsigned)(2 * tx + b % 2));
+                    nq += __popc(bal);
+                }
+                __syncwarp();
+                if (nq > C::QCAP - 64 * RY) drain(31, x0, y0, z0);
+            }
+        }
+        // the queues, shared out over the CTA
+        if (tx == 0) s_nq[ty] = nq;
+        __syncthreads();
+        nq = 0;
+        for (int w = 0, i = tid; w < C::TYT; ++w) {
+            for (; i < s_nq[w]; i += C::NTHR) point(w, (queue + (w - ty) * C::QCAP)[i], x0, y0, z0);
+            i -= s_nq[w];
+        }
+        __syncthreads();  // the next unit reuses the ring, the queues and the exponents
+    }
+    claims_done(g.sched);
+}
+
 // The generic per-line methods (vector_calculus_convolutions.jl:1-170): any N,
 // other axes read at index + 1, operators added in axis order.
 template <typename T, int KIND>
@@ -335,8 +701,33 @@ __global__ void __launch_bounds__(256) k_cross(int64_t npts, const T* __restrict
     u[n + 2 * npts] = sub_rn(mul_rn(a1, b2), mul_rn(a2, b1));
 }
 
+template <int KIND, int NK>
+int launch_fx(const VcDev& V, const VcBfp& B, unsigned int* claims, const double* M, double* out, int ow, cudaStream_t st) {
+    using C = VfCfg<KIND, NK>;
+    static int64_t G = 0;
+    if (!G) {
+        int e = occupancy_grid(k_vc_fx<KIND, NK, true>, C::NTHR, C::SMEM, G);
+        if (!e) e = occupancy_grid(k_vc_fx<KIND, NK, false>, C::NTHR, C::SMEM, G);
+        if (e) return e;
+    }
+    LapGrid g = march_chunks(V.len[0], V.len[1], (int)V.len[2] - 2 * V.bpc, 64, C::TY, NK / 2, G);
+    g.sched = claims;
+    const int grid = (int)std::min<int64_t>(G, g.units);
+    auto go = [&](auto kernel) { kernel<<<grid, dim3(32, C::TYT), C::SMEM, st>>>(V, B, g, M, out); };
+    if (ow) go(k_vc_fx<KIND, NK, true>);
+    else go(k_vc_fx<KIND, NK, false>);
+    return (int)cudaGetLastError();
+}
+
 template <typename T, int KIND, int ND>
-void launch_tiled(const VcDev& V, const T* M, T* out, int ow, cudaStream_t st) {
+int launch_tiled(const VcDev& V, const VcBfp& B, unsigned int* claims, const T* M, T* out, int ow, cudaStream_t st) {
+    if constexpr (ND == 3 && std::is_same<T, double>::value)
+        if (B.ok) switch (V.band_nk) {
+                case 3: return launch_fx<KIND, 3>(V, B, claims, M, out, ow, st);
+                case 5: return launch_fx<KIND, 5>(V, B, claims, M, out, ow, st);
+                case 7: return launch_fx<KIND, 7>(V, B, claims, M, out, ow, st);
+                default: break;
+            }
     // marching kernel: columns x chunks of the last axis within the grid limits
     const int64_t nm = V.len[ND - 1];
     const int64_t ncol1 = ND == 3 ? (V.len[1] + 7) / 8 : 1;
@@ -346,39 +737,38 @@ void launch_tiled(const VcDev& V, const T* M, T* out, int ow, cudaStream_t st) {
     int64_t zb = 4;
     while (zb < 32 && ncols * ((nm + 2 * zb - 1) / (2 * zb)) >= 8192) zb *= 2;
     while ((nm + zb - 1) / zb > 65535) zb *= 2;
-    // Float64 is FP64-bound either way and the per-point row-table kernel keeps
-    // the FP64 pipe busier (gradient 548 us against 624 us at 256^3), so the
-    // marching kernel serves Float32 only
+    // (2-D Float64: the per-point row-table kernel keeps the FP64 pipe busier than this one)
     if (V.band_nk > 0 && ncol1 <= 65535 && !std::is_same<T, double>::value) {
         const unsigned chunks = (unsigned)((nm + zb - 1) / zb);
         const dim3 grid = ND == 3 ? dim3((unsigned)((V.len[0] + 31) / 32), (unsigned)ncol1, chunks)
                                   : dim3((unsigned)((V.len[0] + 255) / 256), chunks, 1);
         const int z = (int)zb;
         switch (V.band_nk) {
-            case 3: k_vc_march<T, KIND, ND, 3><<<grid, 256, 0, st>>>(V, M, out, ow, z); return;
-            case 5: k_vc_march<T, KIND, ND, 5><<<grid, 256, 0, st>>>(V, M, out, ow, z); return;
-            case 7: k_vc_march<T, KIND, ND, 7><<<grid, 256, 0, st>>>(V, M, out, ow, z); return;
-            case 9: k_vc_march<T, KIND, ND, 9><<<grid, 256, 0, st>>>(V, M, out, ow, z); return;
+            case 3: k_vc_march<T, KIND, ND, 3><<<grid, 256, 0, st>>>(V, M, out, ow, z); return (int)cudaGetLastError();
+            case 5: k_vc_march<T, KIND, ND, 5><<<grid, 256, 0, st>>>(V, M, out, ow, z); return (int)cudaGetLastError();
+            case 7: k_vc_march<T, KIND, ND, 7><<<grid, 256, 0, st>>>(V, M, out, ow, z); return (int)cudaGetLastError();
+            case 9: k_vc_march<T, KIND, ND, 9><<<grid, 256, 0, st>>>(V, M, out, ow, z); return (int)cudaGetLastError();
             default: break;
         }
     }
     const int64_t n2 = ND == 3 ? V.len[2] : 1;
     dim3 grid((unsigned)((V.len[0] + 31) / 32), (unsigned)std::min<int64_t>((V.len[1] + 7) / 8, 65535),
               (unsigned)std::min<int64_t>(n2, 65535));
-    k_vc<T, KIND, ND, 0><<<grid, 256, 0, st>>>(V, M, out, ow);
+    k_vc<T, KIND, ND><<<grid, 256, 0, st>>>(V, M, out, ow);
+    return (int)cudaGetLastError();
 }
 
 template <typename T>
-int launch_vc(const VcDev& V, const void* Mv, void* outv, int ow, cudaStream_t st) {
+int launch_vc(const VcDev& V, const VcBfp& B, unsigned int* claims, const void* Mv, void* outv, int ow, cudaStream_t st) {
     const T* M = static_cast<const T*>(Mv);
     T* out = static_cast<T*>(outv);
     if (V.quirk && V.nd == 2) {
-        if (V.kind == DEO_VC_GRADIENT) launch_tiled<T, DEO_VC_GRADIENT, 2>(V, M, out, ow, st);
-        else launch_tiled<T, DEO_VC_DIVERGENCE, 2>(V, M, out, ow, st);
+        if (V.kind == DEO_VC_GRADIENT) return launch_tiled<T, DEO_VC_GRADIENT, 2>(V, B, claims, M, out, ow, st);
+        else return launch_tiled<T, DEO_VC_DIVERGENCE, 2>(V, B, claims, M, out, ow, st);
     } else if (V.quirk && V.nd == 3) {
-        if (V.kind == DEO_VC_GRADIENT) launch_tiled<T, DEO_VC_GRADIENT, 3>(V, M, out, ow, st);
-        else if (V.kind == DEO_VC_DIVERGENCE) launch_tiled<T, DEO_VC_DIVERGENCE, 3>(V, M, out, ow, st);
-        else launch_tiled<T, DEO_VC_CURL, 3>(V, M, out, ow, st);
+        if (V.kind == DEO_VC_GRADIENT) return launch_tiled<T, DEO_VC_GRADIENT, 3>(V, B, claims, M, out, ow, st);
+        else if (V.kind == DEO_VC_DIVERGENCE) return launch_tiled<T, DEO_VC_DIVERGENCE, 3>(V, B, claims, M, out, ow, st);
+        else return launch_tiled<T, DEO_VC_CURL, 3>(V, B, claims, M, out, ow, st);
     } else {
         const unsigned blocks = (unsigned)((V.ovol + 255) / 256);
         if (V.kind == DEO_VC_GRADIENT) k_vc_lines<T, DEO_VC_GRADIENT><<<blocks, 256, 0, st>>>(V, M, out, ow);
@@ -390,12 +780,12 @@ int launch_vc(const VcDev& V, const void* Mv, void* outv, int ow, cudaStream_t s
 }  // namespace
 }  // namespace deo
 
-extern "C" int deo_k_vector_calculus(const deo::VcDev* V, int dtype, const void* M, void* out, int overwrite,
-                                     void* stream) {
+extern "C" int deo_k_vector_calculus(const deo::VcDev* V, const deo::VcBfp* B, unsigned int* claims, int dtype,
+                                     const void* M, void* out, int overwrite, void* stream) {
     if (V->ovol <= 0) return 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return dtype == 0 ? deo::launch_vc<double>(*V, M, out, overwrite, st)
-                      : deo::launch_vc<float>(*V, M, out, overwrite, st);
+    return dtype == 0 ? deo::launch_vc<double>(*V, *B, claims, M, out, overwrite, st)
+                      : deo::launch_vc<float>(*V, *B, claims, M, out, overwrite, st);
 }
 
 extern "C" int deo_k_padded_apply(const deo::VcDev* V, int axis, int64_t coff, int dtype, const void* M, void* out,
