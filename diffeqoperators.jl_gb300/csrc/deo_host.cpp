@@ -2241,7 +2241,10 @@ struct deo_solve {
     double* d_b = nullptr;    // A_b
     double* d_rdiag = nullptr; // 1 / U[j][j]
     double* d_work = nullptr; // Float32 plans: the lines in Float64 while they are solved
+    int* d_meta = nullptr;
+    deo::BandLU lu{};
     ~deo_solve() {
+        if (d_meta) cudaFree(d_meta);
         if (d_rdiag) cudaFree(d_rdiag);
         if (d_ab) cudaFree(d_ab);
         if (d_ipiv) cudaFree(d_ipiv);
@@ -2401,6 +2404,47 @@ extern "C" deo_status deo_solve_plan(const deo_operator* op, const deo_bc* bc, i
     CUDA_TRY(cudaMalloc(&S->d_rdiag, rdiag.size() * sizeof(double)), "cudaMalloc(pivots)");
     CUDA_TRY(cudaMemcpy(S->d_rdiag, rdiag.data(), rdiag.size() * sizeof(double), cudaMemcpyHostToDevice), "cudaMemcpy");
     if (dtype == DEO_F32) CUDA_TRY(cudaMalloc(&S->d_work, (size_t)total * sizeof(double)), "cudaMalloc(workspace)");
+    // what each column really holds (boundary rows widen the band, interior rows use less of it), and the
+    // rows where A_b is not zero (k_band_solve_w; wider bands than its 16 use ipiv alone)
+    deo::BandLU& B = S->lu;
+    std::vector<int> meta(N, 0);
+    const int kv = kl + ku;
+    for (long j = 0; j < N; ++j) {
+        int nl = 0, nu = 0;
+        for (int r = 1; r <= kl && j + r < N; ++r)
+            if (AB[(size_t)(kv + r) * N + j] != 0.0) nl = r;
+        for (int r = 1; r <= kv && j - r >= 0; ++r)
+            if (AB[(size_t)(kv - r) * N + j] != 0.0) nu = r;
+        B.kb = std::max(B.kb, nu);
+        meta[j] = (ipiv[j] - (int)j) | std::min(nl, 255) << 8 | std::min(nu, 255) << 16;
+    }
+    int lo = 0, hi = (int)N;  // zero rows [lo, hi): the longest run around the middle
+    const int mid = (int)(N / 2);
+    if (Ab[mid] == 0.0) {
+        for (lo = mid; lo > 0 && Ab[lo - 1] == 0.0; --lo) {}
+        for (hi = mid + 1; hi < (int)N && Ab[hi] == 0.0; ++hi) {}
+    } else {
+        lo = hi = (int)N;
+    }
+    // the interior's columns, when they are all alike and of a pattern the kernel knows
+    const int pm = meta[mid], plain = 100 * (pm >> 8 & 255) + 10 * (pm >> 16 & 255) + (pm & 255);
+    if (plain == 110 || plain == 121 || plain == 220 || plain == 231) {
+        B.plain = plain;
+        for (B.plo = mid; B.plo > 0 && meta[B.plo - 1] == pm; --B.plo) {}
+        for (B.phi = mid + 1; B.phi < (int)N && meta[B.phi] == pm; ++B.phi) {}
+    }
+    CUDA_TRY(cudaMalloc(&S->d_meta, meta.size() * sizeof(int)), "cudaMalloc(column extents)");
+    CUDA_TRY(cudaMemcpy(S->d_meta, meta.data(), meta.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy");
+    B.n = S->n;
+    B.kl = kl;
+    B.ku = ku;
+    B.alo = lo;
+    B.ahi = hi;
+    B.ab = S->d_ab;
+    B.ipiv = S->d_ipiv;
+    B.meta = S->d_meta;
+    B.Ab = S->d_b;
+    B.rdiag = S->d_rdiag;
     *out = S.release();
     return DEO_OK;
 }
@@ -2416,8 +2460,7 @@ extern "C" deo_status deo_solve_apply(const deo_solve* s, const void* u, void* x
     if (!s || !u || !x) return fail(DEO_ERR_BAD_ARG, "null argument");
     const size_t es = s->dtype == DEO_F64 ? 8 : 4, bytes = (size_t)s->total * es;
     if (u != x && overlaps(u, bytes, x, bytes)) return fail(DEO_ERR_BAD_ARG, "x must be u itself or not overlap it");
-    const int e = deo_k_band_solve(s->n, s->kl, s->ku, s->d_ab, s->d_ipiv, s->d_b, s->d_rdiag, s->stride, s->nlines,
-                                   s->dtype, u, x, s->d_work, stream);
+    const int e = deo_k_band_solve(&s->lu, s->stride, s->nlines, s->dtype, u, x, s->d_work, stream);
     if (e) return cuda_fail((cudaError_t)e, "deo_solve_apply launch");
     return DEO_OK;
 }

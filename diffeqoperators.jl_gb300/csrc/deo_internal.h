@@ -293,12 +293,25 @@ extern "C" int deo_k_padded_apply(const deo::VcDev* V, int axis, int64_t coff, i
 extern "C" int deo_k_vector_algebra(int op, int dtype, int64_t npts, int ncomp, const void* A, const void* B, void* u,
                                     void* stream);
 
+// Banded LU factors of a line (device arrays), for deo_k_band_solve.
+namespace deo {
+struct BandLU {
+    int n, kl, ku;
+    int kb;           // the widest column of U above the diagonal
+    int alo, ahi;     // A_b is zero in the rows [alo, ahi)
+    int plain;        // 100 * multipliers + 10 * entries of U + interchange, of every column in [plo, phi)
+    int plo, phi;
+    const double* ab;     // [2 kl + ku + 1][n]
+    const int* ipiv;
+    const int* meta;      // per column: interchange | multipliers << 8 | entries of U above the diagonal << 16
+    const double* Ab;
+    const double* rdiag;  // reciprocal pivots
+};
+}  // namespace deo
 // Launcher implemented in deo_solve.cu: every line along an axis (stride, n
-// points) of u solved with the banded LU factors ab ([kl+ku+kl+1][n]), pivots
-// ipiv, reciprocal pivots rdiag and offset Ab: x = A_l^-1 (u - A_b).  x may be
-// u.  work: null for Float64 (x is the workspace), else total doubles.
-extern "C" int deo_k_band_solve(int n, int kl, int ku, const double* ab, const int* ipiv, const double* Ab,
-                                const double* rdiag, int64_t stride, int64_t nlines, int dtype, const void* u, void* x,
+// points) of u solved: x = A_l^-1 (u - A_b).  x may be u.  work: null for
+// Float64 (x is the workspace), else total doubles.
+extern "C" int deo_k_band_solve(const deo::BandLU* b, int64_t stride, int64_t nlines, int dtype, const void* u, void* x,
                                 double* work, void* stream);
 
 // Launchers implemented in deo_kernels.cu (return cudaError_t as int).
