@@ -16,7 +16,9 @@
 // below 2^-5 from the rest.  It is at most 2 ulp of the row's sum |w u| when
 // that sum is at least 2^52 units; the kernels test a lower bound of it (one
 // tap, or a sum of taps of one weight) and evaluate the points that fail in the
-// reference's order, unless no value of the block lost a bit.
+// reference's order, unless the whole block is zero.  (That no value of the
+// block lost a bit is not enough: a point whose only nonzero tap has a small
+// weight falls below the total's own unit.)
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -30,7 +32,7 @@ struct Limbs {
 };
 
 // hi word without sign, its lowest bit set when the low word is not zero: orders
-// values by exponent, and is zero only for a zero
+// values by exponent, and is zero for zeros alone
 __device__ __forceinline__ unsigned bfp_key(double v) {
     const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
     return (hi & 0x7fffffffu) | min(lo, 1u);
@@ -39,11 +41,15 @@ __device__ __forceinline__ unsigned bfp_key(double v) {
 // v in units of 2^(E - 1075 - BFP_G), truncated toward zero, as balanced limbs;
 // key: bfp_key(v).  E >= 64 and E >= v's exponent field (a larger one gives
 // garbage, no fault); a subnormal v then shifts out entirely.
+// G: bits kept below the mantissa of a value at the block's exponent.  BFP_G
+// where the kernel adds up to three values, or subtracts two, before the
+// product; 7 (|h| <= 2^30) where every value is multiplied by itself.
+template <int G = BFP_G>
 __device__ __forceinline__ Limbs bfp_convert(double v, unsigned key, int E) {
     const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
     const unsigned d = (unsigned)((E << 20) + 0xfffff - (int)key) >> 20;
     unsigned long long m = ((unsigned long long)((hi & 0xfffffu) | 0x100000u) << 32) | lo;
-    m <<= BFP_G;
+    m <<= G;
     asm("shr.u64 %0, %0, %1;" : "+l"(m) : "r"(d));  // (PTX clamps the amount)
     m += 1ull << 29;
     const int sg = ((int)hi >> 31) | 1;
@@ -63,10 +69,12 @@ __device__ __forceinline__ void bfp_mad(BfpAcc& a, int wh, int wl, int h, int l)
     a.cr += (long long)wl * h;
     a.ll += (long long)wl * l;
 }
-// The sum in units of 2^57 (below 2^62 in magnitude); ll enters by its high word.
+// The sum in units of 2^(51 + G) (below 2^62 in magnitude); ll enters by its high
+// word.
+template <int G = BFP_G>
 __device__ __forceinline__ long long bfp_total(const BfpAcc& a) {
     const long long cr = a.cr + (long long)(int)(a.ll >> 32) * 4;
-    return (a.hh << 3) + (cr >> 27);
+    return (a.hh << (9 - G)) + (cr >> (21 + G));
 }
 // t * 2^k (scale = 2^k; no nonzero t leaves the normal range, see bfp_range_ok).
 __device__ __forceinline__ double bfp_double(long long t, double scale) { return __ll2double_rn(t) * scale; }

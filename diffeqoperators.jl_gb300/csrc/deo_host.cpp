@@ -712,7 +712,11 @@ struct HostTab {
 
 // The table of rows i = 1..len given by `row(i)`.
 template <typename Row>
-static deo_status compile_rows(long len, Row row, HostTab& T, std::vector<int>& rlo, std::vector<int>& rhi) {
+static deo_status compile_rows(long len, Row make, HostTab& T, std::vector<int>& rlo, std::vector<int>& rhi) {
+    // built once where they fit a few MB (both passes below read every row)
+    std::vector<RowSpec> rows(len <= 16384 ? len : 0);
+    for (size_t i = 0; i < rows.size(); ++i) rows[i] = make((long)i + 1);
+    auto row = [&](long i) -> RowSpec { return rows.empty() ? make(i) : rows[i - 1]; };
     // pass 1: longest run of identical rows -> band
     long best_lo = 1, best_len = 0, run_lo = 1;
     RowSpec prev = row(1);
@@ -829,6 +833,7 @@ struct deo_plan {
     PlanDev dev{};
     deo::UniPlan uni{};
     deo::BfpMarch march{};      // 3-D Float64: the marching block fixed-point interior (ok = 0: not this plan)
+    deo::BfpPlan2 rows2{};      // 2-D Float64: the terms' rows in block fixed point (ok = 0: not this plan)
     int fx_rows_set = 0;        // DEO_OPT_FX_FP64_ROWS was set: the caller wants the per-point kernel's rows
     deo::ShellPlan shell{};
     int fast_path = 1;   // DEO_OPT_FAST_PATH
@@ -1154,6 +1159,163 @@ static bool same_bc(const deo_bc& a, const deo_bc& b) {
     return true;
 }
 
+// The rows of a 2-D Float64 plan in block fixed point (BfpPlan2): every row of an
+// axis -- the plain terms' rows added, their ghosts folded through the boundary
+// condition's map -- as a window of K points with weights W = round(w * 2^s) on the
+// row's own scale (the sum of |W| below 2^60).  A product of a ghost's
+// weight and its map's coefficient enters unrounded (hi + lo).  Declined (ok = 0,
+// DEO_OK) when a window is wider than 9 points (4 for the field term), reaches
+// outside its tile's halo, or a term is not of these kinds.
+struct FoldedRow {
+    static constexpr int R = 8;             // points i - R .. i + R
+    double hi[2 * R + 1], lo[2 * R + 1];    // a weight is hi + lo
+    double b;                               // the ghosts' constants
+    bool far;                               // a tap outside those points
+    void add(long at, double w) {           // at: point - (i - R); two-sum into (hi, lo)
+        if (w == 0.0) return;
+        if (at < 0 || at > 2 * R) {
+            far = true;
+            return;
+        }
+        const double s = hi[at] + w, t = s - hi[at];
+        lo[at] += (hi[at] - (s - t)) + (w - t);
+        hi[at] = s;
+    }
+    void product(long at, double w, double a) {
+        const double p = w * a;
+        add(at, p);
+        if (at >= 0 && at <= 2 * R) lo[at] += std::fma(w, a, -p);
+    }
+    // row i (0-based) of a term on a line of n points
+    void fold(const RowSpec& r, const deo_bc& q, long i, long n) {
+        const long o = R - i;
+        for (int k = 0; k < r.nk; ++k) {
+            const long p = r.p0 + k;  // 1-based padded position
+            if (p > 1 && p < n + 2) {
+                add(p - 2 + o, r.w[k]);
+            } else if (q.kind == DEO_BC_PERIODIC) {  // N-D: the edge planes themselves
+                add((p == 1 ? 0 : n - 1) + o, r.w[k]);
+            } else if (p == 1) {
+                for (int j = 0; j < q.m_l; ++j) product(j + o, r.w[k], q.a_l[j]);
+                b += r.w[k] * q.b_l;
+            } else {
+                for (int j = 0; j < q.m_r; ++j) product(n - q.m_r + j + o, r.w[k], q.a_r[j]);
+                b += r.w[k] * q.b_r;
+            }
+        }
+    }
+    bool window(long& first, long& last) const {  // its nonzero taps, relative to i - R
+        first = 2 * R + 1;
+        last = -1;
+        for (long k = 0; k <= 2 * R; ++k)
+            if (hi[k] != 0.0) {
+                first = std::min(first, k);
+                last = k;
+            }
+        return last >= 0 && !far && std::isfinite(b);
+    }
+};
+// One axis's rows as integer windows appended to the blob; false when a window
+// is too wide or reaches outside the halo.
+static bool pack_rows(const std::vector<FoldedRow>& rows, int K, int KP, int halo, std::vector<int>& blob, size_t& w_at,
+                      size_t& meta_at) {
+    const long n = (long)rows.size();
+    const int A = (K - 2) / 2, Z = K - 1 - A;
+    w_at = blob.size();
+    meta_at = w_at + (size_t)n * KP * 2;
+    blob.resize(meta_at + (size_t)n * 4, 0);
+    for (long i = 0; i < n; ++i) {
+        const FoldedRow& R = rows[i];
+        long lo, hi;
+        if (!R.window(lo, hi) || hi - lo + 1 > K) return false;
+        double sum = 0.0;
+        for (long k = lo; k <= hi; ++k) sum += std::fabs(R.hi[k]);
+        int s = 0;
+        if (!bfp_scale(sum, s)) return false;
+        lo += i - FoldedRow::R;
+        hi += i - FoldedRow::R;
+        const long q = std::max(std::min(std::max(i - (K - 1) / 2, hi - K + 1), std::min(lo, n - K)), 0L);
+        if (lo < q || hi >= q + K) return false;
+        // the tiles of 32 rows that hold row i (the last one starts at n - 32)
+        for (long t : {std::min(i / 32 * 32, n - 32), n - 32})
+            if (i >= t && (q < t - halo || q + K > t + 32 + halo)) return false;
+        long long W[9] = {0};
+        double total = 0.0;
+        for (long k = lo; k <= hi; ++k) {
+            const long at = k - i + FoldedRow::R;
+            W[k - q] = std::llrint(std::ldexp(R.hi[at], s)) + std::llrint(std::ldexp(R.lo[at], s));
+            total += std::fabs((double)W[k - q]);
+        }
+        int* w = &blob[w_at + (size_t)i * KP * 2];
+        for (int k = 0; k < K; ++k) split_limbs(W[k], w[2 * k], w[2 * k + 1]);
+        int* m = &blob[meta_at + (size_t)i * 4];  // BfpRowMeta
+        m[0] = (int)q;
+        m[1] = 58 - s - 1075 - 7;
+        m[2] = bfp_threshold(total, std::min(std::fabs((double)W[A]), std::fabs((double)W[Z])), 1.0);
+        m[3] = R.b != 0.0;
+    }
+    return true;
+}
+static deo_status build_rows2(deo_plan& P, const int64_t* sizes, int nterms, const deo_term* terms) {
+    deo::BfpPlan2 B{};
+    if (sizes[0] < 32 || sizes[1] < 32 || sizes[0] > (1 << 20) || (sizes[1] + 31) / 32 > 65535) return DEO_OK;
+    std::vector<FoldedRow> ax[2], f[2];
+    for (int t = 0; t < nterms; ++t) {
+        const deo_term& tm = terms[t];
+        const int a = tm.axis - 1, mode = tm.path == DEO_PATH_PADDED ? 1 : 0;
+        if (tm.line_bcs) return DEO_OK;
+        const long n = (long)sizes[a];
+        const deo_operator& op = *tm.op;
+        if (tm.coeff_field) {
+            if (!op.wind || a != 0 || B.field || op.stl > 4) return DEO_OK;
+            B.field = static_cast<const double*>(tm.coeff_field);
+            for (int v = 0; v < 2; ++v) {
+                f[v].resize(n);
+                for (long i = 0; i < n; ++i) {
+                    const RowSpec r = build_row(op, mode, false, v == 0 ? 1.0 : -1.0, i + 1);
+                    if (r.cidx != (int)i + 1) return DEO_OK;  // the field's value at the point itself
+                    f[v][i].fold(r, *tm.bc, i, n);
+                }
+            }
+        } else {
+            ax[a].resize(n);
+            for (long i = 0; i < n; ++i) ax[a][i].fold(build_row(op, mode, true, 1.0, i + 1), *tm.bc, i, n);
+        }
+    }
+    if (B.field && ax[0].empty()) return DEO_OK;  // (instantiated with plain terms along axis 1)
+    long wide = 0;
+    for (const auto& rows : ax)
+        for (const FoldedRow& R : rows) {
+            long lo, hi;
+            if (!R.window(lo, hi)) return DEO_OK;
+            wide = std::max(wide, hi - lo + 1);
+        }
+    if (wide > 9) return DEO_OK;
+    B.K = std::max(3, (int)(wide | 1));
+    B.n[0] = (int)sizes[0];
+    B.n[1] = (int)sizes[1];
+    const int hk = (B.K - 1) / 2, hx = B.field ? std::max(hk, 3) : hk;
+    std::vector<int> blob;
+    size_t at[4][2] = {};
+    for (int a = 0; a < 2; ++a)
+        if (!ax[a].empty() && !pack_rows(ax[a], B.K, B.K + 1, a == 0 ? hx : hk, blob, at[a][0], at[a][1])) return DEO_OK;
+    for (int v = 0; v < 2 && B.field; ++v)
+        if (!pack_rows(f[v], 4, 4, hx, blob, at[2 + v][0], at[2 + v][1])) return DEO_OK;
+    const void* d = nullptr;
+    const deo_status s = upload(P, blob, &d);
+    if (s != DEO_OK) return s;
+    auto rows = [&](int k) {
+        const int* base = static_cast<const int*>(d);
+        return deo::BfpRows{base + at[k][0], base + at[k][1]};
+    };
+    for (int a = 0; a < 2; ++a)
+        if (!ax[a].empty()) B.ax[a] = rows(a);
+    for (int v = 0; v < 2 && B.field; ++v) B.f[v] = rows(2 + v);
+    B.ok = 1;
+    P.rows2 = B;
+    return DEO_OK;
+}
+
 extern "C" deo_status deo_plan_create(int ndims, const int64_t* sizes, deo_dtype dtype, int nterms,
                                       const deo_term* terms, deo_plan** out) {
     return deo_plan_create_opts(ndims, sizes, dtype, nterms, terms, 0, out);
@@ -1477,6 +1639,10 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             U.enabled = 0;
         }
     }
+    if (ndims == 2 && dtype == DEO_F64 && flags == 0 && !P->uni.lap) {
+        const deo_status rs = build_rows2(*P, sizes, nterms, terms);
+        if (rs != DEO_OK) return rs;
+    }
     CUDA_TRY(cudaMalloc(&P->d_plan, sizeof(PlanDev)), "cudaMalloc(plan)");
     CUDA_TRY(cudaMemcpy(P->d_plan, &P->dev, sizeof(PlanDev), cudaMemcpyHostToDevice), "cudaMemcpy(plan)");
     if (P->march.ok) CUDA_TRY(P->claims.init(), "cudaMalloc(claim counters)");
@@ -1600,6 +1766,14 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     mark(p, 0, stream);
     if (use_march(p)) return launch_march(p, u, du, overwrite, stream);
+    if (p->rows2.ok && p->exact_sums == 1 && p->fast_path) {
+        const int e = deo_k_rows_fx(&p->rows2, p->d_plan, u, du, overwrite, stream);
+        p->last_kernel = "k_rows_fx";
+        p->last_kernel2 = "";
+        p->ev_launches = 1;
+        mark(p, 1, stream);
+        return e;
+    }
     if (p->uni.enabled && p->fast_path) {
         if (p->uni.lap && p->use_tma && deo_k_tma_ok(&p->uni, p->dev.dtype, u)) {
             // overlap only pays beside an interior kernel that leaves the FP64 pipe free: the fixed-point

@@ -265,6 +265,27 @@ struct VcDev {
     TermDev tn[3];
 };
 
+// 2-D Float64 plans in block fixed point (deo_rowsfx.cu): per row of an axis a
+// window of K points [q, q + K) (0-based; ghosts folded in) with integer weights
+// (limbs, KP = K + 1 of them, the last zero; KP = K = 4 for the field term), the
+// exponent k of its units (k + E scales the sum in units of 2^58), the threshold
+// t, and whether a ghost adds a constant (evaluated in the reference's order always).
+struct BfpRowMeta {
+    int q, k, t, always;
+};
+struct BfpRows {
+    const void* w;   // null: no term along the axis
+    const void* meta;
+};
+struct BfpPlan2 {
+    int ok;
+    int K;               // window of the plain terms (3, 5, 7, 9)
+    int n[2];
+    BfpRows ax[2];       // the plain terms of each axis, added
+    BfpRows f[2];        // the field term along axis 1 for coefficients >= 0 / < 0
+    const double* field; // or null
+};
+
 // The first-derivative band of each axis in block fixed point (deo_bfp.cuh), its
 // own scale per axis: a derivative in units of 2^57 times 2^(kbase[a] + E) is the
 // result.  The band is antisymmetric up to a few units: the limbs [o] multiply
@@ -373,6 +394,9 @@ extern "C" int deo_k_apply_vec(const deo::UniPlan* up, unsigned int* sched, cons
 // Float64 interior in block fixed point, marching along axis 3 (deo_march.cu)
 extern "C" int deo_k_apply_march(const deo::UniPlan* up, const deo::BfpMarch* B, unsigned int* sched, const void* u,
                                  void* du, int overwrite, void* stream);
+// A 2-D Float64 plan in block fixed point (deo_rowsfx.cu)
+extern "C" int deo_k_rows_fx(const deo::BfpPlan2* B, const deo::PlanDev* d_plan, const void* u, void* du, int overwrite,
+                             void* stream);
 extern "C" int deo_k_read_vec_status(unsigned int* status);
 // Device concretisation from the plan's tables (deo_concretize.cu): mode 0
 // dense, 1 banded (l, u; *flag set for an entry outside), 2 bandwidths into lu

@@ -57,18 +57,30 @@ struct Cfg {
     static_assert(RY <= 4 && QCAP >= 2 * 64 * RY, "a queued point is 8 bits of plane, 2 of row, 6 of x");
 };
 
-// One point in the reference's order, from global memory.
+// One point in the reference's order, from global memory; zeros, which come in
+// runs (beside a compact support), without FP64.
 template <int H>
 __device__ __forceinline__ double ref_point(const UniPlan& U, const double* __restrict__ u, int64_t idx, int64_t nx,
                                             int64_t sxy) {
     const int64_t st[3] = {1, nx, sxy};
+    double v[3][2 * H + 1];
+    unsigned any = 0;
+#pragma unroll
+    for (int t = 0; t < 3; ++t)
+#pragma unroll
+        for (int k = 0; k < 2 * H + 1; ++k) {
+            v[t][k] = u[idx + (k - H) * st[t]];
+            any |= bfp_key(v[t][k]);
+        }
     double total = 0.0;
+    if (__any_sync(__activemask(), any)) {
 #pragma unroll
-    for (int t = 0; t < 3; ++t) {
-        double acc = 0.0;
+        for (int t = 0; t < 3; ++t) {
+            double acc = 0.0;
 #pragma unroll
-        for (int k = 0; k < 2 * H + 1; ++k) acc = fma(U.t[t].w[k], u[idx + (k - H) * st[t]], acc);
-        total = t == 0 ? acc : total + acc;
+            for (int k = 0; k < 2 * H + 1; ++k) acc = fma(U.t[t].w[k], v[t][k], acc);
+            total = t == 0 ? acc : total + acc;
+        }
     }
     return zero_fix(total);
 }
@@ -82,7 +94,7 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
     extern __shared__ __align__(16) unsigned char smem[];
     Limbs* ring = reinterpret_cast<Limbs*>(smem);
     unsigned short* queue = reinterpret_cast<unsigned short*>(smem + S * C::SLOT * 8) + threadIdx.y * C::QCAP;
-    __shared__ unsigned s_max[16], s_min[16];  // of plane p at p & 15
+    __shared__ unsigned s_max[16];  // the largest key of plane p at p & 15
     __shared__ int s_next;
     const int nx = (int)U.n[0], ny = (int)U.n[1];
     const int64_t sxy = (int64_t)nx * ny;
@@ -136,46 +148,35 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
 #pragma unroll
             for (int j = 0; j < C::NLD; ++j) raw[j] = __ldg(reinterpret_cast<const double*>(s + off[j]));
         };
-        // the loaded plane on exponent E into a slot; its largest and smallest nonzero key
-        auto put = [&](Limbs* w, int E, unsigned& mx, unsigned& mn) {
-            mx = 0;
-            mn = 0xffffffffu;
+        // the loaded plane on exponent E into a slot; its largest key
+        auto put = [&](Limbs* w, int E) {
+            unsigned mx = 0;
 #pragma unroll
             for (int j = 0; j < C::NLD; ++j) {
                 const unsigned key = bfp_key(raw[j]);
                 mx = max(mx, key);
-                mn = min(mn, key - 1u);  // (a zero wraps to the largest value)
                 if (j + 1 < C::NLD || tid + j * C::NTHR < C::PLANE) w[tid + j * C::NTHR] = bfp_convert(raw[j], key, E);
             }
+            return mx;
         };
-        if (tid < 16) {
-            s_max[tid] = 0;
-            s_min[tid] = 0xffffffffu;
-        }
+        if (tid < 16) s_max[tid] = 0;
         load(0);
         __syncthreads();
         int E = 64;
         int low = 0;           // planes since one last reached E
-        unsigned inexact = 0;  // planes in use (bit 0 the newest) of which some value may have lost bits
+        int zeros = 0;         // planes since one last held anything but zeros
         int sl = 0;            // ring slot of plane p
         for (int p = 0; p < npl; ++p) {
             {
-                unsigned mx, mn;
-                put(ring + sl * C::SLOT, E, mx, mn);
+                const unsigned mx = __reduce_max_sync(0xffffffffu, put(ring + sl * C::SLOT, E));
                 if (p + 1 < npl) load(p + 1);
-                mx = __reduce_max_sync(0xffffffffu, mx);
-                mn = __reduce_min_sync(0xffffffffu, mn);
-                if (tx == 0) {
-                    atomicMax(&s_max[p & 15], mx);
-                    atomicMin(&s_min[p & 15], mn);
-                }
-                if (tid == 0) {
-                    s_max[(p + 2) & 15] = 0;
-                    s_min[(p + 2) & 15] = 0xffffffffu;
-                }
+                if (tx == 0) atomicMax(&s_max[p & 15], mx);
+                if (tid == 0) s_max[(p + 2) & 15] = 0;
             }
             __syncthreads();
-            const int ep = (int)(s_max[p & 15] >> 20);
+            const unsigned top = s_max[p & 15];
+            const int ep = (int)(top >> 20);
+            zeros = top == 0 ? zeros + 1 : 0;
             low = ep < E ? low + 1 : 0;
             if (ep > E || low > NQ + 2) {
                 // a new exponent: the planes in use (this one included) again
@@ -184,26 +185,22 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                 low = 0;
                 if (ew != E) {
                     E = ew;
-                    inexact = ~0u;
                     for (int b = min(NQ - 1, p); b >= 0; --b) {
-                        unsigned mx, mn;
                         load(p - b);
-                        put(ring + (sl - b < 0 ? sl - b + S : sl - b) * C::SLOT, E, mx, mn);
+                        put(ring + (sl - b < 0 ? sl - b + S : sl - b) * C::SLOT, E);
                     }
                     if (p + 1 < npl) load(p + 1);
                     __syncthreads();
                 }
             }
-            inexact = inexact << 1 | (unsigned)(E - (int)(s_min[p & 15] >> 20) > BFP_G);  // (key - 1: at most one binade below)
             const int cur = sl;
             sl = sl + 1 == S ? 0 : sl + 1;
             if (p < 2 * H) continue;
             const int kexp = B.kbase + E;
-            // thresholds of this plane: none when no value in use lost a bit, out of reach when the
-            // exponent rules fixed point out
+            // the threshold of this plane: none when everything in use is zero, out of reach when the exponent
+            // rules fixed point out
             const bool special = E >= 2047 || !bfp_range_ok(kexp);
-            const bool exact = !(inexact & ((1u << NQ) - 1u));
-            const int t0 = special ? INT_MAX : (exact ? 0 : B.t0);
+            const int t0 = special ? INT_MAX : (zeros >= NQ ? 0 : B.t0);
             const double scale = special ? 1.0 : bfp_pow2(kexp);
             const int4* pl[NQ];  // own pair of the first row in the planes z - H .. z + H
 #pragma unroll

@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(256) k_vc_march(const VcDev V, const T* __rest
 // derivatives need) is converted once and read from a shared-memory ring -- NK +
 // 1 planes for a component differentiated along axis 3, 2 for the others.  Points
 // whose bound fails in some derivative (the larger of the two nearest taps below
-// the threshold while the block has lost bits) are queued and evaluated by
+// the threshold) are queued and evaluated by
 // vc_point at the end of the unit; points on boundary rows are units of their own.
 //
 // What bounds it: instruction issue, 253 a gradient point (39 multiply-adds, 45 to
@@ -290,7 +290,7 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
     extern __shared__ __align__(16) unsigned char smem[];
     Limbs* ring = reinterpret_cast<Limbs*>(smem);
     unsigned short* queue = reinterpret_cast<unsigned short*>(smem + C::base(NC) * 8) + threadIdx.y * C::QCAP;
-    __shared__ unsigned s_max[NC][16], s_min[NC][16];
+    __shared__ unsigned s_max[NC][16];
     __shared__ int s_next;
     const int n0 = (int)V.len[0], n1 = (int)V.len[1], n2 = (int)V.len[2];
     const int px = n0 + 2, py = n1 + 2, bpc = V.bpc;
@@ -378,19 +378,18 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
             const int i = C::has(c, 2) ? (r6 - back < 0 ? r6 - back + NK + 1 : r6 - back) : ((p - back) & 1);
             return ring + C::base(c) + i * C::plane(c);
         };
-        auto put = [&](auto cc, int p, int back, int E, unsigned& mx, unsigned& mn) {
+        auto put = [&](auto cc, int p, int back, int E) {
             constexpr int c = decltype(cc)::value;
             Limbs* w = slot(cc, p, back);
-            mx = 0;
-            mn = 0xffffffffu;
+            unsigned mx = 0;
 #pragma unroll
             for (int j = 0; j < C::nld(c); ++j) {
                 const unsigned key = bfp_key(raw[c][j]);
                 mx = max(mx, key);
-                mn = min(mn, key - 1u);
                 if (j + 1 < C::nld(c) || tid + j * C::NTHR < C::plane(c))
                     w[tid + j * C::NTHR] = bfp_convert(raw[c][j], key, E);
             }
+            return mx;
         };
         auto each = [&](auto f) {
             f(Comp<0>{});
@@ -408,43 +407,32 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
         const bool all_live = live == (1u << (2 * RY)) - 1u;
         if (tid < 16)
 #pragma unroll
-            for (int c = 0; c < NC; ++c) {
-                s_max[c][tid] = 0;
-                s_min[c][tid] = 0xffffffffu;
-            }
+            for (int c = 0; c < NC; ++c) s_max[c][tid] = 0;
         each([&](auto cc) {
             offsets(cc);
             if constexpr (C::has(decltype(cc)::value, 2)) load(cc, 0);
         });
         __syncthreads();
-        int E[NC], low[NC];
-        unsigned inexact[NC];
+        int E[NC], low[NC], zeros[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) E[c] = 64, low[c] = 0, inexact[c] = 0;
+        for (int c = 0; c < NC; ++c) E[c] = 64, low[c] = 0, zeros[c] = 0;
         for (int p = 0; p < npl; ++p, r6 = r6 == NK ? 0 : r6 + 1) {
             each([&](auto cc) {
                 constexpr int c = decltype(cc)::value;
                 if (C::has(c, 2) || p >= 2 * MID) {
-                    unsigned mx, mn;
-                    put(cc, p, 0, E[c], mx, mn);
-                    mx = __reduce_max_sync(0xffffffffu, mx);
-                    mn = __reduce_min_sync(0xffffffffu, mn);
-                    if (tx == 0) {
-                        atomicMax(&s_max[c][p & 15], mx);
-                        atomicMin(&s_min[c][p & 15], mn);
-                    }
+                    const unsigned mx = __reduce_max_sync(0xffffffffu, put(cc, p, 0, E[c]));
+                    if (tx == 0) atomicMax(&s_max[c][p & 15], mx);
                 }
                 if (p + 1 < npl && (C::has(c, 2) || p + 1 >= 2 * MID)) load(cc, p + 1);
-                if (tid == 0) {
-                    s_max[c][(p + 2) & 15] = 0;
-                    s_min[c][(p + 2) & 15] = 0xffffffffu;
-                }
+                if (tid == 0) s_max[c][(p + 2) & 15] = 0;
             });
             __syncthreads();
             each([&](auto cc) {  // a new exponent: the planes in use again (as in deo_march.cu)
                 constexpr int c = decltype(cc)::value, W = C::has(c, 2) ? NK : 1;
                 if (!C::has(c, 2) && p < 2 * MID) return;
-                const int ep = (int)(s_max[c][p & 15] >> 20);
+                const unsigned top = s_max[c][p & 15];
+                const int ep = (int)(top >> 20);
+                zeros[c] = top == 0 ? zeros[c] + 1 : 0;
                 low[c] = ep < E[c] ? low[c] + 1 : 0;
                 if (ep > E[c] || low[c] > W + 2) {
                     int ew = 64;
@@ -452,17 +440,14 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
                     low[c] = 0;
                     if (ew != E[c]) {
                         E[c] = ew;
-                        inexact[c] = ~0u;
                         for (int b = min(W - 1, p); b >= 0; --b) {
-                            unsigned mx, mn;
                             load(cc, p - b);
-                            put(cc, p, b, E[c], mx, mn);
+                            put(cc, p, b, E[c]);
                         }
                         if (p + 1 < npl) load(cc, p + 1);
                         __syncthreads();
                     }
                 }
-                inexact[c] = inexact[c] << 1 | (unsigned)(E[c] - (int)(s_min[c][p & 15] >> 20) > BFP_G);
             });
             if (p < 2 * MID) continue;
             const int z = z0 + p - 2 * MID;
@@ -489,10 +474,11 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
                 constexpr int c = decltype(cc)::value, BX = C::bx(c);
                 const Limbs* pc = slot(cc, p, C::has(c, 2) ? MID + 1 : 0);
                 const int own = (ty * RY + (C::has(c, 1) ? C::LH : 0)) * BX + (C::has(c, 0) ? C::PL : 0) + 2 * tx;
-                bool special = E[c] >= 2047, exact = !(inexact[c] & ((1u << (C::has(c, 2) ? NK : 1)) - 1u));
+                bool special = E[c] >= 2047;
 #pragma unroll
                 for (int a = 0; a < 3; ++a) special |= C::has(c, a) && !bfp_range_ok(B.kbase[a] + E[c]);
-                const int t0 = special ? INT_MAX : (exact ? 0 : B.t0);
+                // none when everything in use is zero
+                const int t0 = special ? INT_MAX : (zeros[c] >= (C::has(c, 2) ? NK : 1) ? 0 : B.t0);
                 // where the derivative along axis a of this component goes
                 auto place = [&](int a) {
                     // curl x1 = D2 u3 - D3 u2, x2 = -D1 u3 + D3 u1, x3 = D1 u2 - D2 u1

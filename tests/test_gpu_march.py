@@ -29,6 +29,8 @@ def _field(kind, shape):
     elif kind == "zeros":  # a compact support: exact zeros beside values
         v[:, :, shape[2] // 2:] = 0.0
         v[: shape[0] // 3] = 0.0
+    elif kind == "sparse":  # points that see one small-weight tap, or nothing
+        v = np.where(rng.random(shape) < 0.03, np.round(4 * v), 0.0)
     elif kind == "wide":
         v = v * np.exp2(rng.integers(-40, 41, size=shape).astype(np.float64))
     elif kind == "special":
@@ -41,7 +43,7 @@ def _field(kind, shape):
     return np.asfortranarray(v)
 
 
-@pytest.mark.parametrize("field", ["normal", "waves", "zeros", "wide", "special", "tiny", "huge"])
+@pytest.mark.parametrize("field", ["normal", "waves", "zeros", "sparse", "wide", "special", "tiny", "huge"])
 @pytest.mark.parametrize("shape,a,one_band", [((64, 16, 20), 4, True), ((65, 17, 13), 4, False), ((131, 9, 40), 2, True),
                                               ((33, 24, 11), 6, False), ((130, 31, 12), 6, True), ((12, 11, 9), 2, False)])
 def test_march_against_oracle(cuda, shape, a, one_band, field):

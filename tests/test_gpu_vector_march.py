@@ -18,7 +18,7 @@ from test_gpu_vector import _dev, _host, _in_shape, _pair, KINDS
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("field", ["normal", "waves", "zeros", "wide", "special", "tiny", "huge"])
+@pytest.mark.parametrize("field", ["normal", "waves", "zeros", "sparse", "wide", "special", "tiny", "huge"])
 @pytest.mark.parametrize("kind,lens,a", [("gradient", (64, 8, 12), 4), ("gradient", (67, 17, 30), 2),
                                          ("gradient", (131, 9, 9), 6), ("divergence", (66, 10, 21), 4),
                                          ("divergence", (33, 19, 8), 2), ("curl", (20, 20, 20), 4),
@@ -33,6 +33,8 @@ def test_vector_march_against_oracle(cuda, kind, lens, a, field):
     elif field == "zeros":
         M[:, :, shape[2] // 2:] = 0.0
         M[: shape[0] // 3] = 0.0
+    elif field == "sparse":  # points that see one small-weight tap, or nothing
+        M = np.where(rng.random(shape) < 0.03, np.round(4 * M), 0.0)
     elif field == "wide":
         M = M * np.exp2(rng.integers(-40, 41, size=shape).astype(np.float64))
     elif field == "special":
