@@ -22,6 +22,7 @@ SOURCES = {
     "deo_vec.o": ("nvcc", "deo_vec.cu"),
     "deo_march.o": ("nvcc", "deo_march.cu"),
     "deo_rowsfx.o": ("nvcc", "deo_rowsfx.cu"),
+    "deo_nldfx.o": ("nvcc", "deo_nldfx.cu"),
     "deo_concretize.o": ("nvcc", "deo_concretize.cu"),
     "deo_shell.o": ("nvcc", "deo_shell.cu"),
     "deo_static.o": ("nvcc", "deo_static.cu"),

@@ -2077,11 +2077,57 @@ extern "C" deo_status deo_plan_host_sync(deo_plan* p) {
 // nonlinear_diffusion!: a plan over the order-1 .. (m+n) CenteredDifference
 // operators of the grid (term k-1 has order k), whose ghosts are read from the
 // padded inputs themselves (bc_kind 2), evaluated by the generic method.
+// Shortest line for k_nld_fx.  Below it both kernels are one chain of latencies: at
+// 2^16 points 2.9 to 7.6 us by the row tables over the orders built, 3.2 to 6.6 in
+// block fixed point (long bands gain, short ones lose); at 2^17 all gain
+// (4.1 .. 11.7 -> 3.7 .. 7.0).
+constexpr int kNldFxMinPoints = 1 << 17;
+
 struct deo_nld {
     deo_plan* plan = nullptr;
-    int n = 0, m = 0, len = 0;
+    int n = 0, m = 0, len = 0, a = 0;
+    deo::NldBfp bfp = {};
     ~deo_nld() { deo_plan_destroy(plan); }
 };
+
+// The derivatives' bands in block fixed point; ok stays 0 where one is not the
+// centred (anti)symmetric band of a uniform grid, or for an order that k_nld_fx is
+// not built for.
+static void nld_bands(deo_nld* N) {
+    deo::NldBfp& B = N->bfp;
+    const PlanDev& P = N->plan->dev;
+    if (P.dtype != DEO_F64 || N->n > 2 || N->m > 1 || (N->a != 2 && N->a != 4)) return;
+    if (N->len < kNldFxMinPoints || N->len > (1 << 30)) return;
+    B.lo = 0;
+    B.hi = N->len;
+    auto band = [&](int order, deo::NldBand& D, int& t0) {
+        const RowTabDev& tb = P.t[order - 1].tab[0];
+        const int H = (order + N->a - 1 + (order + N->a) % 2) / 2, K = 2 * H + 1;
+        if (tb.band_nk != K || tb.band_p0_off != 1 - H || H > 4) return false;
+        B.lo = std::max(B.lo, tb.ilo - 1);
+        B.hi = std::min(B.hi, tb.ihi);
+        double total = 0.0;
+        int s = 0, wh[DEO_MAX_NW], wl[DEO_MAX_NW];
+        if (!bfp_band(tb.wband, K, s, total, wh, wl)) return false;
+        auto W = [&](int o) { return ((long long)wh[H + o] << 30) + wl[H + o]; };
+        const bool odd = order % 2 == 1;
+        for (int o = 0; o <= H; ++o) {
+            const long long d = o == 0 ? (odd ? W(0) : 0) : (odd ? W(o) + W(-o) : W(-o) - W(o));
+            if (std::llabs(d) >= (1 << 20)) return false;
+            D.wh[o] = wh[H + o];
+            D.wl[o] = wl[H + o];
+            D.wd[o] = (int)d;
+        }
+        t0 = std::max(t0, bfp_threshold(total, (double)std::min(std::llabs(W(-1)), std::llabs(W(1))), 1.0));
+        D.k = 57 - s - 1075 - 6;
+        return true;
+    };
+    for (int k = N->m == 0 ? 1 : 0; k <= N->n; ++k)
+        if (!band(N->m + k, B.q[k], B.tq)) return;
+    for (int k = 1; k <= N->n; ++k)
+        if (!band(k, B.p[k - 1], B.tp)) return;
+    B.ok = 1;
+}
 
 extern "C" deo_status deo_nonlinear_diffusion_plan(int second_order, int first_order, int approx_order,
                                                    const double* dx, int dx_len, int nknots, deo_dtype dtype,
@@ -2113,6 +2159,8 @@ extern "C" deo_status deo_nonlinear_diffusion_plan(int second_order, int first_o
     N->n = second_order;
     N->m = first_order;
     N->len = nknots;
+    N->a = approx_order;
+    nld_bands(N.get());
     *out = N.release();
     return DEO_OK;
 }
@@ -2121,8 +2169,10 @@ extern "C" deo_status deo_nonlinear_diffusion(const deo_nld* nl, const void* p, 
                                               void* stream) {
     if (!nl || !p || !q || !du) return fail(DEO_ERR_BAD_ARG, "null argument");
     if (du == p || du == q) return fail(DEO_ERR_BAD_ARG, "du must not alias p or q");
-    const int e = deo_k_nonlinear_diffusion(&nl->plan->dev, nl->len, nl->n, nl->m, nl->plan->dev.dtype, p, q, du,
-                                            stream);
+    const int e = nl->bfp.ok
+                      ? deo_k_nld_fx(&nl->bfp, nl->plan->d_plan, nl->len, nl->n, nl->m, nl->a, p, q, du, stream)
+                      : deo_k_nonlinear_diffusion(&nl->plan->dev, nl->len, nl->n, nl->m, nl->plan->dev.dtype, p, q, du,
+                                                  stream);
     if (e) return cuda_fail((cudaError_t)e, "deo_nonlinear_diffusion launch");
     return DEO_OK;
 }

@@ -298,7 +298,27 @@ struct VcBfp {
     int kbase[3];
 };
 
+// One derivative of nonlinear_diffusion! in block fixed point: the limbs [o]
+// multiply x(+o) - x(-o) (odd orders) or x(+o) + x(-o) (even); wd[o] units, the
+// rest of W(-o), multiply x(-o) (wd[0]: an odd order's centre).  The result is in
+// units of 2^57 times 2^(k + E).
+struct NldBand {
+    int wh[5], wl[5], wd[5];
+    int k;
+};
+struct NldBfp {
+    int ok;
+    int lo, hi;  // outputs [lo, hi) have every derivative from its band
+    int tp, tq;  // derivatives of p / q are accepted when the larger of their two nearest taps' high limbs reaches this
+    NldBand p[2], q[3];  // p: orders 1 ..; q: orders m ..
+};
+
 }  // namespace deo
+
+// Launcher implemented in deo_nldfx.cu (orders n, m and approximation order a of
+// B; d_plan: the derivatives' tables in device memory).
+extern "C" int deo_k_nld_fx(const deo::NldBfp* B, const deo::PlanDev* d_plan, int len, int n, int m, int a,
+                            const void* p, const void* q, void* du, void* stream);
 
 // Launchers implemented in deo_vector.cu.  kind/nd/quirk come from V; out may
 // not overlap M.  overwrite = 1 writes A*M, 0 adds it to out (mul!).
