@@ -133,7 +133,24 @@ __device__ __forceinline__ const RowTabDev& row_variant(const TermDev& t, int64_
     return t.tab[0];
 }
 
-// One term, one output row: the reference's per-point tap loop.
+// n taps in chunks of 4, 2 and 1: f(first tap, the chunk's length as a constant).
+template <int N>
+struct Chunk {
+    __device__ constexpr operator int() const { return N; }
+};
+template <typename F>
+__device__ __forceinline__ void tap_chunks(int n, F f) {
+    int k = 0;
+    for (; k + 4 <= n; k += 4) f(k, Chunk<4>{});
+    if (n & 2) {
+        f(k, Chunk<2>{});
+        k += 2;
+    }
+    if (n & 1) f(k, Chunk<1>{});
+}
+
+// One term, one output row: the reference's per-point tap loop.  Float32 loads four taps
+// before their products: a boundary row is a chain of latencies.
 template <typename T, bool LBC = false>
 __device__ __forceinline__ T eval_term(const TermDev& t, const T* __restrict__ u, int64_t idx, int i) {
     const int64_t s = t.stride;
@@ -143,30 +160,37 @@ __device__ __forceinline__ T eval_term(const TermDev& t, const T* __restrict__ u
     const RowTabDev& tb = row_variant<T>(t, base, i, c);
     const RowInfo r = row_info(tb, i);
     const int L2 = t.len + 2;
-    // (the field and no-field loops are separate so that the common no-field
-    // rows issue no c * w multiply: a speculated one would double the FP64 work)
-    if (r.band && r.p0 >= 2 && r.p0 + r.nk <= L2) {
-        // band row away from the ghosts: straight tap loop (same order and rounding)
-        const T* __restrict__ xp = line + (int64_t)(r.p0 - 2) * s;
-        T acc = T(0);
-        if (t.has_field == 2) {  // DEO_PLAN_FACTOR_FIELD: c * (sum_k w_k x_k)
-            for (int k = 0; k < r.nk; ++k) acc = fma(band_w<T>(tb, k), __ldg(xp + (int64_t)k * s), acc);
-            acc = c * acc;
-        } else if (t.has_field) {
-            for (int k = 0; k < r.nk; ++k) acc = fma(c * band_w<T>(tb, k), __ldg(xp + (int64_t)k * s), acc);
-        } else {
-            for (int k = 0; k < r.nk; ++k) acc = fma(band_w<T>(tb, k), __ldg(xp + (int64_t)k * s), acc);
-        }
-        return acc;
-    }
     T gl = T(0), gr = T(0);
     if (r.p0 == 1) gl = ghost_left<T, LBC>(t, line, base);
     if (r.p0 + r.nk - 1 == L2) gr = ghost_right<T, LBC>(t, line, base);
+    T acc = T(0);
+    if constexpr (sizeof(T) == 4) {
+        tap_chunks(r.nk, [&](int k, auto n) {
+            T w[n], x[n];
+#pragma unroll
+            for (int m = 0; m < n; ++m) {
+                const int p = r.p0 + k + m;
+                const T v = __ldg(line + (int64_t)min(max(p - 2, 0), t.len - 1) * s);
+                w[m] = row_w<T>(tb, r, k + m);
+                x[m] = (p == 1) ? gl : (p == L2 ? gr : v);
+            }
+            if (t.has_field == 1) {
+#pragma unroll
+                for (int m = 0; m < n; ++m) acc = fma(c * w[m], x[m], acc);
+            } else {
+#pragma unroll
+                for (int m = 0; m < n; ++m) acc = fma(w[m], x[m], acc);
+            }
+        });
+        return t.has_field == 2 ? c * acc : acc;  // 2: DEO_PLAN_FACTOR_FIELD, c * (sum_k w_k x_k)
+    }
+    // Float64 in separate loops, tap by tap: a predicated-off FP64 instruction takes its
+    // turn in the pipe, which is what bounds these rows (a c * w issued for every row
+    // doubled their time; chunks of four cost 5 to 10 % more than they hid)
     auto tap = [&](int k) {
         const int p = r.p0 + k;
         return (p == 1) ? gl : (p == L2 ? gr : __ldg(line + (int64_t)(p - 2) * s));
     };
-    T acc = T(0);
     if (t.has_field == 2) {
         for (int k = 0; k < r.nk; ++k) acc = fma(row_w<T>(tb, r, k), tap(k), acc);
         acc = c * acc;
@@ -197,25 +221,24 @@ __device__ __forceinline__ T adj_column(const TermDev& t, const T* __restrict__ 
     const int64_t s = t.stride;
     const int lo = __ldg(t.rlo + (p - 1)), hi = __ldg(t.rhi + (p - 1));
     T acc = T(0);
-    if (!t.has_field) {
-        // column inside the band: the touching rows are exactly the band rows
-        // p - off - nk + 1 .. p - off; same row order as the general loop below
+    if (!t.has_field) {  // (no c * w multiply issued); the loads of four rows before their products
         const RowTabDev& tb = t.tab[0];
-        const int blo = p - tb.band_p0_off - tb.band_nk + 1, bhi = p - tb.band_p0_off;
-        if (lo == blo && hi == bhi && blo >= tb.ilo && bhi <= tb.ihi) {
-            for (int i = lo; i <= hi; ++i)
-                acc = fma(band_w<T>(tb, p - i - tb.band_p0_off), __ldg(d + base + (int64_t)(i - 1) * s), acc);
-            return acc;
-        }
-    }
-    if (!t.has_field) {  // (no c * w multiply issued, see eval_term)
-        const RowTabDev& tb = t.tab[0];
-        for (int i = lo; i <= hi; ++i) {
-            const RowInfo r = row_info(tb, i);
-            const int k = p - r.p0;
-            if (k < 0 || k >= r.nk) continue;
-            acc = fma(row_w<T>(tb, r, k), __ldg(d + base + (int64_t)(i - 1) * s), acc);
-        }
+        tap_chunks(max(hi - lo + 1, 0), [&](int o, auto n) {
+            T w[n], x[n];
+            bool in[n];
+#pragma unroll
+            for (int m = 0; m < n; ++m) {
+                const int i = lo + o + m;
+                const RowInfo r = row_info(tb, i);
+                const int k = p - r.p0;
+                in[m] = k >= 0 && k < r.nk;
+                w[m] = row_w<T>(tb, r, min(max(k, 0), r.nk - 1));
+                x[m] = __ldg(d + base + (int64_t)(i - 1) * s);
+            }
+#pragma unroll
+            for (int m = 0; m < n; ++m)
+                if (in[m]) acc = fma(w[m], x[m], acc);
+        });
         return acc;
     }
     for (int i = lo; i <= hi; ++i) {
@@ -271,6 +294,84 @@ __device__ __forceinline__ int term_row(const PlanDev& P, const TermDev& t, int6
     return (int)((idx / t.stride) % t.len) + 1;
 }
 
+// nk taps x[m * s] in the order of the general loops: weights w[m] (REV: w[nk - 1 - m]),
+// or w[m * ws], times c when SCALED.  NK > 0: unrolled, all loads before the chain of
+// products; 0: any length, four loads ahead.
+template <typename T, bool REV, bool ROWS, bool SCALED, int NK>
+__device__ __forceinline__ T straight_nk(const T* w, int64_t ws, const T* __restrict__ x, int64_t s, T c, int nk) {
+    T acc = T(0);
+    auto weight = [&](int m) {
+        const T v = ROWS ? __ldg(w + m * ws) : w[REV ? nk - 1 - m : m];
+        return SCALED ? c * v : v;
+    };
+    if constexpr (NK > 0) {
+        T v[NK];
+#pragma unroll
+        for (int m = 0; m < NK; ++m) v[m] = __ldg(x + m * s);
+#pragma unroll
+        for (int m = 0; m < NK; ++m) acc = fma(weight(m), v[m], acc);
+    } else {
+#pragma unroll 4
+        for (int m = 0; m < nk; ++m) acc = fma(weight(m), __ldg(x + m * s), acc);
+    }
+    return acc;
+}
+// Which lengths are unrolled: Float32 waits on its loads (all common lengths: 2048^2,
+// order 2, 45 -> 27 us), Float64 on the FP64 pipe, where the long bands lose by it what
+// the short ones gain (2048^2: 3 taps 70 -> 62 us, 9 taps 158 unrolled, 156 not; the
+// transposed bands 93 -> 87 at 5 taps).
+template <typename T, bool REV, bool ROWS, bool SCALED>
+__device__ __forceinline__ T straight(const T* w, int64_t ws, const T* __restrict__ x, int64_t s, T c, int nk) {
+    if constexpr (sizeof(T) == 8 && REV && !ROWS) {
+        return straight_nk<T, REV, ROWS, SCALED, 0>(w, ws, x, s, c, nk);
+    } else {
+        if (nk == 3) return straight_nk<T, REV, ROWS, SCALED, 3>(w, ws, x, s, c, 3);
+        if (nk == 5) return straight_nk<T, REV, ROWS, SCALED, 5>(w, ws, x, s, c, 5);
+        if constexpr (sizeof(T) == 4 || ROWS) {
+            if (nk == 7) return straight_nk<T, REV, ROWS, SCALED, 7>(w, ws, x, s, c, 7);
+            if (nk == 9) return straight_nk<T, REV, ROWS, SCALED, 9>(w, ws, x, s, c, 9);
+        }
+        return straight_nk<T, REV, ROWS, SCALED, 0>(w, ws, x, s, c, nk);
+    }
+}
+
+// eval_term / adj_term for any row: the straight loops where TermDev's ranges allow
+// them, bit for bit the same sums.  The general loops choose between band and explicit
+// row, ghost and line at every tap (40 instructions a tap) and look up p0, nk and the
+// touching rows at every point, also on graded lines, whose rows differ by their
+// weights alone.  2048^2 at 5 taps, apply / transposed: uniform Float64 97 / 90 ->
+// 94 / 87 us, Float32 49 / 52 -> 31 / 35; graded Float64 107 / 114 -> 90 / 90, Float32
+// 78 / 99 -> 34 / 40.
+template <typename T, bool ADJ, bool LBC>
+__device__ __forceinline__ T term_at(const TermDev& t, const T* __restrict__ u, int64_t idx, int i) {
+    const int64_t s = t.stride;
+    if constexpr (ADJ) {
+        if (i < t.sa_lo || i > t.sa_hi) return adj_term<T, LBC>(t, u, idx, i);
+        // rows i + 2 - s_off - s_nk + m, their taps nk - 1 - m
+        const T* __restrict__ x = u + idx + (2 - t.s_off - t.s_nk) * s;
+        if (t.s_rows) {
+            const T* w = reinterpret_cast<const T*>(t.tab[0].W) + (int64_t)(t.s_nk - 1) * t.tab[0].nexp +
+                         (i + 2 - t.s_off - t.s_nk + t.s_e0);
+            return straight<T, true, true, false>(w, 1 - t.tab[0].nexp, x, s, T(1), t.s_nk);
+        }
+        return straight<T, true, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0, x, s, T(1), t.s_nk);
+    } else {
+        if (i < t.sf_lo || i > t.sf_hi) return eval_term<T, LBC>(t, u, idx, i);
+        if (t.s_rows)
+            return straight<T, false, true, false>(reinterpret_cast<const T*>(t.tab[0].W) + (i + t.s_e0), t.tab[0].nexp,
+                                                   u + idx + (t.s_off - 1) * s, s, T(1), t.s_nk);
+        if (!t.has_field)
+            return straight<T, false, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0,
+                                                    u + idx + (t.s_off - 1) * s, s, T(1), t.s_nk);
+        const T c = __ldg(reinterpret_cast<const T*>(t.field) + idx + t.tab[0].band_cidx_off * s);
+        const RowTabDev& tb = t.nvar == 2 && not_nonneg(c) ? t.tab[1] : t.tab[0];
+        const T* w = reinterpret_cast<const T*>(tb.wband);
+        const T* __restrict__ x = u + idx + (tb.band_p0_off - 1) * s;
+        if (t.has_field == 2) return c * straight<T, false, false, false>(w, 0, x, s, T(1), tb.band_nk);
+        return straight<T, false, false, true>(w, 0, x, s, c, tb.band_nk);
+    }
+}
+
 template <typename T, bool ADJ, bool LBC = false>
 __device__ __forceinline__ T eval_point(const PlanDev& P, const T* __restrict__ u, int64_t idx) {
     if (!ADJ && P.star.n) {  // the merged star at points whose rows read no ghost along any axis
@@ -288,7 +389,7 @@ __device__ __forceinline__ T eval_point(const PlanDev& P, const T* __restrict__ 
     auto term = [&](int tt) {
         const TermDev& t = P.t[tt];
         const int i = term_row(P, t, idx);
-        return ADJ ? adj_term<T, LBC>(t, u, idx, i) : eval_term<T, LBC>(t, u, idx, i);
+        return term_at<T, ADJ, LBC>(t, u, idx, i);
     };
     T acc = term(0);  // the first term as is, then the others added left to right
     for (int tt = 1; tt < P.nterms; ++tt) acc = acc + term(tt);

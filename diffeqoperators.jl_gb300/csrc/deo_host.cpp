@@ -768,6 +768,30 @@ static deo_status compile_rows(long len, Row make, HostTab& T, std::vector<int>&
     return DEO_OK;
 }
 
+// Rows [lo, hi] of one shape: p0 = i + off, nk taps, weights from the band or (rows)
+// from entry i + e0 of the explicit rows, whichever range is longer.
+struct RowRange {
+    int lo = 1, hi = 0, off = 0, nk = 0, e0 = 0, rows = 0;
+    int size() const { return hi - lo + 1; }
+};
+static RowRange row_range(const HostTab& H) {
+    const RowTabDev& d = H.dev;
+    RowRange best, run;
+    if (d.ilo <= d.ihi) best = RowRange{d.ilo, d.ihi, d.band_p0_off, d.band_nk, 0, 0};
+    for (int e = 0; e < d.nexp; ++e) {
+        const int i = e + 1 < d.ilo ? e + 1 : e + 1 + (d.ihi - d.ilo + 1);
+        if (run.nk == H.nk[e] && run.off == H.p0[e] - i && run.hi == i - 1 && run.e0 == e - i) run.hi = i;
+        else run = RowRange{i, i, H.p0[e] - i, H.nk[e], e - i, 1};
+        if (run.size() > best.size()) best = run;
+    }
+    return best;
+}
+// The rows of R that read no ghost.
+static void straight_rows(const RowRange& R, int len, int& lo, int& hi) {
+    lo = std::max({lo, R.lo, 2 - R.off});
+    hi = std::min({hi, R.hi, len + 2 - R.nk - R.off});
+}
+
 static deo_status compile_table(const deo_operator& A, int mode, bool scaled, double sgn, HostTab& T,
                                 std::vector<int>& rlo, std::vector<int>& rhi) {
     return compile_rows(A.len, [&](long i) { return build_row(A, mode, scaled, sgn, i); }, T, rlo, rhi);
@@ -1466,6 +1490,9 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
         std::vector<const deo_operator*> members{&A};
         for (int m = t + 1; m < nterms; ++m)
             if (lead[m] == t) members.push_back(terms[m].op);
+        RowRange R;
+        T.sf_lo = 1;
+        T.sf_hi = A.len;
         for (int v = 0; v < T.nvar; ++v) {
             HostTab H;
             deo_status s;
@@ -1480,6 +1507,9 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             }
             if (s != DEO_OK) return s;
             if (v == 0) shell_rows(H, A.len, dtype, eff[t], P->shell);
+            R = row_range(H);
+            if (R.rows && T.has_field) R = RowRange{};
+            straight_rows(R, A.len, T.sf_lo, T.sf_hi);
             if ((s = upload_tab(*P, H, dtype, T.tab[v])) != DEO_OK) return s;
         }
         for (int p = 0; p < A.len + 2; ++p)
@@ -1503,6 +1533,25 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             T.lbc_stride = 5 + 2 * lmw;
             T.lbc_mw = lmw;
             D.has_lbc = 1;
+        }
+        T.s_off = R.off;
+        T.s_nk = R.nk;
+        T.s_e0 = R.e0;
+        T.s_rows = R.rows;
+        T.sa_lo = 1;
+        T.sa_hi = 0;
+        if (!T.has_field && R.nk > 0) {  // the longest run of columns touched by s_nk rows of R alone and by no ghost
+            const int gl = std::max({q.kind == DEO_BC_AFFINE ? T.ml : 1, T.lbc ? lmw : 0, T.lbc ? 1 : 0});
+            const int gr = std::max({q.kind == DEO_BC_AFFINE ? T.mr : 1, T.lbc ? lmw : 0, T.lbc ? 1 : 0});
+            int run = 0;
+            for (int j = 1 + gl; j <= A.len - gr; ++j) {
+                const int b1 = j + 1 - R.off, b0 = b1 - R.nk + 1;
+                run = b0 >= R.lo && b1 <= R.hi && rlo[j] == b0 && rhi[j] == b1 ? run + 1 : 0;
+                if (run > T.sa_hi - T.sa_lo + 1) {
+                    T.sa_hi = j;
+                    T.sa_lo = j - run + 1;
+                }
+            }
         }
         if (eff[t] < 3) {
             deo::ShellTerm& S = P->shell.t[eff[t]];
@@ -2867,7 +2916,8 @@ extern "C" deo_status deo_apply_each(int n, const deo_instance* in, int adjoint,
 }
 
 static deo_status batch_launch(deo_batch& b, cudaStream_t st) {
-    const int e = b.kind == 1
+    const int e = b.kind == 1 && b.plans.size() == 1 ? deo_k_stage_one(&b.plans[0]->dev, &b.stages[0], st)
+                  : b.kind == 1
                       ? deo_k_stage_batch(b.d_stages, b.d_items, b.n_items, b.d_counter, b.lbc, b.dtype, b.ctas, 256,
                                           st)
                       : deo_k_batch(b.d_inst, b.d_items, b.n_items, b.d_counter, b.dtype, b.adjoint, b.lbc, b.ctas,

@@ -58,6 +58,12 @@ struct TermDev {
     FastDiv div_len;
     int nvar;            // 1, or 2 for an upwind operator with a coefficient field (c>=0 / c<0)
     int has_field;       // 0: none; 1: row i = sum_k (c_i w_k) u_k; 2: c_i * sum_k w_k u_k (forward)
+    // Rows [sf_lo, sf_hi] of the straight tap loop: s_nk taps from p0 = i + s_off that
+    // read no ghost, weights from the band (each variant its own band's offsets) or,
+    // s_rows = 1 (no field), from entry i + s_e0 of tab[0].W.  Columns [sa_lo, sa_hi] of
+    // its transpose: touched by s_nk rows of that form and by no ghost (no field).
+    int sf_lo, sf_hi, sa_lo, sa_hi;
+    int s_off, s_nk, s_e0, s_rows;
     const void* field;   // coefficient field (same shape/dtype as u) or null
     RowTabDev tab[2];
     // adjoint: rows touching padded column p (1..len+2) lie in [rlo[p-1], rhi[p-1]]
@@ -424,6 +430,7 @@ extern "C" int deo_k_concretize(const deo::PlanDev* p, int mode, double* A, doub
                                 unsigned long long* lu, int* flag, void* stream);
 // 1 if deo_k_apply_tma can run on u (tensor-map alignment rules).
 extern "C" int deo_k_tma_ok(const deo::UniPlan* up, int dtype, const void* u);
+extern "C" int deo_k_stage_one(const deo::PlanDev* plan, const deo::StageDev* stage, void* stream);
 extern "C" int deo_k_stage_batch(const deo::StageDev* st, const deo::WorkItem* items, int64_t n_items,
                                  unsigned int* counter, int lbc, int dtype, int ctas_per_sm, int threads,
                                  void* stream);

@@ -20,13 +20,13 @@
 
 namespace deo {
 
-// The forward evaluator without per-line BCs is held to the registers of a
-// full SM: Float64 at 32 (eight CTAs, 64 warps, against five at its natural
-// 44, with a few hundred bytes of spills: its FP64 chains wait on loads and on
-// the FP64 pipe, and the extra warps cover that: 0.219 -> 0.203 ms on the
-// 2048^2 non-uniform sum), Float32 at 40 (six CTAs, no spills).
+// The forward evaluator without per-line BCs is held to the 32 registers of a full
+// SM (eight CTAs, 64 warps) with a few hundred bytes of spills: its chains wait on
+// loads and, in Float64, on the FP64 pipe, and the extra warps cover that.  2048^2,
+// order 2: Float64 62 us against 66 with five CTAs and 72 with four; Float32 27
+// against 31 (six) and 39 (four).
 template <typename T, bool ADJ, bool LBC>
-__global__ void __launch_bounds__(256, (!ADJ && !LBC) ? (sizeof(T) == 8 ? 8 : 6) : 0)
+__global__ void __launch_bounds__(256, !ADJ && !LBC ? 8 : 0)
     k_apply(const __grid_constant__ PlanDev P, const T* __restrict__ u, T* __restrict__ du, int overwrite) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= P.total) return;
@@ -141,6 +141,33 @@ __global__ void __launch_bounds__(256) k_stage(const StageDev* __restrict__ st, 
         });
 }
 
+// A stage of a single instance: the plan in the launch's parameters and a plain grid,
+// two points a thread, five CTAs a SM.  The work-list kernel spends a third of such a
+// stage on the claim, the list and the staged plan, each a trip to L2 before the first
+// point, and its 64 registers leave half of the warps that hide the points' own
+// loads.  768 x 500 Float64, 3 terms: 26 -> 17.5 us a stage; 100 x 50: 9 -> 7.
+// (One point a thread with six CTAs the same; four CTAs 22.)
+constexpr int STAGE_PT = 2;
+template <typename T, bool ADJ, bool LBC>
+__global__ void __launch_bounds__(256, 5)
+    k_stage_one(const __grid_constant__ PlanDev P, const __grid_constant__ StageDev S) {
+    const T* a = reinterpret_cast<const T*>(S.a);  // may alias out
+    const T* b = reinterpret_cast<const T*>(S.b);
+    const T* __restrict__ c = reinterpret_cast<const T*>(S.c);
+    T* out = reinterpret_cast<T*>(S.out);
+    const T al = T(S.alpha), be = T(S.beta), ga = T(S.gamma), dt = T(S.dt);
+#pragma unroll 1
+    for (int m = 0; m < STAGE_PT; ++m) {
+        const int64_t idx = ((int64_t)blockIdx.x * STAGE_PT + m) * 256 + threadIdx.x;
+        if (idx >= P.total) return;
+        const T f = eval_point<T, ADJ, LBC>(P, c, idx);
+        const T t = fma(dt, f, c[idx]);
+        T acc = a ? al * a[idx] : T(0);
+        if (b) acc = fma(be, b[idx], acc);
+        out[idx] = fma(ga, t, acc);
+    }
+}
+
 }  // namespace deo
 
 using namespace deo;
@@ -204,7 +231,7 @@ extern "C" int deo_k_scale(void* x, int64_t n, int dtype, double f, void* stream
 // CTA, of 256 points (one per thread) at the least for the default 8192-point
 // items.  One 768 x 500 Float64 state (47 items) then runs on every SM instead
 // of 47: 97 -> 31 us per Runge-Kutta stage; 256 mixed instances (1100 items)
-// forward + transposed 705 -> 565 us.
+// forward + transposed 705 -> 565 us (487 with the straight loops of deo_eval.cuh).
 static int split_for(int64_t n_items, int64_t ctas) {
     int lsplit = 0;
     while (lsplit < 5 && (n_items << lsplit) < 8 * ctas) ++lsplit;
@@ -223,6 +250,21 @@ extern "C" int deo_k_stage_batch(const StageDev* st, const WorkItem* items, int6
     auto go = [&](auto kernel) { kernel<<<(unsigned)grid, threads, 0, s>>>(st, items, n_items, lsplit, counter); };
     if (dtype == 0) lbc ? go(k_stage<double, true>) : go(k_stage<double, false>);
     else lbc ? go(k_stage<float, true>) : go(k_stage<float, false>);
+    return (int)cudaGetLastError();
+}
+
+extern "C" int deo_k_stage_one(const PlanDev* p, const StageDev* S, void* stream) {
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const int64_t blocks = (p->total + 256 * STAGE_PT - 1) / (256 * STAGE_PT);
+    if (blocks == 0) return 0;
+    auto go = [&](auto kernel) { kernel<<<(unsigned)blocks, 256, 0, st>>>(*p, *S); };
+    if (p->dtype == 0) {
+        if (p->has_lbc) S->adjoint ? go(k_stage_one<double, true, true>) : go(k_stage_one<double, false, true>);
+        else S->adjoint ? go(k_stage_one<double, true, false>) : go(k_stage_one<double, false, false>);
+    } else {
+        if (p->has_lbc) S->adjoint ? go(k_stage_one<float, true, true>) : go(k_stage_one<float, false, true>);
+        else S->adjoint ? go(k_stage_one<float, true, false>) : go(k_stage_one<float, false, false>);
+    }
     return (int)cudaGetLastError();
 }
 
