@@ -838,6 +838,11 @@ constexpr unsigned int kSchedSlots = 1024;
 // integer-pipe rows
 constexpr int kFxFp64Rows = 2;
 
+// k_rows_fx from here on.  Below, the generic kernel has less latency: graded, order 2
+// / 4, generic against k_rows_fx, 512 x 300 5.7 / 7.6 against 10.6 / 11.3 us, 1000 x
+// 700 14.1 / 19.8 against 13.5 / 15.5, 4000 x 3000 183 / 270 against 105 / 126.
+constexpr int64_t kRowsFxMinPoints = 1 << 19;
+
 // Rotating claim counters of the marching kernels: two words each, zeroed here
 // once and left zero by every launch (claims_done in deo_lap.cuh).
 struct ClaimSlots {
@@ -863,6 +868,7 @@ struct deo_plan {
     int fast_path = 1;   // DEO_OPT_FAST_PATH
     int use_tma = 1;     // DEO_OPT_TMA
     int exact_sums = 1;  // DEO_OPT_EXACT_SUMS
+    int sums_set = 0;    // DEO_OPT_EXACT_SUMS was set: its kernels at every size
     int timing = 0;      // DEO_OPT_LAUNCH_TIMING
     int concurrent = 1;  // DEO_OPT_CONCURRENT_SHELL
     // the last deo_plan_autotune: per candidate (f32_vec, vcfg, shell kernel, concurrent) its best ms
@@ -1688,7 +1694,7 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             U.enabled = 0;
         }
     }
-    if (ndims == 2 && dtype == DEO_F64 && flags == 0 && !P->uni.lap) {
+    if (ndims == 2 && dtype == DEO_F64 && flags == 0 && (!P->uni.lap || total >= kRowsFxMinPoints)) {
         const deo_status rs = build_rows2(*P, sizes, nterms, terms);
         if (rs != DEO_OK) return rs;
     }
@@ -1763,9 +1769,25 @@ static void mark(const deo_plan* p, int k, void* stream) {
 // (deo_march.cu) by default, whatever the alignment; the options that ask for
 // another variant, the FP64 rows of the per-point kernel or the TMA kernels'
 // wait test keep theirs.
-static bool use_march(const deo_plan* p) {
+// An odd first size has no tiled kernel to compare with but the generic one, whose
+// single launch is ahead on small arrays: order 2 / 4, generic against marching,
+// 33^3 6 / 9 against 11 / 13 us, 65^3 12.6 / 18.1 against 13.9 / 18.6, 97^3 29 / 43
+// against 20 / 32; transposed 97^3 26.5 / 43.4 against 28.4 / 44.9.  Even sizes march
+// at every size (tiled kernels before: 16^3 18 us against 9, 64^3 21 against 12).
+constexpr int64_t kMarchMinOddPoints = 300000, kMarchMinOddAdjoint = 1 << 20;
+static bool use_march(const deo_plan* p, bool adjoint = false) {
     return p->march.ok && p->exact_sums == 1 && p->fast_path && p->use_tma && !p->fx_rows_set &&
-           !p->uni.test_withhold;
+           !p->uni.test_withhold &&
+           (p->sums_set || p->dev.sizes[0] % 2 == 0 ||
+            p->dev.total >= (adjoint ? kMarchMinOddAdjoint : kMarchMinOddPoints));
+}
+// 2-D Float64 Laplacians by default: k_rows_fx, or the generic kernel below its size;
+// of the tiled kernels, which split such a plan into an interior and a shell launch,
+// only that of one shared band stays there.  Unequal steps, order 4, tiled against
+// now: 512 x 300 21 -> 7.5 us, 1000 x 700 38 -> 16, 4000 x 3000 280 -> 125; transposed
+// (generic) 21 -> 7, 37 -> 19, 279 -> 242.
+static bool plain_2d(const deo_plan* p) {
+    return p->dev.ndims == 2 && p->dev.dtype == DEO_F64 && p->exact_sums == 1 && !p->sums_set && !p->uni.fx;
 }
 static unsigned int* next_sched(const deo_plan* p) {
     return p->d_sched ? p->d_sched + (p->sched_slot.fetch_add(1) % kSchedSlots) : nullptr;
@@ -1815,7 +1837,8 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     mark(p, 0, stream);
     if (use_march(p)) return launch_march(p, u, du, overwrite, stream);
-    if (p->rows2.ok && p->exact_sums == 1 && p->fast_path) {
+    if (p->rows2.ok && p->exact_sums == 1 && p->fast_path && p->use_tma &&
+        (p->sums_set ? !p->uni.lap : p->dev.total >= kRowsFxMinPoints)) {
         const int e = deo_k_rows_fx(&p->rows2, p->d_plan, u, du, overwrite, stream);
         p->last_kernel = "k_rows_fx";
         p->last_kernel2 = "";
@@ -1824,7 +1847,7 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
         return e;
     }
     if (p->uni.enabled && p->fast_path) {
-        if (p->uni.lap && p->use_tma && deo_k_tma_ok(&p->uni, p->dev.dtype, u)) {
+        if (p->uni.lap && p->use_tma && !plain_2d(p) && deo_k_tma_ok(&p->uni, p->dev.dtype, u)) {
             // overlap only pays beside an interior kernel that leaves the FP64 pipe free: the fixed-point
             // kernel (Float64) or any Float32 kernel; the FP64-bound interiors run the shell after them
             const bool fx = p->dev.dtype == DEO_F64 &&
@@ -1893,6 +1916,7 @@ extern "C" deo_status deo_plan_set_option(deo_plan* p, int option, int value) {
         case DEO_OPT_EXACT_SUMS:
             if (value < 0 || value > 5) return fail(DEO_ERR_BAD_ARG, "exact-sums variant %d not in 0..5", value);
             p->exact_sums = value;
+            p->sums_set = 1;
             return DEO_OK;
         case DEO_OPT_CONCURRENT_SHELL: p->concurrent = value ? 1 : 0; return DEO_OK;
         case DEO_OPT_FX_FP64_ROWS:
@@ -2001,7 +2025,7 @@ static void reverse_taps(E* w, int n) {
 }
 
 static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwrite, void* stream) {
-    if (p->adj_ok && use_march(p)) {
+    if (p->adj_ok && use_march(p, true)) {
         deo::UniPlan ua = p->uni;
         deo::BfpMarch B = p->march;
         const int K = 2 * ua.radius + 1;
@@ -2021,7 +2045,7 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
         p->last_kernel2 = "k_shell_adj";
         return 0;
     }
-    if (p->adj_ok && p->uni.enabled && p->uni.lap && p->fast_path && p->use_tma &&
+    if (p->adj_ok && p->uni.enabled && p->uni.lap && p->fast_path && p->use_tma && !plain_2d(p) &&
         deo_k_tma_ok(&p->uni, p->dev.dtype, d)) {
         deo::UniPlan ua = p->uni;
         const int K = 2 * ua.radius + 1;
@@ -2236,6 +2260,7 @@ struct deo_vc {
     deo::VcDev dev{};
     deo::VcBfp bfp{};  // 3-D Float64 with a uniform band: block fixed point (ok = 0: not this plan)
     mutable ClaimSlots claims;
+    int64_t march_min = 0;  // points from which bfp is used
     int dtype = 0;
     int ncomp_in = 1, ncomp_out = 1;
 };
@@ -2327,6 +2352,12 @@ extern "C" deo_status deo_vector_calculus_plan(int kind, int ndims, const deo_op
             V->bfp.kbase[a] = 57 - s - 1075 - 6;
         }
         if (V->bfp.ok) CUDA_TRY(V->claims.init(), "cudaMalloc(claim counters)");
+        // k_vc_fx from here on (units of 64 x 8 columns and their queues want a full chip):
+        // gradient, order 2 / 4, k_vc against k_vc_fx: 80^3 16 / 23 against 17 / 33 us, 100^3
+        // 31 / 45 against 22 / 38; curl 128^3 100 / 141 against 87 / 146, 160^3 187 / 270
+        // against 184 / 249; divergence 160^3 99 / 141 against 124 / 138, 200^3 207 / 299
+        // against 215 / 260, 256^3 385 / 556 against 346 / 433
+        V->march_min = kind == DEO_VC_GRADIENT ? 1000000 : (kind == DEO_VC_DIVERGENCE && bnk == 3 ? 16000000 : 4000000);
     }
     V->dtype = dtype;
     V->ncomp_in = kind == DEO_VC_GRADIENT ? 1 : (kind == DEO_VC_CURL ? 3 : ndims);
@@ -2359,10 +2390,15 @@ extern "C" deo_status deo_vector_calculus_apply(const deo_vc* vc, const void* M,
     const size_t es = vc->dtype == DEO_F64 ? 8 : 4;
     if (overlaps(M, (size_t)(vc->dev.pvol * vc->ncomp_in) * es, out, (size_t)(vc->dev.ovol * vc->ncomp_out) * es))
         return fail(DEO_ERR_BAD_ARG, "the output must not overlap the input");
-    const int e = deo_k_vector_calculus(&vc->dev, &vc->bfp, vc->bfp.ok ? vc->claims.next() : nullptr, vc->dtype, M, out, overwrite ? 1 : 0, stream);
+    const bool march = vc->bfp.ok && vc->dev.ovol >= vc->march_min;
+    const int e = deo_k_vector_calculus(&vc->dev, march ? &vc->bfp : nullptr, march ? vc->claims.next() : nullptr,
+                                        vc->dtype, M, out, overwrite ? 1 : 0, stream);
     if (e) return cuda_fail((cudaError_t)e, "deo_vector_calculus_apply launch");
     return DEO_OK;
 }
+
+// The marching kernel from `points` on (tests of its edges on small arrays).
+extern "C" void deo_vector_calculus_march_min(deo_vc* vc, int64_t points) { vc->march_min = points; }
 
 extern "C" void deo_vector_calculus_destroy(deo_vc* vc) { delete vc; }
 

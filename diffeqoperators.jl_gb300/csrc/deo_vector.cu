@@ -706,12 +706,12 @@ int launch_fx(const VcDev& V, const VcBfp& B, unsigned int* claims, const double
 }
 
 template <typename T, int KIND, int ND>
-int launch_tiled(const VcDev& V, const VcBfp& B, unsigned int* claims, const T* M, T* out, int ow, cudaStream_t st) {
+int launch_tiled(const VcDev& V, const VcBfp* B, unsigned int* claims, const T* M, T* out, int ow, cudaStream_t st) {
     if constexpr (ND == 3 && std::is_same<T, double>::value)
-        if (B.ok) switch (V.band_nk) {
-                case 3: return launch_fx<KIND, 3>(V, B, claims, M, out, ow, st);
-                case 5: return launch_fx<KIND, 5>(V, B, claims, M, out, ow, st);
-                case 7: return launch_fx<KIND, 7>(V, B, claims, M, out, ow, st);
+        if (B) switch (V.band_nk) {
+                case 3: return launch_fx<KIND, 3>(V, *B, claims, M, out, ow, st);
+                case 5: return launch_fx<KIND, 5>(V, *B, claims, M, out, ow, st);
+                case 7: return launch_fx<KIND, 7>(V, *B, claims, M, out, ow, st);
                 default: break;
             }
     // marching kernel: columns x chunks of the last axis within the grid limits
@@ -745,7 +745,7 @@ int launch_tiled(const VcDev& V, const VcBfp& B, unsigned int* claims, const T* 
 }
 
 template <typename T>
-int launch_vc(const VcDev& V, const VcBfp& B, unsigned int* claims, const void* Mv, void* outv, int ow, cudaStream_t st) {
+int launch_vc(const VcDev& V, const VcBfp* B, unsigned int* claims, const void* Mv, void* outv, int ow, cudaStream_t st) {
     const T* M = static_cast<const T*>(Mv);
     T* out = static_cast<T*>(outv);
     if (V.quirk && V.nd == 2) {
@@ -770,8 +770,8 @@ extern "C" int deo_k_vector_calculus(const deo::VcDev* V, const deo::VcBfp* B, u
                                      const void* M, void* out, int overwrite, void* stream) {
     if (V->ovol <= 0) return 0;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return dtype == 0 ? deo::launch_vc<double>(*V, *B, claims, M, out, overwrite, st)
-                      : deo::launch_vc<float>(*V, *B, claims, M, out, overwrite, st);
+    return dtype == 0 ? deo::launch_vc<double>(*V, B, claims, M, out, overwrite, st)
+                      : deo::launch_vc<float>(*V, B, claims, M, out, overwrite, st);
 }
 
 extern "C" int deo_k_padded_apply(const deo::VcDev* V, int axis, int64_t coff, int dtype, const void* M, void* out,

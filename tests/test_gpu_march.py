@@ -54,6 +54,7 @@ def test_march_against_oracle(cuda, shape, a, one_band, field):
     A, oterms, _ = build(case)
     u = _field(field, shape)
     p = deo.Plan(A.terms(), shape, 0)
+    p.set_option(deo.DEO_OPT_EXACT_SUMS, 1)  # the kernel at every size
     base = np.asfortranarray(np.random.default_rng(6).standard_normal(shape))
     out, acc = deo.julia_array(shape, fill=np.nan), to_device(base)
     p.apply(to_device(u), out)

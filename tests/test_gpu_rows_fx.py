@@ -57,6 +57,7 @@ def test_rows_against_oracle(cuda, name, shape, field):
         u = u * 2.0 ** 960
     u = np.asfortranarray(u)
     p = deo.Plan(A.terms(), shape, 0)
+    p.set_option(deo.DEO_OPT_EXACT_SUMS, 1)  # the kernel at every size
     base = np.asfortranarray(rng.standard_normal(shape))
     out, acc = deo.julia_array(shape, fill=np.nan), to_device(base)
     p.apply(to_device(u), out)
@@ -76,3 +77,18 @@ def test_rows_against_oracle(cuda, name, shape, field):
     p.set_option(deo.DEO_OPT_EXACT_SUMS, 0)
     p.apply(to_device(u), out)
     assert p.kernels == ("k_apply",)
+
+
+@pytest.mark.parametrize("a", [2, 4])
+@pytest.mark.parametrize("h", [(1 / 1025, 1 / 1025), (1 / 1025, 1 / 513)])
+@pytest.mark.parametrize("shape,kernel", [((1024, 512), "k_rows_fx"), ((1023, 512), "k_apply"), ((1025, 513), "k_rows_fx")])
+def test_default_2d_laplacian(cuda, shape, kernel, h, a):
+    """Laplacian-type plans on each side of the size from which the default apply takes this kernel."""
+    case = dict(shape=shape, terms=[T("centered", 2, a, axis=k + 1, h=h[k], bc=ROBIN) for k in range(2)], seed=2)
+    A, oterms, u = build(case)
+    p = deo.Plan(A.terms(), shape, 0)
+    out = deo.julia_array(shape, fill=np.nan)
+    p.apply(to_device(u), out)
+    assert p.kernels == (kernel,)
+    ref, scale = O.apply(oterms, u), O.abs_scale(oterms, u)
+    assert (np.abs(to_host(out) - ref) <= 4 * np.spacing(scale)).all()
