@@ -2873,6 +2873,10 @@ struct deo_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t cap = nullptr;
+    // a single stage: k_stage_one, launched with its arguments (no list, counter or graph: a
+    // graph of that one kernel took longer to launch than the kernel, and its capture, the
+    // allocations and their release 250 us of a solve)
+    bool one() const { return kind == 1 && plans.size() == 1; }
     void drop_graph() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -2899,14 +2903,15 @@ static deo_status batch_items(deo_batch& b, int tile) {
     // largest tiles first keeps the tail of the persistent launch short
     std::stable_sort(items.begin(), items.end(),
                      [](const deo::WorkItem& x, const deo::WorkItem& y) { return x.count > y.count; });
+    b.n_items = (int64_t)items.size();
+    b.tile = tile;
+    if (b.one()) return DEO_OK;
     cudaFree(b.d_items);
     b.d_items = nullptr;
-    b.n_items = (int64_t)items.size();
     if (items.empty()) return DEO_OK;
     CUDA_TRY(cudaMalloc(&b.d_items, items.size() * sizeof(deo::WorkItem)), "cudaMalloc(work-list)");
     CUDA_TRY(cudaMemcpy(b.d_items, items.data(), items.size() * sizeof(deo::WorkItem), cudaMemcpyHostToDevice),
              "cudaMemcpy(work-list)");
-    b.tile = tile;
     b.drop_graph();
     return DEO_OK;
 }
@@ -2952,7 +2957,7 @@ extern "C" deo_status deo_apply_each(int n, const deo_instance* in, int adjoint,
 }
 
 static deo_status batch_launch(deo_batch& b, cudaStream_t st) {
-    const int e = b.kind == 1 && b.plans.size() == 1 ? deo_k_stage_one(&b.plans[0]->dev, &b.stages[0], st)
+    const int e = b.one() ? deo_k_stage_one(&b.plans[0]->dev, &b.stages[0], st)
                   : b.kind == 1
                       ? deo_k_stage_batch(b.d_stages, b.d_items, b.n_items, b.d_counter, b.lbc, b.dtype, b.ctas, 256,
                                           st)
@@ -2982,13 +2987,15 @@ extern "C" deo_status deo_stage_batch_create(int n, const deo_stage* in, int til
         b->lbc |= s.plan->dev.has_lbc;
     }
     b->dtype = n > 0 ? in[0].plan->dev.dtype : 0;
-    if (n > 0) {
+    if (n > 1) {
         CUDA_TRY(cudaMalloc(&b->d_stages, n * sizeof(deo::StageDev)), "cudaMalloc(stages)");
         CUDA_TRY(cudaMemcpy(b->d_stages, b->stages.data(), n * sizeof(deo::StageDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(stages)");
     }
-    CUDA_TRY(cudaMalloc(&b->d_counter, 2 * sizeof(unsigned int)), "cudaMalloc(counters)");
-    CUDA_TRY(cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned int)), "cudaMemset(counters)");
+    if (!b->one()) {
+        CUDA_TRY(cudaMalloc(&b->d_counter, 2 * sizeof(unsigned int)), "cudaMalloc(counters)");
+        CUDA_TRY(cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned int)), "cudaMemset(counters)");
+    }
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
@@ -3000,7 +3007,7 @@ extern "C" deo_status deo_batch_run(deo_batch* b, int use_graph, void* stream) {
     if (!b) return fail(DEO_ERR_BAD_ARG, "null batch");
     if (b->n_items == 0) return DEO_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!use_graph) return batch_launch(*b, st);
+    if (!use_graph || b->one()) return batch_launch(*b, st);
     if (!b->exec) {
         if (!b->cap) CUDA_TRY(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking), "cudaStreamCreate");
         CUDA_TRY(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");

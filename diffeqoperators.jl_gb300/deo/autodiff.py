@@ -12,7 +12,7 @@ from __future__ import annotations
 
 import math
 
-from .operators import _dtype_code, julia_array, plan_for
+from .operators import _dtype_code, fortran_strides, julia_array, plan_for, to_julia_layout
 
 NoTangent = None
 
@@ -156,5 +156,4 @@ def ssprk3_grad_norm2(A, u0, dt: float, nsteps: int, checkpoint: str = "none", u
 
 
 def _jl(t):
-    from .operators import fortran_strides, to_julia_layout
-    return t if tuple(t.stride()) == fortran_strides(t.shape) else to_julia_layout(t)
+    return t if t.stride() == fortran_strides(t.shape) else to_julia_layout(t)

@@ -489,7 +489,8 @@ deo_status deo_batch_create(int n, const deo_instance* inst, int adjoint, int ti
  * baseline the batched launch is measured against. */
 deo_status deo_apply_each(int n, const deo_instance* inst, int adjoint, void* stream);
 /* Runs the batch; with use_graph = 1 the launch is captured once into a CUDA
- * graph and replayed. */
+ * graph and replayed.
+ * A stage batch of one instance is one launch with its arguments either way. */
 deo_status deo_batch_run(deo_batch* b, int use_graph, void* stream);
 /* Re-point instance i at new buffers (same plan); invalidates the graph. */
 deo_status deo_batch_set_buffers(deo_batch* b, int i, const void* u, void* du);
