@@ -1793,39 +1793,52 @@ static unsigned int* next_sched(const deo_plan* p) {
     return p->d_sched ? p->d_sched + (p->sched_slot.fetch_add(1) % kSchedSlots) : nullptr;
 }
 
-// The interior first, then the shell with its full grid, which fills the SMs as
-// the interior's CTAs leave them (the face kernel where TMA can read the array,
-// else one thread per point): 188 us at 256^3, against 213 with the line
-// kernel, 231-256 with the face kernel's one-CTA-per-SM form and 220 with the
-// shell after the interior (interior alone 164, shell alone 55).
-static int launch_march(const deo_plan* p, const void* u, void* du, int overwrite, void* stream) {
+// Interior and shell write different points: with conc the shell runs on the plan's
+// side stream, launched after the interior and free to fill the SMs as the interior's
+// CTAs leave them, and the caller's stream waits for it.
+template <class Interior, class Shell>
+static int interior_then_shell(const deo_plan* p, bool conc, void* stream, Interior interior, Shell shell) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    deo::UniPlan us = p->uni;
-    if (us.shell_kernel == 0) us.shell_kernel = 1;
-    const bool conc = p->concurrent && p->side && p->d_shell;
-    const deo::ShellPlan* sp = p->d_shell ? &p->shell : nullptr;
-    const char* k2 = "";
     std::unique_lock<std::mutex> lk(p->apply_mu, std::defer_lock);
     if (conc) {
         lk.lock();
         const cudaError_t c = cudaEventRecord(p->ev_fork, st);
         if (c != cudaSuccess) return (int)c;
     }
-    int e = deo_k_apply_march(&p->uni, &p->march, p->claims.next(), u, du, overwrite, stream);
+    int e = interior();
     if (e) return e;
-    mark(p, 1, stream);
-    if (conc) {
-        const cudaError_t c = cudaStreamWaitEvent(p->side, p->ev_fork, 0);
-        if (c != cudaSuccess) return (int)c;
-    }
-    e = deo_k_apply_shell(&us, sp, p->d_shell, DEO_SHELL_ALONE, p->d_plan, p->dev.dtype, u, du, overwrite,
-                          conc ? static_cast<void*>(p->side) : stream, &k2);
+    if (!conc) return shell(stream);
+    cudaError_t c = cudaStreamWaitEvent(p->side, p->ev_fork, 0);
+    if (c != cudaSuccess) return (int)c;
+    e = shell(static_cast<void*>(p->side));
     if (e) return e;
-    if (conc) {
-        cudaError_t c = cudaEventRecord(p->ev_join, p->side);
-        if (c == cudaSuccess) c = cudaStreamWaitEvent(st, p->ev_join, 0);
-        if (c != cudaSuccess) return (int)c;
-    }
+    c = cudaEventRecord(p->ev_join, p->side);
+    if (c == cudaSuccess) c = cudaStreamWaitEvent(st, p->ev_join, 0);
+    return (int)c;
+}
+
+// The interior first, then the shell with its full grid, which fills the SMs as
+// the interior's CTAs leave them (the face kernel where TMA can read the array,
+// else one thread per point): 188 us at 256^3, against 213 with the line
+// kernel, 231-256 with the face kernel's one-CTA-per-SM form and 220 with the
+// shell after the interior (interior alone 164, shell alone 55).
+static int launch_march(const deo_plan* p, const void* u, void* du, int overwrite, void* stream) {
+    deo::UniPlan us = p->uni;
+    if (us.shell_kernel == 0) us.shell_kernel = 1;
+    const deo::ShellPlan* sp = p->d_shell ? &p->shell : nullptr;
+    const char* k2 = "";
+    const int e = interior_then_shell(
+        p, p->concurrent && p->side && p->d_shell, stream,
+        [&] {
+            const int ei = deo_k_apply_march(&p->uni, &p->march, p->claims.next(), u, du, overwrite, stream);
+            mark(p, 1, stream);
+            return ei;
+        },
+        [&](void* s2) {
+            return deo_k_apply_shell(&us, sp, p->d_shell, DEO_SHELL_ALONE, p->d_plan, p->dev.dtype, u, du, overwrite,
+                                     s2, &k2);
+        });
+    if (e) return e;
     p->last_kernel = "k_lap_fx";
     p->last_kernel2 = k2;
     p->ev_launches = 2;
@@ -2011,14 +2024,18 @@ extern "C" deo_status deo_apply(const deo_plan* p, const void* u, void* du, int 
     return DEO_OK;
 }
 
-// Transposed applies.  Laplacian-type plans on the TMA path: the interior
-// kernel of the forward apply, with every band's taps reversed, on the box
-// of columns read only by band rows (there column j of the transpose is
-// sum_k w[2H - k] d[j + k - H], the order in which the generic column
-// evaluator adds the rows), then the generic column evaluator on the rest
-// (k_shell_adj, a full grid; beside the interior, in the one CTA per SM that
-// fits there, it took longer than the interior: 0.52 against 0.37 ms at
-// 256^3).  Other plans: the generic transposed kernel.
+// Transposed applies.  Laplacian-type plans: the interior kernel of the forward apply,
+// with every band's taps reversed, on the box of columns read only by band rows (there
+// column j of the transpose is sum_k w[2H - k] d[j + k - H], the order in which the
+// generic column evaluator adds the rows), and the generic column evaluator on the rest
+// (k_shell_adj, a full grid).  Other plans: the generic transposed kernel.
+//
+// The two run side by side in Float32 (after / beside: 64^3 order 2 21 / 17 us, 160 x 128
+// x 96 order 4 39 / 35, 256^3 56 / 52) and, in Float64, where the column evaluator is
+// short against the marching interior (order 2: 64^3 19 / 13, 160 x 128 x 96 42 / 35,
+// 256^3 174 / 171) or latency is all (64^3 order 4 27 / 19).  From order 4 on it is as
+// long as the interior and takes its CTAs' places: 256^3 316 / 328.
+constexpr int64_t kAdjBesideMaxPoints = 1 << 18;
 template <typename E>
 static void reverse_taps(E* w, int n) {
     for (int k = 0; k < n / 2; ++k) std::swap(w[k], w[n - 1 - k]);
@@ -2038,8 +2055,10 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
             reverse_taps(B.wh[a], K);
             reverse_taps(B.wl[a], K);
         }
-        int e = deo_k_apply_march(&ua, &B, p->claims.next(), d, ub, overwrite, stream);
-        if (!e) e = deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, stream);
+        const int e = interior_then_shell(
+            p, p->concurrent && p->side && (ua.radius == 1 || p->dev.total <= kAdjBesideMaxPoints), stream,
+            [&] { return deo_k_apply_march(&ua, &B, p->claims.next(), d, ub, overwrite, stream); },
+            [&](void* s2) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
         if (e) return e;
         p->last_kernel = "k_lap_fx";
         p->last_kernel2 = "k_shell_adj";
@@ -2062,11 +2081,13 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
         reverse_taps(ua.bfx_w, K);
         unsigned int* sched = p->d_sched ? p->d_sched + (p->sched_slot.fetch_add(1) % kSchedSlots) : nullptr;
         const char* k = "";
-        const int e = deo_k_apply_tma(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, p->exact_sums, stream, &k,
-                                      sched);
+        const int e = interior_then_shell(
+            p, p->concurrent && p->side && p->dev.dtype == DEO_F32, stream,
+            [&] {
+                return deo_k_apply_tma(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, p->exact_sums, stream, &k, sched);
+            },
+            [&](void* s2) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
         if (e) return e;
-        const int e2 = deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, stream);
-        if (e2) return e2;
         p->last_kernel = k;
         p->last_kernel2 = "k_shell_adj";
         return 0;
