@@ -317,7 +317,7 @@ __device__ __forceinline__ T straight_nk(const T* w, int64_t ws, const T* __rest
     return acc;
 }
 // Which lengths are unrolled: Float32 waits on its loads (all common lengths: 2048^2,
-// order 2, 45 -> 27 us), Float64 on the FP64 pipe, where the long bands lose by it what
+// order 2, 45 -> 28 us), Float64 on the FP64 pipe, where the long bands lose by it what
 // the short ones gain (2048^2: 3 taps 70 -> 62 us, 9 taps 158 unrolled, 156 not; the
 // transposed bands 93 -> 87 at 5 taps).
 template <typename T, bool REV, bool ROWS, bool SCALED>
@@ -339,36 +339,46 @@ __device__ __forceinline__ T straight(const T* w, int64_t ws, const T* __restric
 // them, bit for bit the same sums.  The general loops choose between band and explicit
 // row, ghost and line at every tap (40 instructions a tap) and look up p0, nk and the
 // touching rows at every point, also on graded lines, whose rows differ by their
-// weights alone.  2048^2 at 5 taps, apply / transposed: uniform Float64 97 / 90 ->
-// 94 / 87 us, Float32 49 / 52 -> 31 / 35; graded Float64 107 / 114 -> 90 / 90, Float32
-// 78 / 99 -> 34 / 40.
+// weights alone.  A warp with one row outside the range takes the general loop as a
+// whole: both loops one after the other were the longest chain of the small and the
+// ragged launches (graded 542 x 226 with a field 24.0 us, 20.8 so; 65 x 33 x 41, 9 taps,
+// 15.4 / 15.9 and 13.8 / 14.5).  2048^2 at 5 taps, general / straight, apply and
+// transposed: uniform Float64 97 -> 95 and 90 -> 86 us, Float32 49 -> 32 and 52 -> 35;
+// graded Float64 107 -> 89 and 114 -> 90, Float32 78 -> 36 and 99 -> 40.
 template <typename T, bool ADJ, bool LBC>
 __device__ __forceinline__ T term_at(const TermDev& t, const T* __restrict__ u, int64_t idx, int i) {
     const int64_t s = t.stride;
     if constexpr (ADJ) {
-        if (i < t.sa_lo || i > t.sa_hi) return adj_term<T, LBC>(t, u, idx, i);
-        // rows i + 2 - s_off - s_nk + m, their taps nk - 1 - m
-        const T* __restrict__ x = u + idx + (2 - t.s_off - t.s_nk) * s;
+        if (!__all_sync(__activemask(), i >= t.sa_lo && i <= t.sa_hi)) return adj_term<T, LBC>(t, u, idx, i);
+        const int i0 = i + 2 - t.s_off[0] - t.s_nk[0];  // rows i0 + m, their taps nk - 1 - m
+        const T* __restrict__ x = u + idx + (i0 - i) * s;
         if (t.s_rows) {
-            const T* w = reinterpret_cast<const T*>(t.tab[0].W) + (int64_t)(t.s_nk - 1) * t.tab[0].nexp +
-                         (i + 2 - t.s_off - t.s_nk + t.s_e0);
-            return straight<T, true, true, false>(w, 1 - t.tab[0].nexp, x, s, T(1), t.s_nk);
+            const T* w = reinterpret_cast<const T*>(t.tab[0].W) + (int64_t)(t.s_nk[0] - 1) * t.tab[0].nexp + (i0 + t.s_e0[0]);
+            return straight<T, true, true, false>(w, 1 - t.tab[0].nexp, x, s, T(1), t.s_nk[0]);
         }
-        return straight<T, true, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0, x, s, T(1), t.s_nk);
+        return straight<T, true, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0, x, s, T(1), t.s_nk[0]);
     } else {
-        if (i < t.sf_lo || i > t.sf_hi) return eval_term<T, LBC>(t, u, idx, i);
-        if (t.s_rows)
-            return straight<T, false, true, false>(reinterpret_cast<const T*>(t.tab[0].W) + (i + t.s_e0), t.tab[0].nexp,
-                                                   u + idx + (t.s_off - 1) * s, s, T(1), t.s_nk);
-        if (!t.has_field)
-            return straight<T, false, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0,
-                                                    u + idx + (t.s_off - 1) * s, s, T(1), t.s_nk);
-        const T c = __ldg(reinterpret_cast<const T*>(t.field) + idx + t.tab[0].band_cidx_off * s);
-        const RowTabDev& tb = t.nvar == 2 && not_nonneg(c) ? t.tab[1] : t.tab[0];
+        if (!__all_sync(__activemask(), i >= t.sf_lo && i <= t.sf_hi)) return eval_term<T, LBC>(t, u, idx, i);
+        if (!t.has_field) {
+            const T* __restrict__ x = u + idx + (t.s_off[0] - 1) * s;
+            if (t.s_rows)
+                return straight<T, false, true, false>(reinterpret_cast<const T*>(t.tab[0].W) + (i + t.s_e0[0]),
+                                                       t.tab[0].nexp, x, s, T(1), t.s_nk[0]);
+            return straight<T, false, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0, x, s, T(1), t.s_nk[0]);
+        }
+        const T c = __ldg(reinterpret_cast<const T*>(t.field) + idx + t.s_cidx * s);
+        const int v = t.nvar == 2 && not_nonneg(c);
+        const RowTabDev& tb = t.tab[v];
+        const T* __restrict__ x = u + idx + (t.s_off[v] - 1) * s;
         const T* w = reinterpret_cast<const T*>(tb.wband);
-        const T* __restrict__ x = u + idx + (tb.band_p0_off - 1) * s;
-        if (t.has_field == 2) return c * straight<T, false, false, false>(w, 0, x, s, T(1), tb.band_nk);
-        return straight<T, false, false, true>(w, 0, x, s, c, tb.band_nk);
+        const int nk = t.s_nk[v];
+        if (t.s_rows) {
+            w = reinterpret_cast<const T*>(tb.W) + (i + t.s_e0[v]);
+            if (t.has_field == 2) return c * straight_nk<T, false, true, false, 0>(w, tb.nexp, x, s, T(1), nk);
+            return straight_nk<T, false, true, true, 0>(w, tb.nexp, x, s, c, nk);
+        }
+        if (t.has_field == 2) return c * straight_nk<T, false, false, false, 0>(w, 0, x, s, T(1), nk);
+        return straight_nk<T, false, false, true, 0>(w, 0, x, s, c, nk);
     }
 }
 

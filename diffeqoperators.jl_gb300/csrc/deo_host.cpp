@@ -771,17 +771,18 @@ static deo_status compile_rows(long len, Row make, HostTab& T, std::vector<int>&
 // Rows [lo, hi] of one shape: p0 = i + off, nk taps, weights from the band or (rows)
 // from entry i + e0 of the explicit rows, whichever range is longer.
 struct RowRange {
-    int lo = 1, hi = 0, off = 0, nk = 0, e0 = 0, rows = 0;
+    int lo = 1, hi = 0, off = 0, nk = 0, e0 = 0, rows = 0, cidx = 0;
     int size() const { return hi - lo + 1; }
 };
 static RowRange row_range(const HostTab& H) {
     const RowTabDev& d = H.dev;
     RowRange best, run;
-    if (d.ilo <= d.ihi) best = RowRange{d.ilo, d.ihi, d.band_p0_off, d.band_nk, 0, 0};
+    if (d.ilo <= d.ihi) best = RowRange{d.ilo, d.ihi, d.band_p0_off, d.band_nk, 0, 0, d.band_cidx_off};
     for (int e = 0; e < d.nexp; ++e) {
         const int i = e + 1 < d.ilo ? e + 1 : e + 1 + (d.ihi - d.ilo + 1);
-        if (run.nk == H.nk[e] && run.off == H.p0[e] - i && run.hi == i - 1 && run.e0 == e - i) run.hi = i;
-        else run = RowRange{i, i, H.p0[e] - i, H.nk[e], e - i, 1};
+        if (run.nk == H.nk[e] && run.off == H.p0[e] - i && run.hi == i - 1 && run.e0 == e - i && run.cidx == H.cidx[e] - i)
+            run.hi = i;
+        else run = RowRange{i, i, H.p0[e] - i, H.nk[e], e - i, 1, H.cidx[e] - i};
         if (run.size() > best.size()) best = run;
     }
     return best;
@@ -840,8 +841,9 @@ constexpr int kFxFp64Rows = 2;
 
 // k_rows_fx from here on.  Below, the generic kernel has less latency: graded, order 2
 // / 4, generic against k_rows_fx, 512 x 300 5.7 / 7.6 against 10.6 / 11.3 us, 1000 x
-// 700 14.1 / 19.8 against 13.5 / 15.5, 4000 x 3000 183 / 270 against 105 / 126.
-constexpr int64_t kRowsFxMinPoints = 1 << 19;
+// 700 13.5 / 19.1 against 13.5 / 15.5, 4000 x 3000 183 / 270 against 105 / 126.  With a
+// field term and order 6: 542 x 226 20.8 against 22.0, 700 x 500 37 against 28.
+constexpr int64_t kRowsFxMinPoints = 1 << 19, kRowsFxMinFieldPoints = 1 << 18;
 
 // Rotating claim counters of the marching kernels: two words each, zeroed here
 // once and left zero by every launch (claims_done in deo_lap.cuh).
@@ -1513,9 +1515,15 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             }
             if (s != DEO_OK) return s;
             if (v == 0) shell_rows(H, A.len, dtype, eff[t], P->shell);
-            R = row_range(H);
-            if (R.rows && T.has_field) R = RowRange{};
-            straight_rows(R, A.len, T.sf_lo, T.sf_hi);
+            const RowRange Q = row_range(H);
+            straight_rows(Q, A.len, T.sf_lo, T.sf_hi);
+            if (v > 0 && (Q.rows != R.rows || Q.cidx != R.cidx)) T.sf_hi = 0;
+            T.s_off[v] = Q.off;
+            T.s_nk[v] = Q.nk;
+            T.s_e0[v] = Q.e0;
+            T.s_rows = Q.rows;
+            T.s_cidx = Q.cidx;
+            R = Q;
             if ((s = upload_tab(*P, H, dtype, T.tab[v])) != DEO_OK) return s;
         }
         for (int p = 0; p < A.len + 2; ++p)
@@ -1540,10 +1548,6 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             T.lbc_mw = lmw;
             D.has_lbc = 1;
         }
-        T.s_off = R.off;
-        T.s_nk = R.nk;
-        T.s_e0 = R.e0;
-        T.s_rows = R.rows;
         T.sa_lo = 1;
         T.sa_hi = 0;
         if (!T.has_field && R.nk > 0) {  // the longest run of columns touched by s_nk rows of R alone and by no ghost
@@ -1851,7 +1855,7 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
     mark(p, 0, stream);
     if (use_march(p)) return launch_march(p, u, du, overwrite, stream);
     if (p->rows2.ok && p->exact_sums == 1 && p->fast_path && p->use_tma &&
-        (p->sums_set ? !p->uni.lap : p->dev.total >= kRowsFxMinPoints)) {
+        (p->sums_set ? !p->uni.lap : p->dev.total >= (p->rows2.field ? kRowsFxMinFieldPoints : kRowsFxMinPoints))) {
         const int e = deo_k_rows_fx(&p->rows2, p->d_plan, u, du, overwrite, stream);
         p->last_kernel = "k_rows_fx";
         p->last_kernel2 = "";

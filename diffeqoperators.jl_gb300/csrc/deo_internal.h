@@ -59,11 +59,11 @@ struct TermDev {
     int nvar;            // 1, or 2 for an upwind operator with a coefficient field (c>=0 / c<0)
     int has_field;       // 0: none; 1: row i = sum_k (c_i w_k) u_k; 2: c_i * sum_k w_k u_k (forward)
     // Rows [sf_lo, sf_hi] of the straight tap loop: s_nk taps from p0 = i + s_off that
-    // read no ghost, weights from the band (each variant its own band's offsets) or,
-    // s_rows = 1 (no field), from entry i + s_e0 of tab[0].W.  Columns [sa_lo, sa_hi] of
-    // its transpose: touched by s_nk rows of that form and by no ghost (no field).
+    // read no ghost, weights from the band or, s_rows = 1, from entry i + s_e0 of tab.W
+    // (each per variant); the field's value s_cidx points away.  Columns [sa_lo, sa_hi]
+    // of its transpose: touched by s_nk rows of that form and by no ghost (no field).
     int sf_lo, sf_hi, sa_lo, sa_hi;
-    int s_off, s_nk, s_e0, s_rows;
+    int s_off[2], s_nk[2], s_e0[2], s_rows, s_cidx;
     const void* field;   // coefficient field (same shape/dtype as u) or null
     RowTabDev tab[2];
     // adjoint: rows touching padded column p (1..len+2) lie in [rlo[p-1], rhi[p-1]]

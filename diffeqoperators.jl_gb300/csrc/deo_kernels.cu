@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) k_stage(const StageDev* __restrict__ st, 
 // two points a thread, five CTAs a SM.  The work-list kernel spends a third of such a
 // stage on the claim, the list and the staged plan, each a trip to L2 before the first
 // point, and its 64 registers leave half of the warps that hide the points' own
-// loads.  768 x 500 Float64, 3 terms: 26 -> 17.5 us a stage; 100 x 50: 9 -> 7.
+// loads.  768 x 500 Float64, 3 terms: 26 -> 16 us a stage; 100 x 50: 9 -> 6.7.
 // (One point a thread with six CTAs the same; four CTAs 22.)
 constexpr int STAGE_PT = 2;
 template <typename T, bool ADJ, bool LBC>
@@ -231,7 +231,7 @@ extern "C" int deo_k_scale(void* x, int64_t n, int dtype, double f, void* stream
 // CTA, of 256 points (one per thread) at the least for the default 8192-point
 // items.  One 768 x 500 Float64 state (47 items) then runs on every SM instead
 // of 47: 97 -> 31 us per Runge-Kutta stage; 256 mixed instances (1100 items)
-// forward + transposed 705 -> 565 us (487 with the straight loops of deo_eval.cuh).
+// forward + transposed 705 -> 565 us (456 with the straight loops of deo_eval.cuh).
 static int split_for(int64_t n_items, int64_t ctas) {
     int lsplit = 0;
     while (lsplit < 5 && (n_items << lsplit) < 8 * ctas) ++lsplit;
