@@ -234,6 +234,12 @@ int deo_plan_star_taps(const deo_plan* plan);
  *         any bands; within 2 ulp of sum|c_k u_k| of the exact sum); else the
  *         per-point fixed-point kernel (variant 4) when the band's weights
  *         allow it, else variant 3;
+ *         2-D Float64 plans of any kind take the rows kernel (each axis's
+ *         rows as integer windows in block fixed point, one launch) from 2^19
+ *         points on, 2^18 with a field term; smaller ones, and 3-D Laplacians
+ *         with an odd first size below 300,000 points, the generic kernel,
+ *         which is faster there.  Setting the option to 1 asks for its
+ *         kernels at every size (2-D Laplacians: the tiled ones);
  *       5 for three axes the block fixed-point kernel (values aligned once
  *         per plane to one exponent per plane tile, no FP64 instruction per
  *         point; points near a zero of u, where that alignment cannot bound
