@@ -2761,9 +2761,11 @@ extern "C" deo_status deo_solve_plan(const deo_operator* op, const deo_bc* bc, i
         lo = hi = (int)N;
     }
     // the interior's columns, when they are all alike and of a pattern the kernel knows
-    const int pm = meta[mid], plain = 100 * (pm >> 8 & 255) + 10 * (pm >> 16 & 255) + (pm & 255);
-    if (plain == 110 || plain == 121 || plain == 220 || plain == 231) {
-        B.plain = plain;
+    // (compared field by field: a wide band's counts have two digits)
+    const int pm = meta[mid];
+    for (int plain : {110, 121, 220, 231})
+        if (pm == (plain / 100 << 8 | plain / 10 % 10 << 16 | plain % 10)) B.plain = plain;
+    if (B.plain) {
         for (B.plo = mid; B.plo > 0 && meta[B.plo - 1] == pm; --B.plo) {}
         for (B.phi = mid + 1; B.phi < (int)N && meta[B.phi] == pm; ++B.phi) {}
     }
