@@ -1154,6 +1154,13 @@ static bool bfp_band(const double* w, int K, int& s, double& total, int* wh, int
     }
     return true;
 }
+// Of a centre weight c0 and the weight w1 of the neighbours at +1.
+static deo::BfpMarch::Limit march_limit(double total, double c0, double w1) {
+    const int t1 = bfp_threshold(total, w1, 2.0);
+    deo::BfpMarch::Limit L{bfp_threshold(total, c0, 1.0), 0, 0};
+    while (L.sh1 < 31 && ((long long)L.t << L.sh1) < t1) ++L.sh1;  // |n1| >> sh1 >= t implies |n1| >= t1
+    return L;
+}
 static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
     const int K = 2 * H + 1;
     double sum = 0.0;
@@ -1172,10 +1179,8 @@ static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
         }
     split_limbs(c0, B.c0h, B.c0l);
     B.shared = std::memcmp(w[0], w[1], K * sizeof(double)) == 0 && std::memcmp(w[0], w[2], K * sizeof(double)) == 0;
-    B.t0 = bfp_threshold(total, (double)c0, 1.0);
-    const int t1 = bfp_threshold(total, std::ldexp(w[0][H + 1], s), 2.0);
-    B.sh1 = 0;
-    while (B.sh1 < 31 && ((long long)B.t0 << B.sh1) < t1) ++B.sh1;  // |n1| >> sh1 >= t0 implies |n1| >= t1
+    B.limit = march_limit(total, (double)c0, std::ldexp(w[0][H + 1], s));
+    B.rev = march_limit(total, (double)c0, std::ldexp(w[0][H - 1], s));
     B.kbase = 57 - s - 1075 - 6;
     return true;
 }
@@ -2059,6 +2064,7 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
             reverse_taps(B.wh[a], K);
             reverse_taps(B.wl[a], K);
         }
+        B.limit = B.rev;
         const int e = interior_then_shell(
             p, p->concurrent && p->side && (ua.radius == 1 || p->dev.total <= kAdjBesideMaxPoints), stream,
             [&] { return deo_k_apply_march(&ua, &B, p->claims.next(), d, ub, overwrite, stream); },

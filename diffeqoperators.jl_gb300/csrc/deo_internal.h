@@ -185,7 +185,12 @@ struct BfpMarch {
     int lo[3], hi[3];     // interior box, 0-based inclusive
     int c0h, c0l;
     int wh[3][9], wl[3][9];
-    int t0, sh1;          // a point is accepted when its centre's high limb, or its +1 neighbours' >> sh1, reaches t0
+    // A point is accepted when its centre's high limb, or that of its neighbours at +1,
+    // shifted right by sh0 / sh1, reaches t.  rev: the limits of the reversed band (the
+    // transpose), whose neighbours at +1 have the weight of those at -1.
+    struct Limit {
+        int t, sh0, sh1;
+    } limit, rev;
     int kbase;            // the sum in units of 2^57 times 2^(kbase + E) is the result
 };
 

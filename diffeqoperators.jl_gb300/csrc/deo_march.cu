@@ -14,7 +14,7 @@
 // it, the resident planes are converted again from global memory (rare, and
 // uniform over the CTA).
 //
-// A point whose error bound fails (BfpMarch::t0) is queued by its warp and
+// A point whose error bound fails (BfpMarch::Limit) is queued by its warp and
 // evaluated in the reference's order, from global memory, 32 at a time at the
 // end of the unit (draining as the queue passed 32 held every other warp at the
 // plane's barrier: 8 us more at 256^3).  A plane with Inf/NaN, or with an exponent
@@ -200,7 +200,7 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
             // the threshold of this plane: none when everything in use is zero, out of reach when the exponent
             // rules fixed point out
             const bool special = E >= 2047 || !bfp_range_ok(kexp);
-            const int t0 = special ? INT_MAX : (zeros >= NQ ? 0 : B.t0);
+            const int t0 = special ? INT_MAX : (zeros >= NQ ? 0 : B.limit.t);
             const double scale = special ? 1.0 : bfp_pow2(kexp);
             const int4* pl[NQ];  // own pair of the first row in the planes z - H .. z + H
 #pragma unroll
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                             }
                         }
                     r[j][v] = bfp_double(bfp_total(a), scale);
-                    far[j][v] = max(abs(c.h), abs(n1) >> B.sh1);
+                    far[j][v] = max(abs(c.h), abs(n1) >> B.limit.sh1);
                 }
             }
             int nearest = INT_MAX;
