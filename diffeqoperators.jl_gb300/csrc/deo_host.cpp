@@ -1154,11 +1154,15 @@ static bool bfp_band(const double* w, int K, int& s, double& total, int* wh, int
     }
     return true;
 }
-// Of a centre weight c0 and the weight w1 of the neighbours at +1.
+// Of a centre weight c0 and the weight w1 of the neighbours at +1: the lower of the two
+// thresholds, and the shift that makes it serve for the other (|n| >> sh >= t implies
+// |n| >= t << sh).  A first or third derivative's sum has no centre weight: its points
+// are accepted by their neighbours alone.
 static deo::BfpMarch::Limit march_limit(double total, double c0, double w1) {
-    const int t1 = bfp_threshold(total, w1, 2.0);
-    deo::BfpMarch::Limit L{bfp_threshold(total, c0, 1.0), 0, 0};
-    while (L.sh1 < 31 && ((long long)L.t << L.sh1) < t1) ++L.sh1;  // |n1| >> sh1 >= t implies |n1| >= t1
+    const int t0 = bfp_threshold(total, c0, 1.0), t1 = bfp_threshold(total, w1, 2.0);
+    deo::BfpMarch::Limit L{std::min(t0, t1), 0, 0};
+    while (L.sh0 < 31 && ((long long)L.t << L.sh0) < t0) ++L.sh0;
+    while (L.sh1 < 31 && ((long long)L.t << L.sh1) < t1) ++L.sh1;
     return L;
 }
 static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {

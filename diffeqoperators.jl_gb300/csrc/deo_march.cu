@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                             }
                         }
                     r[j][v] = bfp_double(bfp_total(a), scale);
-                    far[j][v] = max(abs(c.h), abs(n1) >> B.limit.sh1);
+                    far[j][v] = max(abs(c.h) >> B.limit.sh0, abs(n1) >> B.limit.sh1);
                 }
             }
             int nearest = INT_MAX;
