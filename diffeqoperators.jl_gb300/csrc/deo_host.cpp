@@ -845,6 +845,14 @@ constexpr int kFxFp64Rows = 2;
 // field term and order 6: 542 x 226 20.8 against 22.0, 700 x 500 37 against 28.
 constexpr int64_t kRowsFxMinPoints = 1 << 19, kRowsFxMinFieldPoints = 1 << 18;
 
+// n zeroed words.  The zeros have arrived on return: a memset on the default stream is not
+// ordered before work on a non-blocking stream, where the first launch may be.
+static cudaError_t alloc_zeroed(unsigned int** d, size_t n) {
+    cudaError_t e = cudaMalloc(d, n * sizeof(unsigned int));
+    if (e == cudaSuccess) e = cudaMemset(*d, 0, n * sizeof(unsigned int));
+    return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
+}
+
 // Rotating claim counters of the marching kernels: two words each, zeroed here
 // once and left zero by every launch (claims_done in deo_lap.cuh).
 struct ClaimSlots {
@@ -853,10 +861,7 @@ struct ClaimSlots {
     ~ClaimSlots() {
         if (d) cudaFree(d);
     }
-    cudaError_t init() {
-        cudaError_t e = cudaMalloc(&d, 2 * kSchedSlots * sizeof(unsigned int));
-        return e == cudaSuccess ? cudaMemset(d, 0, 2 * kSchedSlots * sizeof(unsigned int)) : e;
-    }
+    cudaError_t init() { return alloc_zeroed(&d, 2 * kSchedSlots); }
     unsigned int* next() { return d + 2 * (slot.fetch_add(1) % kSchedSlots); }
 };
 
@@ -2974,8 +2979,7 @@ extern "C" deo_status deo_batch_create(int n, const deo_instance* in, int adjoin
         CUDA_TRY(cudaMemcpy(b->d_inst, b->inst.data(), n * sizeof(deo::InstDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(instances)");
     }
-    CUDA_TRY(cudaMalloc(&b->d_counter, 2 * sizeof(unsigned int)), "cudaMalloc(counters)");
-    CUDA_TRY(cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned int)), "cudaMemset(counters)");
+    CUDA_TRY(alloc_zeroed(&b->d_counter, 2), "counters");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
@@ -3029,10 +3033,7 @@ extern "C" deo_status deo_stage_batch_create(int n, const deo_stage* in, int til
         CUDA_TRY(cudaMemcpy(b->d_stages, b->stages.data(), n * sizeof(deo::StageDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(stages)");
     }
-    if (!b->one()) {
-        CUDA_TRY(cudaMalloc(&b->d_counter, 2 * sizeof(unsigned int)), "cudaMalloc(counters)");
-        CUDA_TRY(cudaMemset(b->d_counter, 0, 2 * sizeof(unsigned int)), "cudaMemset(counters)");
-    }
+    if (!b->one()) CUDA_TRY(alloc_zeroed(&b->d_counter, 2), "counters");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
