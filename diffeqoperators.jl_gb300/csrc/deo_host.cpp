@@ -853,16 +853,34 @@ static cudaError_t alloc_zeroed(unsigned int** d, size_t n) {
     return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;
 }
 
-// Rotating claim counters of the marching kernels: two words each, zeroed here
-// once and left zero by every launch (claims_done in deo_lap.cuh).
+// Claim counters of the marching and batched kernels (claims_done in deo_lap.cuh): blocks
+// of two pairs.  A launch takes the next block; every lap of the blocks takes the other
+// pair, which the pair's launch before it has zeroed.  A launch that is being captured
+// takes a block that no direct launch ever uses, zeroed by a memset of its own: a graph
+// may be replayed beside any number of later launches.
 struct ClaimSlots {
+    static constexpr unsigned int kBlocks = kSchedSlots / 4;  // of direct launches, and as many of captured ones
     unsigned int* d = nullptr;
-    std::atomic<unsigned int> slot{0};
+    std::atomic<unsigned int> direct{0}, captured{0};
     ~ClaimSlots() {
         if (d) cudaFree(d);
     }
-    cudaError_t init() { return alloc_zeroed(&d, 2 * kSchedSlots); }
-    unsigned int* next() { return d + 2 * (slot.fetch_add(1) % kSchedSlots); }
+    cudaError_t init() { return alloc_zeroed(&d, 2 * 4 * kBlocks); }
+    unsigned int* graph_block() { return d + 4 * (kBlocks + captured.fetch_add(1) % kBlocks); }
+    static bool capturing(cudaStream_t st) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();  // (the launch reports what is wrong)
+        return cap == cudaStreamCaptureStatusActive;
+    }
+    cudaError_t next(cudaStream_t st, unsigned int** pair) {
+        if (capturing(st)) {
+            *pair = graph_block();
+            return cudaMemsetAsync(*pair, 0, 2 * sizeof(unsigned int), st);
+        }
+        const unsigned int k = direct.fetch_add(1);
+        *pair = d + 4 * (k % kBlocks) + 2 * (k / kBlocks % 2);
+        return cudaSuccess;
+    }
 };
 
 struct deo_plan {
@@ -1848,7 +1866,9 @@ static int launch_march(const deo_plan* p, const void* u, void* du, int overwrit
     const int e = interior_then_shell(
         p, p->concurrent && p->side && p->d_shell, stream,
         [&] {
-            const int ei = deo_k_apply_march(&p->uni, &p->march, p->claims.next(), u, du, overwrite, stream);
+            unsigned int* pair;
+            int ei = (int)p->claims.next(static_cast<cudaStream_t>(stream), &pair);
+            if (!ei) ei = deo_k_apply_march(&p->uni, &p->march, pair, u, du, overwrite, stream);
             mark(p, 1, stream);
             return ei;
         },
@@ -2076,7 +2096,11 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
         B.limit = B.rev;
         const int e = interior_then_shell(
             p, p->concurrent && p->side && (ua.radius == 1 || p->dev.total <= kAdjBesideMaxPoints), stream,
-            [&] { return deo_k_apply_march(&ua, &B, p->claims.next(), d, ub, overwrite, stream); },
+            [&] {
+                unsigned int* pair;
+                const int ei = (int)p->claims.next(static_cast<cudaStream_t>(stream), &pair);
+                return ei ? ei : deo_k_apply_march(&ua, &B, pair, d, ub, overwrite, stream);
+            },
             [&](void* s2) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
         if (e) return e;
         p->last_kernel = "k_lap_fx";
@@ -2431,8 +2455,10 @@ extern "C" deo_status deo_vector_calculus_apply(const deo_vc* vc, const void* M,
     if (overlaps(M, (size_t)(vc->dev.pvol * vc->ncomp_in) * es, out, (size_t)(vc->dev.ovol * vc->ncomp_out) * es))
         return fail(DEO_ERR_BAD_ARG, "the output must not overlap the input");
     const bool march = vc->bfp.ok && vc->dev.ovol >= vc->march_min;
-    const int e = deo_k_vector_calculus(&vc->dev, march ? &vc->bfp : nullptr, march ? vc->claims.next() : nullptr,
-                                        vc->dtype, M, out, overwrite ? 1 : 0, stream);
+    unsigned int* pair = nullptr;
+    if (march) CUDA_TRY(vc->claims.next(static_cast<cudaStream_t>(stream), &pair), "cudaMemsetAsync(claim counters)");
+    const int e = deo_k_vector_calculus(&vc->dev, march ? &vc->bfp : nullptr, pair, vc->dtype, M, out,
+                                        overwrite ? 1 : 0, stream);
     if (e) return cuda_fail((cudaError_t)e, "deo_vector_calculus_apply launch");
     return DEO_OK;
 }
@@ -2911,7 +2937,7 @@ struct deo_batch {
     int64_t n_items = 0;
     deo::InstDev* d_inst = nullptr;
     deo::WorkItem* d_items = nullptr;
-    unsigned int* d_counter = nullptr;
+    ClaimSlots claims;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaStream_t cap = nullptr;
@@ -2931,7 +2957,6 @@ struct deo_batch {
         cudaFree(d_inst);
         cudaFree(d_stages);
         cudaFree(d_items);
-        cudaFree(d_counter);
     }
 };
 
@@ -2979,7 +3004,7 @@ extern "C" deo_status deo_batch_create(int n, const deo_instance* in, int adjoin
         CUDA_TRY(cudaMemcpy(b->d_inst, b->inst.data(), n * sizeof(deo::InstDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(instances)");
     }
-    CUDA_TRY(alloc_zeroed(&b->d_counter, 2), "counters");
+    CUDA_TRY(b->claims.init(), "cudaMalloc(claim counters)");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
@@ -2997,13 +3022,16 @@ extern "C" deo_status deo_apply_each(int n, const deo_instance* in, int adjoint,
     return DEO_OK;
 }
 
-static deo_status batch_launch(deo_batch& b, cudaStream_t st) {
+// own_graph: into the batch's graph, whose launches CUDA runs one after another: a
+// captured block without the memset.
+static deo_status batch_launch(deo_batch& b, cudaStream_t st, bool own_graph = false) {
+    unsigned int* pair = nullptr;
+    if (own_graph) pair = b.claims.graph_block();
+    else if (!b.one()) CUDA_TRY(b.claims.next(st, &pair), "cudaMemsetAsync(claim counters)");
     const int e = b.one() ? deo_k_stage_one(&b.plans[0]->dev, &b.stages[0], st)
                   : b.kind == 1
-                      ? deo_k_stage_batch(b.d_stages, b.d_items, b.n_items, b.d_counter, b.lbc, b.dtype, b.ctas, 256,
-                                          st)
-                      : deo_k_batch(b.d_inst, b.d_items, b.n_items, b.d_counter, b.dtype, b.adjoint, b.lbc, b.ctas,
-                                    256, st);
+                      ? deo_k_stage_batch(b.d_stages, b.d_items, b.n_items, pair, b.lbc, b.dtype, b.ctas, 256, st)
+                      : deo_k_batch(b.d_inst, b.d_items, b.n_items, pair, b.dtype, b.adjoint, b.lbc, b.ctas, 256, st);
     if (e) return cuda_fail((cudaError_t)e, "batched launch");
     return DEO_OK;
 }
@@ -3033,7 +3061,7 @@ extern "C" deo_status deo_stage_batch_create(int n, const deo_stage* in, int til
         CUDA_TRY(cudaMemcpy(b->d_stages, b->stages.data(), n * sizeof(deo::StageDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(stages)");
     }
-    if (!b->one()) CUDA_TRY(alloc_zeroed(&b->d_counter, 2), "counters");
+    if (!b->one()) CUDA_TRY(b->claims.init(), "cudaMalloc(claim counters)");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
@@ -3045,11 +3073,11 @@ extern "C" deo_status deo_batch_run(deo_batch* b, int use_graph, void* stream) {
     if (!b) return fail(DEO_ERR_BAD_ARG, "null batch");
     if (b->n_items == 0) return DEO_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (!use_graph || b->one()) return batch_launch(*b, st);
+    if (!use_graph || b->one() || ClaimSlots::capturing(st)) return batch_launch(*b, st);
     if (!b->exec) {
         if (!b->cap) CUDA_TRY(cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking), "cudaStreamCreate");
         CUDA_TRY(cudaStreamBeginCapture(b->cap, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-        deo_status s = batch_launch(*b, b->cap);
+        deo_status s = batch_launch(*b, b->cap, true);
         cudaGraph_t g = nullptr;
         cudaError_t ec = cudaStreamEndCapture(b->cap, &g);
         if (s != DEO_OK) {

@@ -372,8 +372,8 @@ extern "C" int deo_k_apply(const deo::PlanDev* p, const void* u, void* du, int o
 // x *= f over n points (dtype 0 f64, 1 f32), stream-ordered.
 extern "C" int deo_k_scale(void* x, int64_t n, int dtype, double f, void* stream);
 // Commits k_batch's module image and launch resources on the current device
-// (one empty launch of each instantiation).  counter: two zeroed words, left zero
-// by every launch of the batched kernels.
+// (one empty launch of each instantiation).  counter, here and below: a pair of
+// claim words in a block of four (claims_done in deo_lap.cuh), zero before and after.
 extern "C" int deo_k_batch_prepare(unsigned int* counter, void* stream);
 // lbc: some instance's plan has per-line boundary conditions (the kernel
 // instantiation with that branch)

@@ -17,6 +17,7 @@
 #include <algorithm>
 
 #include "deo_eval.cuh"
+#include "deo_lap.cuh"
 
 namespace deo {
 
@@ -41,9 +42,8 @@ __global__ void __launch_bounds__(256, !ADJ && !LBC ? 8 : 0)
 // within a size class, so consecutive pulls usually share it): the header, the
 // plan's own terms and, when it has one, its star, not the whole 8-term struct.
 // The next item is claimed while the current one is evaluated (its atomic's
-// latency is covered), one barrier pair per item.  The CTA that leaves last
-// zeroes the counters, so a launch needs no memset before it: counter[0] the
-// next item, counter[1] the CTAs that have left.  Each work item is claimed in
+// latency is covered), one barrier pair per item.  The counters are those of
+// claims_done (deo_lap.cuh).  Each work item is claimed in
 // 1 << lsplit parts of a multiple of 256 points (split_for).
 struct PlanCache {
     static_assert(sizeof(PlanDev) % 8 == 0 && offsetof(PlanDev, t) % 8 == 0 && sizeof(TermDev) % 8 == 0 &&
@@ -91,13 +91,7 @@ __device__ __forceinline__ void walk_items(const WorkItem* __restrict__ items, i
         __syncthreads();  // every thread is done with the plan and has seen this item; the next claim is visible
         ph ^= 1;
     }
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(counter + 1, 1u) == gridDim.x - 1) {  // every CTA has made its last claim
-            counter[0] = 0u;
-            counter[1] = 0u;
-        }
-    }
+    claims_done(counter);
 }
 
 template <typename T, bool ADJ, bool LBC>

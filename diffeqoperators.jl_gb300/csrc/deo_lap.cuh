@@ -34,9 +34,11 @@ __device__ __forceinline__ int claim_unit(const LapGrid& g, int& s_next, int k_s
     return s_next;
 }
 
-// The marching kernels' claims: counter[0] the next unit, counter[1] the CTAs
-// that have left; the last to leave zeroes both, so a launch needs no memset
-// before it (a memset node costs about 2 us of a short apply).
+// The marching and batched kernels' claims: counter[0] the next unit, counter[1] the CTAs
+// that have left; the last to leave zeroes both, so a launch needs no memset before it
+// (a memset node costs about 2 us of a short apply).  It zeroes the other pair of its
+// block of four words too, whose turn comes half a rotation later (ClaimSlots): launches
+// that overlapped on one pair, against the rules, leave no pair wrong for good.
 __device__ __forceinline__ int claim_next(unsigned int* counter, int& s_next) {
     if (threadIdx.x == 0 && threadIdx.y == 0) s_next = (int)atomicAdd(counter, 1u);
     __syncthreads();
@@ -45,9 +47,9 @@ __device__ __forceinline__ int claim_next(unsigned int* counter, int& s_next) {
 __device__ __forceinline__ void claims_done(unsigned int* counter) {
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         __threadfence();
-        if (atomicAdd(counter + 1, 1u) == gridDim.x - 1) {
-            counter[0] = 0u;
-            counter[1] = 0u;
+        if (atomicAdd(counter + 1, 1u) == gridDim.x - 1) {  // every CTA has made its last claim
+            *reinterpret_cast<uint2*>(counter) = make_uint2(0u, 0u);
+            *reinterpret_cast<uint2*>(reinterpret_cast<uintptr_t>(counter) ^ 8) = make_uint2(0u, 0u);
         }
     }
 }

@@ -495,7 +495,7 @@ deo_status deo_batch_create(int n, const deo_instance* inst, int adjoint, int ti
  * baseline the batched launch is measured against. */
 deo_status deo_apply_each(int n, const deo_instance* inst, int adjoint, void* stream);
 /* Runs the batch; with use_graph = 1 the launch is captured once into a CUDA
- * graph and replayed.
+ * graph and replayed (on a stream under capture it is captured as it is).
  * A stage batch of one instance is one launch with its arguments either way. */
 deo_status deo_batch_run(deo_batch* b, int use_graph, void* stream);
 /* Re-point instance i at new buffers (same plan); invalidates the graph. */
