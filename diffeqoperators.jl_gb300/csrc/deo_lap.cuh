@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "deo_internal.h"
+#include "deo_once.h"
 
 namespace deo {
 
@@ -123,24 +124,33 @@ static inline LapGrid march_chunks(int64_t nx, int64_t ny, int nz, int tx, int t
     return g;
 }
 
-template <typename K>
-static inline int occupancy_grid(K kernel, int threads, int smem, int64_t& G) {
-    static thread_local int dummy = 0;
-    (void)dummy;
-    int dev = 0, sms = 0, per_sm = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    // the largest shared-memory carveout: an SM configured for the interior's CTAs alone would leave
-    // no room for the boundary-shell CTAs that run beside them
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
+// The resident grid of a kernel's instantiations, which run with one grid (that of the
+// last), found once per device: `known` is a static of the launcher.
+template <typename... K>
+static inline int occupancy_grid(PerDevice<int64_t>& known, int threads, int smem, int64_t& G, K... kernels) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-    if (e != cudaSuccess || per_sm < 1) per_sm = 1;
-    G = (int64_t)sms * per_sm;
-    return 0;
+    return known.get(dev, G, [&](int64_t& grid) {
+        auto one = [&](auto kernel) {
+            int sms = 0, per_sm = 0;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            // the largest shared-memory carveout: an SM configured for the interior's CTAs alone would leave
+            // no room for the boundary-shell CTAs that run beside them
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                         (int)cudaSharedmemCarveoutMaxShared);
+            if (e != cudaSuccess) return (int)e;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+            if (e != cudaSuccess || per_sm < 1) per_sm = 1;
+            grid = (int64_t)sms * per_sm;
+            return 0;
+        };
+        int err = 0;
+        ((err = err ? err : one(kernels)), ...);
+        return err;
+    });
 }
 
 

@@ -307,12 +307,11 @@ template <int H, bool SH, int TYT, int RY>
 int launch(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du, int ow,
            cudaStream_t st) {
     using C = march::Cfg<H, TYT, RY>;
-    static int64_t G = 0;
-    if (!G) {
-        int e = occupancy_grid(march::k_lap_fx<H, SH, true, TYT, RY>, C::NTHR, C::SMEM, G);
-        if (!e) e = occupancy_grid(march::k_lap_fx<H, SH, false, TYT, RY>, C::NTHR, C::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::NTHR, C::SMEM, G,
+                                  march::k_lap_fx<H, SH, true, TYT, RY>, march::k_lap_fx<H, SH, false, TYT, RY>);
+    if (eg) return eg;
     LapGrid g = march_chunks(up->n[0], up->n[1], B->hi[2] - B->lo[2] + 1, C::TX, C::TY, H, G);
     g.sched = sched;
     const int grid = (int)std::min<int64_t>(G, g.units);

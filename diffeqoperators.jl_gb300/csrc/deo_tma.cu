@@ -934,11 +934,10 @@ static int launch_tma(const UniPlan* up, const PlanDev* dp, const void* u, void*
     using C = TmaCfg<T, H>;
     CUtensorMap map;
     if (!make_map(map, u, C::ES, up->n[0], up->n[1], up->n[2], C::BX, C::BY)) return (int)cudaErrorNotSupported;
-    static int64_t G = 0;
-    if (!G) {
-        const int e = occupancy_grid(k_lap_tma<T, H, NT, ENS>, C::TX * C::TY, C::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::TX * C::TY, C::SMEM, G, k_lap_tma<T, H, NT, ENS>);
+    if (eg) return eg;
     const LapGrid g = make_grid(up, C::TX, C::TY, H, NT, G);
     const int grid = (int)std::min<int64_t>(G, g.units);
     k_lap_tma<T, H, NT, ENS><<<grid, dim3(C::TX, C::TY), C::SMEM, st>>>(map, *up, g, dp, (const T*)u, (T*)du, ow);
@@ -951,11 +950,10 @@ static int launch_ens2(const UniPlan* up, const PlanDev* dp, const void* u, void
     using E = Ens2Cfg<H>;
     CUtensorMap map;
     if (!make_map(map, u, 8, up->n[0], up->n[1], up->n[2], C::BX, C::BY)) return (int)cudaErrorNotSupported;
-    static int64_t G = 0;
-    if (!G) {
-        const int e = occupancy_grid(k_lap_ens2<H, NT>, C::TX * C::TY, E::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::TX * C::TY, E::SMEM, G, k_lap_ens2<H, NT>);
+    if (eg) return eg;
     const LapGrid g = make_grid(up, C::TX, C::TY, H, NT, G);
     const int grid = (int)std::min<int64_t>(G, g.units);
     k_lap_ens2<H, NT><<<grid, dim3(C::TX, C::TY), E::SMEM, st>>>(map, *up, g, dp, (const double*)u, (double*)du, ow);
@@ -967,12 +965,11 @@ static int launch_q(const UniPlan* up, unsigned int* sched, const void* u, void*
     using C = QCfg<T, H>;
     CUtensorMap map;
     if (!make_map(map, u, C::ES, up->n[0], up->n[1], up->n[2], C::BX, C::BY)) return (int)cudaErrorNotSupported;
-    static int64_t G = 0;
-    if (!G) {
-        int e = occupancy_grid(k_lap_q<T, H, NT, true>, C::TX * C::TYT, C::SMEM, G);
-        if (!e) e = occupancy_grid(k_lap_q<T, H, NT, false>, C::TX * C::TYT, C::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::TX * C::TYT, C::SMEM, G,
+                                  k_lap_q<T, H, NT, true>, k_lap_q<T, H, NT, false>);
+    if (eg) return eg;
     const LapGrid g = make_grid(up, C::TX, C::TY, H, NT, G);
     LapGrid g2 = g;
     g2.sched = sched;
@@ -1036,11 +1033,10 @@ static int launch_fx(const UniPlan* up, unsigned int* sched, const void* u, void
     using F = FxCfg<H>;
     CUtensorMap map;
     if (!make_map(map, u, 8, up->n[0], up->n[1], up->n[2], C::BX, C::BY)) return (int)cudaErrorNotSupported;
-    static int64_t G = 0;
-    if (!G) {
-        const int e = occupancy_grid(k_lap_fx<H, NT>, C::TX * C::TY, F::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::TX * C::TY, F::SMEM, G, k_lap_fx<H, NT>);
+    if (eg) return eg;
     const LapGrid g = make_grid(up, C::TX, C::TY, H, NT, G);
     LapGrid g2 = g;
     g2.sched = sched;
@@ -1058,11 +1054,10 @@ static int launch_bfx(const UniPlan* up, unsigned int* sched, const void* u, voi
     using C = BfxCfg<H>;
     CUtensorMap map;
     if (!make_map(map, u, 8, up->n[0], up->n[1], up->n[2], C::BX, C::BY)) return (int)cudaErrorNotSupported;
-    static int64_t G = 0;
-    if (!G) {
-        const int e = occupancy_grid(k_lap_bfx<H, CNEG>, C::NTHR, C::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::NTHR, C::SMEM, G, k_lap_bfx<H, CNEG>);
+    if (eg) return eg;
     const LapGrid g = make_grid(up, C::TX, C::TY, H, 3, G);
     LapGrid g2 = g;
     g2.sched = sched;

@@ -236,12 +236,11 @@ int launch_v(const UniPlan* up, unsigned int* sched, const void* u, void* du, in
     alignas(64) CUtensorMap map;
     if (deo_k_encode_map3(&map, u, 4, up->n[0], up->n[1], up->n[2], C::BX, C::BY, 1))
         return (int)cudaErrorNotSupported;
-    static int64_t G = 0;
-    if (!G) {
-        int e = occupancy_grid(k_lap_v<H, NT, true, TYT, RYB>, C::NTHR, C::SMEM, G);
-        if (!e) e = occupancy_grid(k_lap_v<H, NT, false, TYT, RYB>, C::NTHR, C::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::NTHR, C::SMEM, G,
+                                  k_lap_v<H, NT, true, TYT, RYB>, k_lap_v<H, NT, false, TYT, RYB>);
+    if (eg) return eg;
     const LapGrid g = make_grid(up, C::TX, C::TY, H, NT, G);
     LapGrid g2 = g;
     g2.sched = sched;

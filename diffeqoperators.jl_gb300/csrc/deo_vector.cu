@@ -690,12 +690,10 @@ __global__ void __launch_bounds__(256) k_cross(int64_t npts, const T* __restrict
 template <int KIND, int NK>
 int launch_fx(const VcDev& V, const VcBfp& B, unsigned int* claims, const double* M, double* out, int ow, cudaStream_t st) {
     using C = VfCfg<KIND, NK>;
-    static int64_t G = 0;
-    if (!G) {
-        int e = occupancy_grid(k_vc_fx<KIND, NK, true>, C::NTHR, C::SMEM, G);
-        if (!e) e = occupancy_grid(k_vc_fx<KIND, NK, false>, C::NTHR, C::SMEM, G);
-        if (e) return e;
-    }
+    static PerDevice<int64_t> known;
+    int64_t G;
+    const int eg = occupancy_grid(known, C::NTHR, C::SMEM, G, k_vc_fx<KIND, NK, true>, k_vc_fx<KIND, NK, false>);
+    if (eg) return eg;
     LapGrid g = march_chunks(V.len[0], V.len[1], (int)V.len[2] - 2 * V.bpc, 64, C::TY, NK / 2, G);
     g.sched = claims;
     const int grid = (int)std::min<int64_t>(G, g.units);
