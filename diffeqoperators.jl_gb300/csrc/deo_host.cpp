@@ -2219,6 +2219,10 @@ extern "C" deo_status deo_plan_host_sync(deo_plan* p) {
 // block fixed point (long bands gain, short ones lose); at 2^17 all gain
 // (4.1 .. 11.7 -> 3.7 .. 7.0).
 constexpr int kNldFxMinPoints = 1 << 17;
+// Most rows outside the bands: one for each thread of the block that takes them.  (2^18
+// points, steps of np.diff(linspace) or of two sizes: 3.9 ms through that block, 0.63 ms
+// by the row tables.)
+constexpr int kNldFxMaxRows = 128;
 
 struct deo_nld {
     deo_plan* plan = nullptr;
@@ -2263,7 +2267,9 @@ static void nld_bands(deo_nld* N) {
         if (!band(N->m + k, B.q[k], B.tq)) return;
     for (int k = 1; k <= N->n; ++k)
         if (!band(k, B.p[k - 1], B.tp)) return;
-    B.ok = 1;
+    // the rows outside the band go one by one through the kernel's first block: the boundary's,
+    // not those of a line whose steps differ somewhere
+    B.ok = B.lo + N->len - B.hi <= kNldFxMaxRows;
 }
 
 extern "C" deo_status deo_nonlinear_diffusion_plan(int second_order, int first_order, int approx_order,
