@@ -1811,11 +1811,21 @@ static void mark(const deo_plan* p, int k, void* stream) {
 // against 20 / 32; transposed 97^3 26.5 / 43.4 against 28.4 / 44.9.  Even sizes march
 // at every size (tiled kernels before: 16^3 18 us against 9, 64^3 21 against 12).
 constexpr int64_t kMarchMinOddPoints = 300000, kMarchMinOddAdjoint = 1 << 20;
+// Nor with a small interior: the points outside the marching kernel's box take one thread
+// each in the shell, twice the generic kernel's time a point.  255 x 160 x 128, order 2 / 4,
+// generic against marching: graded over 12 points at both ends of axes 2 and 3 (0.69 of the
+// points inside) 148 / 201 us against 135 / 179; two step sizes along an axis (half) 149 /
+// 203 against 173-192 / 208-240; few equal rows 155 / 209 against 263 / 293.
+static bool mostly_inside(const deo_plan* p) {
+    int64_t in = 1;
+    for (int a = 0; a < 3; ++a) in *= std::max(p->march.hi[a] - p->march.lo[a] + 1, 0);
+    return 3 * in >= 2 * p->dev.total;
+}
 static bool use_march(const deo_plan* p, bool adjoint = false) {
     return p->march.ok && p->exact_sums == 1 && p->fast_path && p->use_tma && !p->fx_rows_set &&
            !p->uni.test_withhold &&
            (p->sums_set || p->dev.sizes[0] % 2 == 0 ||
-            p->dev.total >= (adjoint ? kMarchMinOddAdjoint : kMarchMinOddPoints));
+            (p->dev.total >= (adjoint ? kMarchMinOddAdjoint : kMarchMinOddPoints) && mostly_inside(p)));
 }
 // 2-D Float64 Laplacians by default: k_rows_fx, or the generic kernel below its size;
 // of the tiled kernels, which split such a plan into an interior and a shell launch,
