@@ -1736,7 +1736,11 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
     }
     CUDA_TRY(cudaMalloc(&P->d_plan, sizeof(PlanDev)), "cudaMalloc(plan)");
     CUDA_TRY(cudaMemcpy(P->d_plan, &P->dev, sizeof(PlanDev), cudaMemcpyHostToDevice), "cudaMemcpy(plan)");
-    if (P->march.ok) CUDA_TRY(P->claims.init(), "cudaMalloc(claim counters)");
+    if (P->march.ok) {
+        CUDA_TRY(P->claims.init(), "cudaMalloc(claim counters)");
+        const int planes = P->march.hi[2] - P->march.lo[2] + 1;
+        CUDA_TRY((cudaError_t)deo_k_march_chunk(&P->uni, &P->march, planes, &P->march.zc), "marching kernel");
+    }
     if (P->shell.ok && P->uni.enabled && P->uni.lap) {
         CUDA_TRY(cudaMalloc(&P->d_shell, sizeof(deo::ShellPlan)), "cudaMalloc(shell rows)");
         CUDA_TRY(cudaMemcpy(P->d_shell, &P->shell, sizeof(deo::ShellPlan), cudaMemcpyHostToDevice),
@@ -1762,6 +1766,9 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
                 P->adj_hi[a] = hi;
             }
             P->adj_ok = ok ? 1 : 0;
+            if (ok && P->march.ok)
+                CUDA_TRY((cudaError_t)deo_k_march_chunk(&P->uni, &P->march, P->adj_hi[2] - P->adj_lo[2] + 1, &P->march.zc_rev),
+                         "marching kernel");
         }
         CUDA_TRY(cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming), "cudaEventCreate");
         CUDA_TRY(cudaEventCreateWithFlags(&P->ev_join, cudaEventDisableTiming), "cudaEventCreate");
@@ -2104,6 +2111,7 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
             reverse_taps(B.wl[a], K);
         }
         B.limit = B.rev;
+        B.zc = B.zc_rev;
         const int e = interior_then_shell(
             p, p->concurrent && p->side && (ua.radius == 1 || p->dev.total <= kAdjBesideMaxPoints), stream,
             [&] {
@@ -2431,7 +2439,10 @@ extern "C" deo_status deo_vector_calculus_plan(int kind, int ndims, const deo_op
             V->bfp.t0 = std::max(V->bfp.t0, bfp_threshold(total, (double)W(mid + 1), 1.0));
             V->bfp.kbase[a] = 57 - s - 1075 - 6;
         }
-        if (V->bfp.ok) CUDA_TRY(V->claims.init(), "cudaMalloc(claim counters)");
+        if (V->bfp.ok) {
+            CUDA_TRY(V->claims.init(), "cudaMalloc(claim counters)");
+            CUDA_TRY((cudaError_t)deo_k_vector_chunk(&D, &V->bfp.zc), "marching kernel");
+        }
         // k_vc_fx from here on (units of 64 x 8 columns and their queues want a full chip):
         // gradient, order 2 / 4, k_vc against k_vc_fx: 80^3 16 / 23 against 17 / 33 us, 100^3
         // 31 / 45 against 22 / 38; curl 128^3 100 / 141 against 87 / 146, 160^3 187 / 270

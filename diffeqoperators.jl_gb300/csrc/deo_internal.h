@@ -191,6 +191,7 @@ struct BfpMarch {
     struct Limit {
         int t, sh0, sh1;
     } limit, rev;
+    int zc, zc_rev;       // planes of a unit; of the transpose's box
     int kbase;            // the sum in units of 2^57 times 2^(kbase + E) is the result
 };
 
@@ -307,6 +308,7 @@ struct VcBfp {
     int wh[3][5], wl[3][5], wd[3][5];
     int t0;  // a derivative is accepted when the larger of its two nearest taps' high limbs reaches this
     int kbase[3];
+    int zc;  // planes of a unit
 };
 
 // One derivative of nonlinear_diffusion! in block fixed point: the limbs [o]
@@ -335,6 +337,8 @@ extern "C" int deo_k_nld_fx(const deo::NldBfp* B, const deo::PlanDev* d_plan, in
 // not overlap M.  overwrite = 1 writes A*M, 0 adds it to out (mul!).
 extern "C" int deo_k_vector_calculus(const deo::VcDev* V, const deo::VcBfp* B, unsigned int* claims, int dtype,
                                      const void* M, void* out, int overwrite, void* stream);
+// The planes of its units (for B.zc), V.kind's kernel of V.band_nk taps.
+extern "C" int deo_k_vector_chunk(const deo::VcDev* V, int* zc);
 // L*M on a padded array: V.t[0] is the operator's table (generic methods),
 // V.len the output size, V.pstride M's strides; coff the offset of the
 // stripped edge planes of M's other axes.
@@ -425,6 +429,8 @@ extern "C" int deo_k_apply_vec(const deo::UniPlan* up, unsigned int* sched, cons
 // Float64 interior in block fixed point, marching along axis 3 (deo_march.cu)
 extern "C" int deo_k_apply_march(const deo::UniPlan* up, const deo::BfpMarch* B, unsigned int* sched, const void* u,
                                  void* du, int overwrite, void* stream);
+// The planes of its units over a box of `planes` (for B.zc)
+extern "C" int deo_k_march_chunk(const deo::UniPlan* up, const deo::BfpMarch* B, int planes, int* zc);
 // A 2-D Float64 plan in block fixed point (deo_rowsfx.cu)
 extern "C" int deo_k_rows_fx(const deo::BfpPlan2* B, const deo::PlanDev* d_plan, const void* u, void* du, int overwrite,
                              void* stream);

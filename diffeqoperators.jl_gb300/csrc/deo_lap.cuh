@@ -97,29 +97,34 @@ static inline LapGrid make_grid(const UniPlan* up, int tx, int ty, int H, int nt
     return g;
 }
 
-// Units of (tile, chunk of nz planes) for the marching block fixed-point kernels
-// with G resident CTAs that share them out.  A unit of zc planes costs about
+// The chunk of nz planes of the marching block fixed-point kernels, whose units of (tile,
+// chunk) G resident CTAs share out.  A unit of zc planes costs about
 // zc + 0.4 * 2H + 3 planes (the planes that only fill the ring are converted, not
 // evaluated), and the last round leaves about a third of a unit idle.  A queued
-// point holds its plane in 8 bits, so zc <= 256.
-static inline LapGrid march_chunks(int64_t nx, int64_t ny, int nz, int tx, int ty, int H, int64_t G) {
-    LapGrid g{};
-    g.tiles_x = (int)((nx + tx - 1) / tx);
-    g.tiles_y = (int)((ny + ty - 1) / ty);
-    const int64_t tiles = (int64_t)g.tiles_x * g.tiles_y;
+// point holds its plane in 8 bits, so zc <= 256.  Searched once, when a plan is made.
+static inline int march_zc(int64_t nx, int64_t ny, int nz, int tx, int ty, int H, int64_t G) {
+    const int64_t tiles = ((nx + tx - 1) / tx) * ((ny + ty - 1) / ty);
+    int found = 1;
     double best = 1e300;
-    for (int c = (nz + 255) / 256; c <= nz; ++c) {
-        const int zc = (nz + c - 1) / c;
+    for (int c = (nz + 255) / 256, zc; c <= nz; c = (nz + zc - 2) / (zc - 1)) {  // (the next shorter chunk)
+        zc = (nz + c - 1) / c;
         const double rounds = std::max(1.0, (double)(tiles * ((nz + zc - 1) / zc)) / (double)G + 0.35);
         const double t = rounds * (zc + 0.8 * H + 3.0);
         if (t < best) {
             best = t;
-            g.zc = zc;
+            found = zc;
         }
         if (zc <= 4) break;
     }
-    g.chunks = (nz + g.zc - 1) / g.zc;
-    g.units = (int)(tiles * g.chunks);
+    return found;
+}
+static inline LapGrid march_grid(int64_t nx, int64_t ny, int nz, int tx, int ty, int zc) {
+    LapGrid g{};
+    g.tiles_x = (int)((nx + tx - 1) / tx);
+    g.tiles_y = (int)((ny + ty - 1) / ty);
+    g.zc = zc;
+    g.chunks = (nz + zc - 1) / zc;
+    g.units = (int)((int64_t)g.tiles_x * g.tiles_y * g.chunks);
     g.perm = 1;
     return g;
 }

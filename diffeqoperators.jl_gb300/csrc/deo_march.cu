@@ -303,41 +303,59 @@ using namespace deo;
 
 namespace {
 
-template <int H, bool SH, int TYT, int RY>
-int launch(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du, int ow,
-           cudaStream_t st) {
+template <int H, bool SH, int TYT = 4, int RY = 2>
+struct Kernel {
     using C = march::Cfg<H, TYT, RY>;
-    static PerDevice<int64_t> known;
-    int64_t G;
-    const int eg = occupancy_grid(known, C::NTHR, C::SMEM, G,
-                                  march::k_lap_fx<H, SH, true, TYT, RY>, march::k_lap_fx<H, SH, false, TYT, RY>);
-    if (eg) return eg;
-    LapGrid g = march_chunks(up->n[0], up->n[1], B->hi[2] - B->lo[2] + 1, C::TX, C::TY, H, G);
-    g.sched = sched;
-    const int grid = (int)std::min<int64_t>(G, g.units);
-    const int pairs = up->n[0] % 2 == 0 && (uintptr_t)du % 16 == 0;  // 16-byte stores
-    auto go = [&](auto kernel) {
-        kernel<<<grid, dim3(32, TYT), C::SMEM, st>>>(*up, *B, g, (const double*)u, (double*)du, pairs);
-    };
-    if (ow) go(march::k_lap_fx<H, SH, true, TYT, RY>);
-    else go(march::k_lap_fx<H, SH, false, TYT, RY>);
-    return (int)cudaGetLastError();
+    static int resident(int64_t& G) {
+        static PerDevice<int64_t> known;
+        return occupancy_grid(known, C::NTHR, C::SMEM, G, march::k_lap_fx<H, SH, true, TYT, RY>,
+                              march::k_lap_fx<H, SH, false, TYT, RY>);
+    }
+    static int chunk(const UniPlan* up, int planes, int* zc) {
+        int64_t G;
+        const int e = resident(G);
+        if (!e) *zc = march_zc(up->n[0], up->n[1], planes, C::TX, C::TY, H, G);
+        return e;
+    }
+    static int launch(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du, int ow,
+                      cudaStream_t st) {
+        int64_t G;
+        const int e = resident(G);
+        if (e) return e;
+        LapGrid g = march_grid(up->n[0], up->n[1], B->hi[2] - B->lo[2] + 1, C::TX, C::TY, B->zc);
+        g.sched = sched;
+        const int grid = (int)std::min<int64_t>(G, g.units);
+        const int pairs = up->n[0] % 2 == 0 && (uintptr_t)du % 16 == 0;  // 16-byte stores
+        auto go = [&](auto kernel) {
+            kernel<<<grid, dim3(32, TYT), C::SMEM, st>>>(*up, *B, g, (const double*)u, (double*)du, pairs);
+        };
+        if (ow) go(march::k_lap_fx<H, SH, true, TYT, RY>);
+        else go(march::k_lap_fx<H, SH, false, TYT, RY>);
+        return (int)cudaGetLastError();
+    }
+};
+
+// f(the kernel of a plan's radius and bands)
+template <typename F>
+int pick(const UniPlan* up, const BfpMarch* B, F f) {
+    switch (up->radius) {
+        case 1: return B->shared ? f(Kernel<1, true>{}) : f(Kernel<1, false>{});
+        case 2: return B->shared ? f(Kernel<2, true>{}) : f(Kernel<2, false>{});
+        case 3: return B->shared ? f(Kernel<3, true>{}) : f(Kernel<3, false>{});
+    }
+    return (int)cudaErrorNotSupported;
 }
 
 }  // namespace
+
+extern "C" int deo_k_march_chunk(const UniPlan* up, const BfpMarch* B, int planes, int* zc) {
+    return planes < 1 ? 0 : pick(up, B, [&](auto k) { return k.chunk(up, planes, zc); });
+}
 
 extern "C" int deo_k_apply_march(const UniPlan* up, const BfpMarch* B, unsigned int* sched, const void* u, void* du,
                                  int overwrite, void* stream) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     for (int a = 0; a < 3; ++a)
         if (B->lo[a] > B->hi[a]) return 0;  // no interior point
-    switch (up->radius) {
-        case 1: return B->shared ? launch<1, true, 4, 2>(up, B, sched, u, du, overwrite, st)
-                                 : launch<1, false, 4, 2>(up, B, sched, u, du, overwrite, st);
-        case 2: return B->shared ? launch<2, true, 4, 2>(up, B, sched, u, du, overwrite, st)
-                                 : launch<2, false, 4, 2>(up, B, sched, u, du, overwrite, st);
-        case 3: return B->shared ? launch<3, true, 4, 2>(up, B, sched, u, du, overwrite, st)
-                                 : launch<3, false, 4, 2>(up, B, sched, u, du, overwrite, st);
-    }
-    return (int)cudaErrorNotSupported;
+    return pick(up, B, [&](auto k) { return k.launch(up, B, sched, u, du, overwrite, st); });
 }

@@ -688,19 +688,42 @@ __global__ void __launch_bounds__(256) k_cross(int64_t npts, const T* __restrict
 }
 
 template <int KIND, int NK>
-int launch_fx(const VcDev& V, const VcBfp& B, unsigned int* claims, const double* M, double* out, int ow, cudaStream_t st) {
+int resident_fx(int64_t& G) {
     using C = VfCfg<KIND, NK>;
     static PerDevice<int64_t> known;
+    return occupancy_grid(known, C::NTHR, C::SMEM, G, k_vc_fx<KIND, NK, true>, k_vc_fx<KIND, NK, false>);
+}
+
+template <int KIND, int NK>
+int launch_fx(const VcDev& V, const VcBfp& B, unsigned int* claims, const double* M, double* out, int ow, cudaStream_t st) {
+    using C = VfCfg<KIND, NK>;
     int64_t G;
-    const int eg = occupancy_grid(known, C::NTHR, C::SMEM, G, k_vc_fx<KIND, NK, true>, k_vc_fx<KIND, NK, false>);
-    if (eg) return eg;
-    LapGrid g = march_chunks(V.len[0], V.len[1], (int)V.len[2] - 2 * V.bpc, 64, C::TY, NK / 2, G);
+    const int e = resident_fx<KIND, NK>(G);
+    if (e) return e;
+    LapGrid g = march_grid(V.len[0], V.len[1], (int)V.len[2] - 2 * V.bpc, 64, C::TY, B.zc);
     g.sched = claims;
     const int grid = (int)std::min<int64_t>(G, g.units);
     auto go = [&](auto kernel) { kernel<<<grid, dim3(32, C::TYT), C::SMEM, st>>>(V, B, g, M, out); };
     if (ow) go(k_vc_fx<KIND, NK, true>);
     else go(k_vc_fx<KIND, NK, false>);
     return (int)cudaGetLastError();
+}
+
+template <int KIND>
+int chunk_fx(const VcDev& V, int* zc) {
+    auto find = [&](auto nk) {
+        constexpr int NK = decltype(nk)::value;
+        int64_t G;
+        const int e = resident_fx<KIND, NK>(G);
+        if (!e) *zc = march_zc(V.len[0], V.len[1], (int)V.len[2] - 2 * V.bpc, 64, VfCfg<KIND, NK>::TY, NK / 2, G);
+        return e;
+    };
+    switch (V.band_nk) {
+        case 3: return find(std::integral_constant<int, 3>{});
+        case 5: return find(std::integral_constant<int, 5>{});
+        case 7: return find(std::integral_constant<int, 7>{});
+    }
+    return 0;  // (9 taps: not this kernel)
 }
 
 template <typename T, int KIND, int ND>
@@ -763,6 +786,12 @@ int launch_vc(const VcDev& V, const VcBfp* B, unsigned int* claims, const void* 
 
 }  // namespace
 }  // namespace deo
+
+extern "C" int deo_k_vector_chunk(const deo::VcDev* V, int* zc) {
+    return V->kind == DEO_VC_GRADIENT     ? deo::chunk_fx<DEO_VC_GRADIENT>(*V, zc)
+           : V->kind == DEO_VC_DIVERGENCE ? deo::chunk_fx<DEO_VC_DIVERGENCE>(*V, zc)
+                                          : deo::chunk_fx<DEO_VC_CURL>(*V, zc);
+}
 
 extern "C" int deo_k_vector_calculus(const deo::VcDev* V, const deo::VcBfp* B, unsigned int* claims, int dtype,
                                      const void* M, void* out, int overwrite, void* stream) {

@@ -2,6 +2,8 @@
 replayed on one stream beside direct calls on another, as many captured calls as there
 are counters, and a batch run directly on two streams at once.  Every output is complete,
 then and in every later call."""
+import gc
+
 import numpy as np
 import pytest
 
@@ -42,6 +44,7 @@ def test_replays_beside_direct_calls(cuda, kind):
     run(want)
     torch.cuda.synchronize()
     want = want.clone()
+    gc.collect()  # (a plan of an earlier test freed during the capture would end it)
     graph, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
     with torch.cuda.graph(graph, stream=s):
         for _ in range(1024):
