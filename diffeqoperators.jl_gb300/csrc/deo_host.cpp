@@ -768,6 +768,26 @@ static deo_status compile_rows(long len, Row make, HostTab& T, std::vector<int>&
     return DEO_OK;
 }
 
+// Row i (1-based) of a Float64 table.
+static RowSpec table_row(const HostTab& H, long i) {
+    const RowTabDev& d = H.dev;
+    const bool band = i >= d.ilo && i <= d.ihi;
+    const long e = i < d.ilo ? i - 1 : i - 1 - (d.ihi - d.ilo + 1);
+    RowSpec r;
+    r.p0 = band ? (int)i + d.band_p0_off : H.p0[e];
+    r.nk = band ? d.band_nk : H.nk[e];
+    r.cidx = band ? (int)i + d.band_cidx_off : H.cidx[e];
+    for (int k = 0; k < r.nk; ++k) r.w[k] = band ? d.wband[k] : H.W[(size_t)k * d.nexp + e];
+    return r;
+}
+// What a 2-D plan's rows in block fixed point are built from (build_rows2).
+struct Rows2Term {
+    int axis, wind, stl;
+    const double* field;
+    deo_bc bc;
+    HostTab tab[2];
+};
+
 // Rows [lo, hi] of one shape: p0 = i + off, nk taps, weights from the band or (rows)
 // from entry i + e0 of the explicit rows, whichever range is longer.
 struct RowRange {
@@ -888,6 +908,7 @@ struct deo_plan {
     deo::UniPlan uni{};
     deo::BfpMarch march{};      // 3-D Float64: the marching block fixed-point interior (ok = 0: not this plan)
     deo::BfpPlan2 rows2{};      // 2-D Float64: the terms' rows in block fixed point (ok = 0: not this plan)
+    std::vector<Rows2Term> later_rows;  // or what they are built from
     int fx_rows_set = 0;        // DEO_OPT_FX_FP64_ROWS was set: the caller wants the per-point kernel's rows
     deo::ShellPlan shell{};
     int fast_path = 1;   // DEO_OPT_FAST_PATH
@@ -1279,17 +1300,16 @@ struct FoldedRow {
         return last >= 0 && !far && std::isfinite(b);
     }
 };
-// One axis's rows as integer windows appended to the blob; false when a window
-// is too wide or reaches outside the halo.
-static bool pack_rows(const std::vector<FoldedRow>& rows, int K, int KP, int halo, std::vector<int>& blob, size_t& w_at,
-                      size_t& meta_at) {
-    const long n = (long)rows.size();
+// One axis's n rows, row(i) in order, as integer windows appended to the blob; false when a
+// window is too wide or reaches outside the halo.
+template <typename RowAt>
+static bool pack_rows(long n, RowAt row, int K, int KP, int halo, std::vector<int>& blob, size_t& w_at, size_t& meta_at) {
     const int A = (K - 2) / 2, Z = K - 1 - A;
     w_at = blob.size();
     meta_at = w_at + (size_t)n * KP * 2;
     blob.resize(meta_at + (size_t)n * 4, 0);
     for (long i = 0; i < n; ++i) {
-        const FoldedRow& R = rows[i];
+        const FoldedRow R = row(i);
         long lo, hi;
         if (!R.window(lo, hi) || hi - lo + 1 > K) return false;
         double sum = 0.0;
@@ -1320,51 +1340,67 @@ static bool pack_rows(const std::vector<FoldedRow>& rows, int K, int KP, int hal
     }
     return true;
 }
-static deo_status build_rows2(deo_plan& P, const int64_t* sizes, int nterms, const deo_term* terms) {
+// The smallest plan of these terms that takes k_rows_fx by itself.
+static int64_t rows_fx_min(int nterms, const deo_term* terms) {
+    for (int t = 0; t < nterms; ++t)
+        if (terms[t].coeff_field) return kRowsFxMinFieldPoints;
+    return kRowsFxMinPoints;
+}
+static bool rows2_terms(const int64_t* sizes, int nterms, const deo_term* terms) {
+    return sizes[0] >= 32 && sizes[1] >= 32 && sizes[0] <= (1 << 20) && (sizes[1] + 31) / 32 <= 65535 &&
+           std::none_of(terms, terms + nterms, [](const deo_term& t) { return t.line_bcs != nullptr; });
+}
+static deo_status build_rows2(deo_plan& P, const int64_t* sizes, const std::vector<Rows2Term>& terms) {
     deo::BfpPlan2 B{};
-    if (sizes[0] < 32 || sizes[1] < 32 || sizes[0] > (1 << 20) || (sizes[1] + 31) / 32 > 65535) return DEO_OK;
-    std::vector<FoldedRow> ax[2], f[2];
-    for (int t = 0; t < nterms; ++t) {
-        const deo_term& tm = terms[t];
-        const int a = tm.axis - 1, mode = tm.path == DEO_PATH_PADDED ? 1 : 0;
-        if (tm.line_bcs) return DEO_OK;
-        const long n = (long)sizes[a];
-        const deo_operator& op = *tm.op;
-        if (tm.coeff_field) {
-            if (!op.wind || a != 0 || B.field || op.stl > 4) return DEO_OK;
-            B.field = static_cast<const double*>(tm.coeff_field);
-            for (int v = 0; v < 2; ++v) {
-                f[v].resize(n);
-                for (long i = 0; i < n; ++i) {
-                    const RowSpec r = build_row(op, mode, false, v == 0 ? 1.0 : -1.0, i + 1);
-                    if (r.cidx != (int)i + 1) return DEO_OK;  // the field's value at the point itself
-                    f[v][i].fold(r, *tm.bc, i, n);
-                }
-            }
-        } else {
-            ax[a].resize(n);
-            for (long i = 0; i < n; ++i) ax[a][i].fold(build_row(op, mode, true, 1.0, i + 1), *tm.bc, i, n);
+    const Rows2Term* field = nullptr;
+    std::vector<const Rows2Term*> plain[2];
+    for (const Rows2Term& tm : terms) {
+        if (!tm.field) {
+            plain[tm.axis].push_back(&tm);
+            continue;
         }
+        if (!tm.wind || tm.axis != 0 || field || tm.stl > 4) return DEO_OK;
+        field = &tm;
     }
-    if (B.field && ax[0].empty()) return DEO_OK;  // (instantiated with plain terms along axis 1)
+    if (field && plain[0].empty()) return DEO_OK;  // (instantiated with plain terms along axis 1)
+    auto fold = [&](int a, long i) {  // row i of an axis's plain terms
+        FoldedRow R{};
+        for (const Rows2Term* t : plain[a]) R.fold(table_row(t->tab[0], i + 1), t->bc, i, (long)sizes[a]);
+        return R;
+    };
+    // the widest window; the rows are kept for packing up to 19 MB of them
+    std::vector<FoldedRow> kept[2];
     long wide = 0;
-    for (const auto& rows : ax)
-        for (const FoldedRow& R : rows) {
+    for (int a = 0; a < 2; ++a)
+        for (long i = 0; i < (plain[a].empty() ? 0 : (long)sizes[a]); ++i) {
+            const FoldedRow R = fold(a, i);
             long lo, hi;
-            if (!R.window(lo, hi)) return DEO_OK;
+            if (!R.window(lo, hi) || hi - lo + 1 > 9) return DEO_OK;
             wide = std::max(wide, hi - lo + 1);
+            if (sizes[a] <= 65536) kept[a].push_back(R);
         }
-    if (wide > 9) return DEO_OK;
     B.K = std::max(3, (int)(wide | 1));
     B.n[0] = (int)sizes[0];
     B.n[1] = (int)sizes[1];
-    const int hk = (B.K - 1) / 2, hx = B.field ? std::max(hk, 3) : hk;
+    const int hk = (B.K - 1) / 2, hx = field ? std::max(hk, 3) : hk;
     std::vector<int> blob;
     size_t at[4][2] = {};
-    for (int a = 0; a < 2; ++a)
-        if (!ax[a].empty() && !pack_rows(ax[a], B.K, B.K + 1, a == 0 ? hx : hk, blob, at[a][0], at[a][1])) return DEO_OK;
-    for (int v = 0; v < 2 && B.field; ++v)
-        if (!pack_rows(f[v], 4, 4, hx, blob, at[2 + v][0], at[2 + v][1])) return DEO_OK;
+    for (int a = 0; a < 2; ++a) {
+        if (plain[a].empty()) continue;
+        auto row = [&](long i) { return kept[a].empty() ? fold(a, i) : kept[a][i]; };
+        if (!pack_rows((long)sizes[a], row, B.K, B.K + 1, a == 0 ? hx : hk, blob, at[a][0], at[a][1])) return DEO_OK;
+    }
+    for (int v = 0; v < 2 && field; ++v) {
+        bool own = true;  // the field's value at the point itself
+        auto row = [&](long i) {
+            const RowSpec r = table_row(field->tab[v], i + 1);
+            own = own && r.cidx == (int)i + 1;
+            FoldedRow R{};
+            R.fold(r, field->bc, i, (long)sizes[0]);
+            return R;
+        };
+        if (!pack_rows((long)sizes[0], row, 4, 4, hx, blob, at[2 + v][0], at[2 + v][1]) || !own) return DEO_OK;
+    }
     const void* d = nullptr;
     const deo_status s = upload(P, blob, &d);
     if (s != DEO_OK) return s;
@@ -1373,13 +1409,13 @@ static deo_status build_rows2(deo_plan& P, const int64_t* sizes, int nterms, con
         return deo::BfpRows{base + at[k][0], base + at[k][1]};
     };
     for (int a = 0; a < 2; ++a)
-        if (!ax[a].empty()) B.ax[a] = rows(a);
-    for (int v = 0; v < 2 && B.field; ++v) B.f[v] = rows(2 + v);
+        if (!plain[a].empty()) B.ax[a] = rows(a);
+    for (int v = 0; v < 2 && field; ++v) B.f[v] = rows(2 + v);
+    if (field) B.field = field->field;
     B.ok = 1;
     P.rows2 = B;
     return DEO_OK;
 }
-
 extern "C" deo_status deo_plan_create(int ndims, const int64_t* sizes, deo_dtype dtype, int nterms,
                                       const deo_term* terms, deo_plan** out) {
     return deo_plan_create_opts(ndims, sizes, dtype, nterms, terms, 0, out);
@@ -1439,6 +1475,8 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
         for (int t = 0; t < nterms; ++t) eff[t] = lead[t] < 0 ? ne++ : eff[lead[t]];
         D.nterms = ne;
     }
+    const bool rows2 = ndims == 2 && dtype == DEO_F64 && flags == 0 && rows2_terms(sizes, nterms, terms);
+    std::vector<Rows2Term> rows2_from;
     for (int t = 0; t < nterms; ++t) {
         const deo_term& tm = terms[t];
         if (tm.path < DEO_PATH_AUTO || tm.path > DEO_PATH_GENERIC)
@@ -1530,6 +1568,7 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
         std::vector<const deo_operator*> members{&A};
         for (int m = t + 1; m < nterms; ++m)
             if (lead[m] == t) members.push_back(terms[m].op);
+        if (rows2) rows2_from.push_back(Rows2Term{T.axis, A.wind, A.stl, static_cast<const double*>(tm.coeff_field), *tm.bc, {}});
         RowRange R;
         T.sf_lo = 1;
         T.sf_hi = A.len;
@@ -1557,6 +1596,7 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             T.s_cidx = Q.cidx;
             R = Q;
             if ((s = upload_tab(*P, H, dtype, T.tab[v])) != DEO_OK) return s;
+            if (rows2) rows2_from.back().tab[v] = std::move(H);
         }
         for (int p = 0; p < A.len + 2; ++p)
             if (rhi[p] < rlo[p]) { rlo[p] = 1; rhi[p] = 0; }
@@ -1730,9 +1770,12 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
             U.enabled = 0;
         }
     }
-    if (ndims == 2 && dtype == DEO_F64 && flags == 0 && (!P->uni.lap || total >= kRowsFxMinPoints)) {
-        const deo_status rs = build_rows2(*P, sizes, nterms, terms);
+    // its rows now, or, in a plan below the kernel's size, when DEO_OPT_EXACT_SUMS asks for it
+    if (rows2 && total >= rows_fx_min(nterms, terms)) {
+        const deo_status rs = build_rows2(*P, sizes, rows2_from);
         if (rs != DEO_OK) return rs;
+    } else if (rows2 && !P->uni.lap) {
+        P->later_rows = std::move(rows2_from);
     }
     CUDA_TRY(cudaMalloc(&P->d_plan, sizeof(PlanDev)), "cudaMalloc(plan)");
     CUDA_TRY(cudaMemcpy(P->d_plan, &P->dev, sizeof(PlanDev), cudaMemcpyHostToDevice), "cudaMemcpy(plan)");
@@ -1983,6 +2026,11 @@ extern "C" deo_status deo_plan_set_option(deo_plan* p, int option, int value) {
         case DEO_OPT_TMA: p->use_tma = value ? 1 : 0; return DEO_OK;
         case DEO_OPT_EXACT_SUMS:
             if (value < 0 || value > 5) return fail(DEO_ERR_BAD_ARG, "exact-sums variant %d not in 0..5", value);
+            if (value == 1 && !p->later_rows.empty()) {
+                const deo_status s = build_rows2(*p, p->dev.sizes, p->later_rows);
+                if (s != DEO_OK) return s;
+                p->later_rows.clear();
+            }
             p->exact_sums = value;
             p->sums_set = 1;
             return DEO_OK;
