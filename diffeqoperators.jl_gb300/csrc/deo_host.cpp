@@ -877,16 +877,20 @@ static cudaError_t alloc_zeroed(unsigned int** d, size_t n) {
 // of two pairs.  A launch takes the next block; every lap of the blocks takes the other
 // pair, which the pair's launch before it has zeroed.  A launch that is being captured
 // takes a block that no direct launch ever uses, zeroed by a memset of its own: a graph
-// may be replayed beside any number of later launches.
+// may be replayed beside any number of later launches.  n direct launches may be in flight
+// at once.
 struct ClaimSlots {
-    static constexpr unsigned int kBlocks = kSchedSlots / 4;  // of direct launches, and as many of captured ones
     unsigned int* d = nullptr;
+    unsigned int n = 0;  // blocks of direct launches, and as many of captured ones
     std::atomic<unsigned int> direct{0}, captured{0};
     ~ClaimSlots() {
         if (d) cudaFree(d);
     }
-    cudaError_t init() { return alloc_zeroed(&d, 2 * 4 * kBlocks); }
-    unsigned int* graph_block() { return d + 4 * (kBlocks + captured.fetch_add(1) % kBlocks); }
+    cudaError_t init(unsigned int launches) {
+        n = launches;
+        return alloc_zeroed(&d, 2 * 4 * n);
+    }
+    unsigned int* graph_block() { return d + 4 * (n + captured.fetch_add(1) % n); }
     static bool capturing(cudaStream_t st) {
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();  // (the launch reports what is wrong)
@@ -898,7 +902,7 @@ struct ClaimSlots {
             return cudaMemsetAsync(*pair, 0, 2 * sizeof(unsigned int), st);
         }
         const unsigned int k = direct.fetch_add(1);
-        *pair = d + 4 * (k % kBlocks) + 2 * (k / kBlocks % 2);
+        *pair = d + 4 * (k % n) + 2 * (k / n % 2);
         return cudaSuccess;
     }
 };
@@ -1780,7 +1784,7 @@ extern "C" deo_status deo_plan_create_opts(int ndims, const int64_t* sizes, deo_
     CUDA_TRY(cudaMalloc(&P->d_plan, sizeof(PlanDev)), "cudaMalloc(plan)");
     CUDA_TRY(cudaMemcpy(P->d_plan, &P->dev, sizeof(PlanDev), cudaMemcpyHostToDevice), "cudaMemcpy(plan)");
     if (P->march.ok) {
-        CUDA_TRY(P->claims.init(), "cudaMalloc(claim counters)");
+        CUDA_TRY(P->claims.init(kSchedSlots), "cudaMalloc(claim counters)");
         const int planes = P->march.hi[2] - P->march.lo[2] + 1;
         CUDA_TRY((cudaError_t)deo_k_march_chunk(&P->uni, &P->march, planes, &P->march.zc), "marching kernel");
     }
@@ -2488,7 +2492,7 @@ extern "C" deo_status deo_vector_calculus_plan(int kind, int ndims, const deo_op
             V->bfp.kbase[a] = 57 - s - 1075 - 6;
         }
         if (V->bfp.ok) {
-            CUDA_TRY(V->claims.init(), "cudaMalloc(claim counters)");
+            CUDA_TRY(V->claims.init(kSchedSlots), "cudaMalloc(claim counters)");
             CUDA_TRY((cudaError_t)deo_k_vector_chunk(&D, &V->bfp.zc), "marching kernel");
         }
         // k_vc_fx from here on (units of 64 x 8 columns and their queues want a full chip):
@@ -3079,7 +3083,7 @@ extern "C" deo_status deo_batch_create(int n, const deo_instance* in, int adjoin
         CUDA_TRY(cudaMemcpy(b->d_inst, b->inst.data(), n * sizeof(deo::InstDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(instances)");
     }
-    CUDA_TRY(b->claims.init(), "cudaMalloc(claim counters)");
+    CUDA_TRY(b->claims.init(64), "cudaMalloc(claim counters)");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
@@ -3136,7 +3140,7 @@ extern "C" deo_status deo_stage_batch_create(int n, const deo_stage* in, int til
         CUDA_TRY(cudaMemcpy(b->d_stages, b->stages.data(), n * sizeof(deo::StageDev), cudaMemcpyHostToDevice),
                  "cudaMemcpy(stages)");
     }
-    if (!b->one()) CUDA_TRY(b->claims.init(), "cudaMalloc(claim counters)");
+    if (!b->one()) CUDA_TRY(b->claims.init(64), "cudaMalloc(claim counters)");
     b->ctas = ctas > 0 ? ctas : 4;
     deo_status s = batch_items(*b, tile > 0 ? tile : 8192);
     if (s != DEO_OK) return s;
