@@ -1881,6 +1881,11 @@ static bool use_march(const deo_plan* p, bool adjoint = false) {
            (p->sums_set || p->dev.sizes[0] % 2 == 0 ||
             (p->dev.total >= (adjoint ? kMarchMinOddAdjoint : kMarchMinOddPoints) && mostly_inside(p)));
 }
+// 2-D Float64 plans: k_rows_fx.
+static bool use_rows(const deo_plan* p) {
+    return p->rows2.ok && p->exact_sums == 1 && p->fast_path && p->use_tma &&
+           (p->sums_set ? !p->uni.lap : p->dev.total >= (p->rows2.field ? kRowsFxMinFieldPoints : kRowsFxMinPoints));
+}
 // 2-D Float64 Laplacians by default: k_rows_fx, or the generic kernel below its size;
 // of the tiled kernels, which split such a plan into an interior and a shell launch,
 // only that of one shared band stays there.  Unequal steps, order 4, tiled against
@@ -1952,8 +1957,7 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     mark(p, 0, stream);
     if (use_march(p)) return launch_march(p, u, du, overwrite, stream);
-    if (p->rows2.ok && p->exact_sums == 1 && p->fast_path && p->use_tma &&
-        (p->sums_set ? !p->uni.lap : p->dev.total >= (p->rows2.field ? kRowsFxMinFieldPoints : kRowsFxMinPoints))) {
+    if (use_rows(p)) {
         const int e = deo_k_rows_fx(&p->rows2, p->d_plan, u, du, overwrite, stream);
         p->last_kernel = "k_rows_fx";
         p->last_kernel2 = "";
@@ -2070,10 +2074,11 @@ extern "C" deo_status deo_plan_set_option(deo_plan* p, int option, int value) {
 extern "C" int deo_plan_get_option(const deo_plan* p, int option) {
     if (!p) return -1;
     switch (option) {
-        case DEO_OPT_FAST_PATH: return p->fast_path && p->uni.enabled;
-        case DEO_OPT_TMA: return p->use_tma && p->uni.enabled && p->uni.lap;
+        case DEO_OPT_FAST_PATH: return p->fast_path && (p->uni.enabled || use_rows(p));
+        case DEO_OPT_TMA: return p->use_tma && ((p->uni.enabled && p->uni.lap) || use_rows(p));
         case DEO_OPT_EXACT_SUMS:
-            return p->exact_sums && p->uni.enabled && p->uni.lap && (p->uni.ens || p->uni.fx || p->uni.bfx);
+            return use_march(p) || use_rows(p) ||
+                   (p->exact_sums && p->uni.enabled && p->uni.lap && (p->uni.ens || p->uni.fx || p->uni.bfx));
         case DEO_OPT_LAUNCH_TIMING: return p->timing;
         case DEO_OPT_TEST_WITHHOLD: return p->uni.test_withhold;
         case DEO_OPT_SHELL_KERNEL: return p->uni.shell_kernel;
@@ -2088,8 +2093,8 @@ extern "C" int deo_plan_get_option(const deo_plan* p, int option) {
                        ? p->uni.fx_rows
                        : 0;
         case DEO_OPT_CONCURRENT_SHELL:
-            return p->concurrent && p->side && p->d_shell && p->uni.enabled && p->uni.lap &&
-                   (p->dev.dtype == DEO_F32 ||
+            return p->concurrent && p->side && p->d_shell && p->uni.enabled && p->uni.lap && !use_rows(p) &&
+                   (p->dev.dtype == DEO_F32 || use_march(p) ||
                     (((p->exact_sums == 5 && (p->uni.fx || p->uni.bfx)) ||
                       ((p->exact_sums == 1 || p->exact_sums == 4) && p->uni.fx)) &&
                      p->uni.radius <= 3));

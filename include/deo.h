@@ -222,12 +222,14 @@ int deo_plan_terms(const deo_plan* plan);
 int deo_plan_star_taps(const deo_plan* plan);
 /* Plan options (defaults 1 unless stated):
  *   DEO_OPT_FAST_PATH: Laplacian-type 2-D/3-D plans (term t a centred band on
- *     axis t) use the tiled TMA kernels below for interior points; 0 forces
- *     the generic row-table kernel (which every other plan runs).
- *   DEO_OPT_TMA: those plans stream planes with TMA into a shared-memory ring;
- *     0 uses the generic kernel as well.
- *   DEO_OPT_EXACT_SUMS: Float64 Laplacian-type plans whose terms share one
- *     band evaluate interior points in integer arithmetic and round once
+ *     axis t) use the tiled kernels below for interior points, 2-D Float64
+ *     plans the rows kernel; 0 forces the generic row-table kernel (which every
+ *     other plan runs).
+ *   DEO_OPT_TMA: those plans stream planes through a shared-memory ring, with
+ *     TMA in all but the marching kernel, whose shell alone uses it; 0 uses the
+ *     generic kernel as well.
+ *   DEO_OPT_EXACT_SUMS: Float64 Laplacian-type plans, and 2-D Float64 plans of
+ *     any kind, evaluate in integer arithmetic and round once
  *     (result within a few ulp of sum|c_k u_k| of the reference's order):
  *       1 the best variant that applies (default): for three axes with band
  *         radius <= 3 the marching block fixed-point kernel (any alignment and
@@ -237,7 +239,8 @@ int deo_plan_star_taps(const deo_plan* plan);
  *         2-D Float64 plans of any kind take the rows kernel (each axis's
  *         rows as integer windows in block fixed point, one launch) from 2^19
  *         points on, 2^18 with a field term; smaller ones, and 3-D Laplacians
- *         with an odd first size below 300,000 points, the generic kernel,
+ *         with an odd first size below 300,000 points or with less than two
+ *         thirds of the points in uniform rows, the generic kernel,
  *         which is faster there.  Setting the option to 1 asks for its
  *         kernels at every size (2-D Laplacians: the tiled ones);
  *       5 for three axes the block fixed-point kernel (values aligned once
@@ -260,9 +263,9 @@ int deo_plan_star_taps(const deo_plan* plan);
  *     same time as the interior (forked from and joined back into the
  *     caller's stream, so the apply stays stream-ordered; the shell's CTAs
  *     are sized to fit beside the interior kernel's).  It applies to Float32
- *     plans and to the fixed-point Float64 interior (whose FP64 pipe is free
- *     for the shell); other Float64 interiors are FP64-bound and run the
- *     shell after them.  0 runs the shell after the interior always.
+ *     plans and to the marching and fixed-point Float64 interiors (whose FP64
+ *     pipe is free for the shell); other Float64 interiors are FP64-bound and
+ *     run the shell after them.  0 runs the shell after the interior always.
  *   DEO_OPT_FX_FP64_ROWS: 0..8 (default 2): in the fixed-point Float64
  *     interior kernel, the points with ((y mod 8) - value * (floor(y/8) + z))
  *     mod 8 < value (y, z the 0-based indices along axes 2 and 3, z = 0 in
