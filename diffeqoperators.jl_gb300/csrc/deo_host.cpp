@@ -918,7 +918,7 @@ struct deo_plan {
     int fast_path = 1;   // DEO_OPT_FAST_PATH
     int use_tma = 1;     // DEO_OPT_TMA
     int exact_sums = 1;  // DEO_OPT_EXACT_SUMS
-    int sums_set = 0;    // DEO_OPT_EXACT_SUMS was set: its kernels at every size
+    int sums_set = 0;    // DEO_OPT_EXACT_SUMS was set to 1 on top of 1: its kernels at every size
     int timing = 0;      // DEO_OPT_LAUNCH_TIMING
     int concurrent = 1;  // DEO_OPT_CONCURRENT_SHELL
     // the last deo_plan_autotune: per candidate (f32_vec, vcfg, shell kernel, concurrent) its best ms
@@ -2034,13 +2034,15 @@ extern "C" deo_status deo_plan_set_option(deo_plan* p, int option, int value) {
         case DEO_OPT_TMA: p->use_tma = value ? 1 : 0; return DEO_OK;
         case DEO_OPT_EXACT_SUMS:
             if (value < 0 || value > 5) return fail(DEO_ERR_BAD_ARG, "exact-sums variant %d not in 0..5", value);
-            if (value == 1 && !p->later_rows.empty()) {
+            if (value == 1 && p->exact_sums == 1 && !p->later_rows.empty()) {
                 const deo_status s = build_rows2(*p, p->dev.sizes, p->later_rows);
                 if (s != DEO_OK) return s;
                 p->later_rows.clear();
             }
+            // 1 on top of 1 asks for its kernels at every size; 1 after another variant is the default again
+            p->sums_set = value == 1 && p->exact_sums == 1;
+            if (value == 1 && p->exact_sums != 1) p->fx_rows_set = 0;
             p->exact_sums = value;
-            p->sums_set = 1;
             return DEO_OK;
         case DEO_OPT_CONCURRENT_SHELL: p->concurrent = value ? 1 : 0; return DEO_OK;
         case DEO_OPT_FX_FP64_ROWS:

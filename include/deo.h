@@ -241,8 +241,9 @@ int deo_plan_star_taps(const deo_plan* plan);
  *         points on, 2^18 with a field term; smaller ones, and 3-D Laplacians
  *         with an odd first size below 300,000 points or with less than two
  *         thirds of the points in uniform rows, the generic kernel,
- *         which is faster there.  Setting the option to 1 asks for its
- *         kernels at every size (2-D Laplacians: the tiled ones);
+ *         which is faster there.  Setting the option to 1 while it is 1 asks
+ *         for its kernels at every size (2-D Laplacians: the tiled ones);
+ *         setting it to 1 after another variant is the default again;
  *       5 for three axes the block fixed-point kernel (values aligned once
  *         per plane to one exponent per plane tile, no FP64 instruction per
  *         point; points near a zero of u, where that alignment cannot bound
@@ -273,7 +274,8 @@ int deo_plan_star_taps(const deo_plan* plan);
  *     plane; whole warps) are evaluated in the reference's per-term tap order
  *     on the FP64 pipe, bit-identical to the generic kernel, while the others
  *     use the integer pipes; 0 evaluates every interior point in fixed point.
- *     Setting it keeps a plan on the per-point kernel.  deo_plan_get_option
+ *     Setting it keeps a plan on the per-point kernel, until the exact-sums
+ *     option goes back to 1 from another variant.  deo_plan_get_option
  *     returns the value when that kernel applies, else 0.
  *   DEO_OPT_TEST_WITHHOLD: 0 (default) or k in 1..64, for tests of the
  *     bounded waits only: the TMA kernels (interior and shell) withhold the

@@ -1,8 +1,10 @@
-"""GPU: what a plan's options report is what its applies do."""
+"""GPU: what a plan's options report is what its applies do, and the exact-sums option
+returned from another variant is the default again."""
+import numpy as np
 import pytest
 
 import deo
-from cases import build, to_device
+from cases import build, to_device, to_host
 from test_gpu_parity import T
 
 pytestmark = pytest.mark.gpu
@@ -26,3 +28,17 @@ def test_what_applies_is_reported(cuda, shape, h, sums, concurrent, kernel):
     assert p.get_option(deo.DEO_OPT_EXACT_SUMS) == sums and p.get_option(deo.DEO_OPT_CONCURRENT_SHELL) == concurrent
     p.set_option(deo.DEO_OPT_EXACT_SUMS, 0)
     assert p.get_option(deo.DEO_OPT_EXACT_SUMS) == 0
+    want = to_host(out)
+    p.set_option(deo.DEO_OPT_EXACT_SUMS, 1)
+    p.apply(ud, out)
+    assert p.kernels[0] == kernel and np.array_equal(to_host(out), want)
+
+
+def test_rows_option_given_back(cuda):
+    A, _, u = _lap((64, 40, 32), (0.1, 0.1, 0.1))
+    p, out = deo.Plan(A.terms(), (64, 40, 32), 0), deo.julia_array((64, 40, 32))
+    p.set_option(deo.DEO_OPT_FX_FP64_ROWS, 2)
+    assert p.get_option(deo.DEO_OPT_FX_FP64_ROWS) == 2
+    p.set_option(deo.DEO_OPT_EXACT_SUMS, 0)
+    p.set_option(deo.DEO_OPT_EXACT_SUMS, 1)
+    assert p.get_option(deo.DEO_OPT_FX_FP64_ROWS) == 0
