@@ -3237,9 +3237,9 @@ static std::map<std::string, PlanTune> g_plan_tune;
 static std::string plan_signature(const deo_plan& p) {
     const deo::UniPlan& U = p.uni;
     char buf[256];
-    std::snprintf(buf, sizeof buf, "lap/%s/%lldx%lldx%lld/t%d/H%d/es%d/bc%d%d%d", p.dev.dtype == DEO_F64 ? "f64" : "f32",
+    std::snprintf(buf, sizeof buf, "lap/%s/%lldx%lldx%lld/t%d/H%d/es%d/bc%d%d%d%s", p.dev.dtype == DEO_F64 ? "f64" : "f32",
                   (long long)U.n[0], (long long)U.n[1], (long long)U.n[2], U.nterms, U.radius, p.exact_sums,
-                  p.shell.t[0].bc_kind, p.shell.t[1].bc_kind, p.shell.t[2].bc_kind);
+                  p.shell.t[0].bc_kind, p.shell.t[1].bc_kind, p.shell.t[2].bc_kind, use_march(&p) ? "/march" : "");
     return buf;
 }
 

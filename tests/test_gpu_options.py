@@ -42,3 +42,13 @@ def test_rows_option_given_back(cuda):
     p.set_option(deo.DEO_OPT_EXACT_SUMS, 0)
     p.set_option(deo.DEO_OPT_EXACT_SUMS, 1)
     assert p.get_option(deo.DEO_OPT_FX_FP64_ROWS) == 0
+
+
+def test_tuned_choices_belong_to_the_kernel_they_were_timed_with(cuda, tmp_path):
+    A, _, u = _lap((64, 40, 32), (0.1, 0.1, 0.1))
+    path = tmp_path / "tuned"
+    # a choice stored for the per-point kernel under the key that both kernels once shared
+    path.write_text("lap/f64/64x40x32/t3/H1/es1/bc000 0 0 2 0\n")
+    p, out, ud = deo.Plan(A.terms(), (64, 40, 32), 0), deo.julia_array((64, 40, 32)), to_device(u)
+    p.autotune(ud, out, cache_path=str(path))
+    assert any(line.startswith("lap/f64/64x40x32/t3/H1/es1/bc000/march ") for line in path.read_text().splitlines())
