@@ -2305,6 +2305,7 @@ struct deo_nld {
     deo_plan* plan = nullptr;
     int n = 0, m = 0, len = 0, a = 0;
     deo::NldBfp bfp = {};
+    std::atomic<int64_t> bfp_min{0};  // points from which bfp is used, where it can be
     ~deo_nld() { deo_plan_destroy(plan); }
 };
 
@@ -2389,12 +2390,16 @@ extern "C" deo_status deo_nonlinear_diffusion(const deo_nld* nl, const void* p, 
                                               void* stream) {
     if (!nl || !p || !q || !du) return fail(DEO_ERR_BAD_ARG, "null argument");
     if (du == p || du == q) return fail(DEO_ERR_BAD_ARG, "du must not alias p or q");
-    const int e = nl->bfp.ok
+    const int e = nl->bfp.ok && nl->len >= nl->bfp_min
                       ? deo_k_nld_fx(&nl->bfp, nl->plan->d_plan, nl->len, nl->n, nl->m, nl->a, p, q, du, stream)
                       : deo_k_nonlinear_diffusion(&nl->plan->dev, nl->len, nl->n, nl->m, nl->plan->dev.dtype, p, q, du,
                                                   stream);
     if (e) return cuda_fail((cudaError_t)e, "deo_nonlinear_diffusion launch");
     return DEO_OK;
+}
+
+extern "C" void deo_nonlinear_diffusion_march_min(deo_nld* nl, int64_t points) {
+    if (nl) nl->bfp_min = points;
 }
 
 extern "C" void deo_nonlinear_diffusion_destroy(deo_nld* nl) { delete nl; }
@@ -2407,7 +2412,7 @@ struct deo_vc {
     deo::VcDev dev{};
     deo::VcBfp bfp{};  // 3-D Float64 with a uniform band: block fixed point (ok = 0: not this plan)
     mutable ClaimSlots claims;
-    int64_t march_min = 0;  // points from which bfp is used
+    std::atomic<int64_t> march_min{0};  // points from which bfp is used
     int dtype = 0;
     int ncomp_in = 1, ncomp_out = 1;
 };
@@ -2549,8 +2554,9 @@ extern "C" deo_status deo_vector_calculus_apply(const deo_vc* vc, const void* M,
     return DEO_OK;
 }
 
-// The marching kernel from `points` on (tests of its edges on small arrays).
-extern "C" void deo_vector_calculus_march_min(deo_vc* vc, int64_t points) { vc->march_min = points; }
+extern "C" void deo_vector_calculus_march_min(deo_vc* vc, int64_t points) {
+    if (vc) vc->march_min = points;
+}
 
 extern "C" void deo_vector_calculus_destroy(deo_vc* vc) { delete vc; }
 

@@ -156,6 +156,8 @@ def lib():
     proto("deo_vector_calculus_plan", st, C.c_int, C.c_int, C.POINTER(_vp), C.c_int, C.POINTER(_vp))
     proto("deo_vector_calculus_sizes", st, _vp, C.POINTER(C.c_int64), C.POINTER(C.c_int64))
     proto("deo_vector_calculus_apply", st, _vp, _vp, _vp, C.c_int, _vp)
+    proto("deo_vector_calculus_march_min", None, _vp, C.c_int64)
+    proto("deo_nonlinear_diffusion_march_min", None, _vp, C.c_int64)
     proto("deo_vector_calculus_info", st, _vp, C.POINTER(C.c_int))
     proto("deo_vector_calculus_destroy", None, _vp)
     proto("deo_dot_product", st, C.c_int, C.c_int64, C.c_int, _vp, _vp, _vp, _vp)
@@ -217,6 +219,7 @@ EXPORTED = [
     "deo_serve_create", "deo_serve_submit", "deo_serve_pump", "deo_serve_poll", "deo_serve_cancel", "deo_serve_stats_get",
     "deo_serve_inject_alloc_failures", "deo_serve_destroy",
     "deo_batch_autotune", "deo_plan_autotune", "deo_plan_autotune_times", "deo_vector_calculus_plan", "deo_vector_calculus_sizes", "deo_vector_calculus_apply", "deo_vector_calculus_info",
+    "deo_vector_calculus_march_min", "deo_nonlinear_diffusion_march_min",
     "deo_vector_calculus_destroy", "deo_dot_product", "deo_cross_product", "deo_square_norm",
     "deo_solve_plan", "deo_solve_bands", "deo_solve_apply", "deo_solve_destroy",
     "deo_padded_plan", "deo_padded_plan_view", "deo_padded_apply", "deo_padded_destroy",

@@ -359,12 +359,18 @@ deo_status deo_apply_adjoint(const deo_plan* plan, const void* dbar, void* ubar,
  *      + (D_{m+n} q) .* p[2:nknots+1]
  * with D_k = CenteredDifference(k, approx_order, dx, nknots) applied to the
  * padded vectors p, q (nknots + 2 entries, ghosts first and last) by the
- * generic method, in the reference's operation order.  Planned once
- * (operators and tables), applied on device vectors p, q -> du (nknots). */
+ * generic method, the products and sums in the reference's operation order.
+ * Planned once (operators and tables), applied on device vectors p, q -> du
+ * (nknots).  Float64 on a uniform grid, orders n <= 2, m <= 1, approx_order 2 or
+ * 4, from 2^17 points on: each derivative in block fixed point, rounded once,
+ * within 2 ulp of its sum |w x|.  deo_nonlinear_diffusion_march_min gives the
+ * points from which that is done (INT64_MAX: never, every derivative tap by tap in
+ * the reference's order). */
 typedef struct deo_nld deo_nld;
 deo_status deo_nonlinear_diffusion_plan(int second_order, int first_order, int approx_order, const double* dx,
                                         int dx_len, int nknots, deo_dtype dtype, deo_nld** out);
 deo_status deo_nonlinear_diffusion(const deo_nld* plan, const void* p, const void* q, void* du, void* stream);
+void deo_nonlinear_diffusion_march_min(deo_nld* plan, int64_t points);
 void deo_nonlinear_diffusion_destroy(deo_nld* plan);
 
 /* ------------------------------------------------------------------------
@@ -445,6 +451,11 @@ deo_status deo_vector_calculus_sizes(const deo_vc* plan, int64_t* in_elems, int6
  * unrolled marching kernel), 0 when every row goes through the row tables. */
 deo_status deo_vector_calculus_info(const deo_vc* plan, int* band_nk);
 deo_status deo_vector_calculus_apply(const deo_vc* plan, const void* M, void* out, int overwrite, void* stream);
+/* The output points from which a Float64 plan of three uniform axes evaluates its
+ * derivatives in block fixed point (each rounded once, within 2 ulp of its sum |w x|;
+ * default 1, 4 or 16 million by kind and order).  0: at every size; INT64_MAX: never,
+ * every derivative tap by tap in the reference's order. */
+void deo_vector_calculus_march_min(deo_vc* plan, int64_t points);
 void deo_vector_calculus_destroy(deo_vc* plan);
 
 /* Pointwise vector algebra over npts points of ncomp components stored
