@@ -1898,24 +1898,35 @@ static unsigned int* next_sched(const deo_plan* p) {
     return p->d_sched ? p->d_sched + (p->sched_slot.fetch_add(1) % kSchedSlots) : nullptr;
 }
 
+// Whether a launch on st may use the plan's side stream: not while that is part of a
+// capture that st is not part of (another thread's, until it ends).
+static bool side_free(const deo_plan* p, cudaStream_t st) {
+    cudaStreamCaptureStatus sa = cudaStreamCaptureStatusNone, sb = cudaStreamCaptureStatusNone;
+    unsigned long long ia = 0, ib = 0;
+    if (cudaStreamGetCaptureInfo(p->side, &sb, &ib) != cudaSuccess || sb == cudaStreamCaptureStatusNone) return true;
+    return cudaStreamGetCaptureInfo(st, &sa, &ia) == cudaSuccess && sa == sb && ia == ib;
+}
+
 // Interior and shell write different points: with conc the shell runs on the plan's
 // side stream, launched after the interior and free to fill the SMs as the interior's
-// CTAs leave them, and the caller's stream waits for it.
+// CTAs leave them, and the caller's stream waits for it; else after the interior.
+// shell(stream, beside the interior).
 template <class Interior, class Shell>
 static int interior_then_shell(const deo_plan* p, bool conc, void* stream, Interior interior, Shell shell) {
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     std::unique_lock<std::mutex> lk(p->apply_mu, std::defer_lock);
     if (conc) {
         lk.lock();
-        const cudaError_t c = cudaEventRecord(p->ev_fork, st);
+        conc = side_free(p, st);
+        const cudaError_t c = conc ? cudaEventRecord(p->ev_fork, st) : cudaSuccess;
         if (c != cudaSuccess) return (int)c;
     }
     int e = interior();
     if (e) return e;
-    if (!conc) return shell(stream);
+    if (!conc) return shell(stream, false);
     cudaError_t c = cudaStreamWaitEvent(p->side, p->ev_fork, 0);
     if (c != cudaSuccess) return (int)c;
-    e = shell(static_cast<void*>(p->side));
+    e = shell(static_cast<void*>(p->side), true);
     if (e) return e;
     c = cudaEventRecord(p->ev_join, p->side);
     if (c == cudaSuccess) c = cudaStreamWaitEvent(st, p->ev_join, 0);
@@ -1941,7 +1952,7 @@ static int launch_march(const deo_plan* p, const void* u, void* du, int overwrit
             mark(p, 1, stream);
             return ei;
         },
-        [&](void* s2) {
+        [&](void* s2, bool) {
             return deo_k_apply_shell(&us, sp, p->d_shell, DEO_SHELL_ALONE, p->d_plan, p->dev.dtype, u, du, overwrite,
                                      s2, &k2);
         });
@@ -1954,7 +1965,6 @@ static int launch_march(const deo_plan* p, const void* u, void* du, int overwrit
 }
 
 static int launch_forward(const deo_plan* p, const void* u, void* du, int overwrite, void* stream) {
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     mark(p, 0, stream);
     if (use_march(p)) return launch_march(p, u, du, overwrite, stream);
     if (use_rows(p)) {
@@ -1979,37 +1989,25 @@ static int launch_forward(const deo_plan* p, const void* u, void* du, int overwr
             const char* k2 = "";
             // a counter of its own for this launch (applies of one plan may run on several streams at once)
             unsigned int* sched = next_sched(p);
-            if (conc) {
-                // the interior first, on the caller's stream: its persistent grid takes its CTAs' places
-                // on every SM at once; then the shell on the side stream, whose CTAs fill the place left
-                // beside them (both kernels ask for the largest shared-memory carveout so that this
-                // place exists: with the interior's SMs configured for its CTAs alone the shell ran
-                // after it, 420 against 303 us at 256^3); the caller's stream waits for the shell
-                std::lock_guard<std::mutex> lk(p->apply_mu);
-                cudaError_t c = cudaEventRecord(p->ev_fork, st);
-                if (c != cudaSuccess) return (int)c;
-                const int e = deo_k_apply_tma(up, p->d_plan, p->dev.dtype, u, du, overwrite, p->exact_sums,
-                                              stream, &k, sched);
-                if (e) return e;  // (cudaErrorNotSupported cannot occur: the tensor-map rules were checked)
-                mark(p, 1, stream);
-                c = cudaStreamWaitEvent(p->side, p->ev_fork, 0);
-                if (c != cudaSuccess) return (int)c;
-                int e2 = deo_k_apply_shell(up, &p->shell, p->d_shell, DEO_SHELL_CONCURRENT, p->d_plan,
-                                           p->dev.dtype, u, du, overwrite, p->side, &k2);
-                if (e2) return e2;
-                c = cudaEventRecord(p->ev_join, p->side);
-                if (c == cudaSuccess) c = cudaStreamWaitEvent(st, p->ev_join, 0);
-                if (c != cudaSuccess) return (int)c;
-            } else {
-                const int e = deo_k_apply_tma(up, p->d_plan, p->dev.dtype, u, du, overwrite, p->exact_sums,
-                                              stream, &k, sched);
-                if (e) return e;
-                mark(p, 1, stream);
-                const int e2 = deo_k_apply_shell(up, p->d_shell ? &p->shell : nullptr, p->d_shell,
-                                                 DEO_SHELL_ALONE, p->d_plan, p->dev.dtype, u, du, overwrite,
-                                                 stream, &k2);
-                if (e2) return e2;
-            }
+            // the interior first, on the caller's stream: its persistent grid takes its CTAs' places
+            // on every SM at once; then the shell on the side stream, whose CTAs fill the place left
+            // beside them (both kernels ask for the largest shared-memory carveout so that this
+            // place exists: with the interior's SMs configured for its CTAs alone the shell ran
+            // after it, 420 against 303 us at 256^3); the caller's stream waits for the shell
+            const int e = interior_then_shell(
+                p, conc, stream,
+                [&] {  // (cudaErrorNotSupported cannot occur: the tensor-map rules were checked)
+                    const int ei = deo_k_apply_tma(up, p->d_plan, p->dev.dtype, u, du, overwrite, p->exact_sums, stream,
+                                                   &k, sched);
+                    if (!ei) mark(p, 1, stream);
+                    return ei;
+                },
+                [&](void* s2, bool beside) {
+                    return deo_k_apply_shell(up, p->d_shell ? &p->shell : nullptr, p->d_shell,
+                                             beside ? DEO_SHELL_CONCURRENT : DEO_SHELL_ALONE, p->d_plan, p->dev.dtype,
+                                             u, du, overwrite, s2, &k2);
+                });
+            if (e) return e;
             p->last_kernel = k;
             p->last_kernel2 = k2;
             p->ev_launches = 2;
@@ -2178,7 +2176,7 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
                 const int ei = (int)p->claims.next(static_cast<cudaStream_t>(stream), &pair);
                 return ei ? ei : deo_k_apply_march(&ua, &B, pair, d, ub, overwrite, stream);
             },
-            [&](void* s2) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
+            [&](void* s2, bool) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
         if (e) return e;
         p->last_kernel = "k_lap_fx";
         p->last_kernel2 = "k_shell_adj";
@@ -2206,7 +2204,7 @@ static int launch_adjoint(const deo_plan* p, const void* d, void* ub, int overwr
             [&] {
                 return deo_k_apply_tma(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, p->exact_sums, stream, &k, sched);
             },
-            [&](void* s2) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
+            [&](void* s2, bool) { return deo_k_apply_shell_adj(&ua, p->d_plan, p->dev.dtype, d, ub, overwrite, 0, s2); });
         if (e) return e;
         p->last_kernel = k;
         p->last_kernel2 = "k_shell_adj";
