@@ -1208,9 +1208,10 @@ static bool bfp_band(const double* w, int K, int& s, double& total, int* wh, int
 // are accepted by their neighbours alone.
 static deo::BfpMarch::Limit march_limit(double total, double c0, double w1) {
     const int t0 = bfp_threshold(total, c0, 1.0), t1 = bfp_threshold(total, w1, 2.0);
-    deo::BfpMarch::Limit L{std::min(t0, t1), 0, 0};
+    deo::BfpMarch::Limit L{std::min(t0, t1), 0, 0, 0};
     while (L.sh0 < 31 && ((long long)L.t << L.sh0) < t0) ++L.sh0;
     while (L.sh1 < 31 && ((long long)L.t << L.sh1) < t1) ++L.sh1;
+    L.gap = std::max(28 - std::ilogb((double)L.t), 0);
     return L;
 }
 static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
@@ -1231,6 +1232,11 @@ static bool march_weights(const double* const w[3], int H, deo::BfpMarch& B) {
         }
     split_limbs(c0, B.c0h, B.c0l);
     B.shared = std::memcmp(w[0], w[1], K * sizeof(double)) == 0 && std::memcmp(w[0], w[2], K * sizeof(double)) == 0;
+    double least = std::fabs((double)c0);
+    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < K; ++k)
+            if (k != H) least = std::min(least, std::fabs(std::ldexp(w[a][k], s)));
+    B.own_any = std::ldexp(least, B.shared ? 8 : deo::BFP_OWN[H] + 1) >= 1.05 * total;
     B.limit = march_limit(total, (double)c0, std::ldexp(w[0][H + 1], s));
     B.rev = march_limit(total, (double)c0, std::ldexp(w[0][H - 1], s));
     B.kbase = 57 - s - 1075 - 6;

@@ -179,6 +179,9 @@ struct UniPlan {
 // (deo_bfp.cuh, deo_march.cu): W = round(w * 2^s) = wh * 2^30 + wl, |wl| <= 2^29,
 // with the sum of |W| over all taps below 2^60.  [k] is the offset k - H; c0 the
 // centre weights of the three axes added.
+// Bits below a value's mantissa at the exponent of its own point: 7, or 6 where the cross
+// column's sum over 19 taps could leave int64.
+constexpr int BFP_OWN[4] = {0, 7, 7, 6};  // by radius
 struct BfpMarch {
     int ok;
     int shared;           // the three axes share one band: neighbours are added before the product
@@ -188,9 +191,11 @@ struct BfpMarch {
     // A point is accepted when its centre's high limb, or that of its neighbours at +1,
     // shifted right by sh0 / sh1, reaches t.  rev: the limits of the reversed band (the
     // transpose), whose neighbours at +1 have the weight of those at -1.
+    // A value more than gap binades below the block's cannot reach t.
     struct Limit {
-        int t, sh0, sh1;
+        int t, sh0, sh1, gap;
     } limit, rev;
+    int own_any;          // points on exponents of their own are all within the bound
     int zc, zc_rev;       // planes of a unit; of the transpose's box
     int kbase;            // the sum in units of 2^57 times 2^(kbase + E) is the result
 };

@@ -20,6 +20,23 @@
 // plane's barrier: 8 us more at 256^3).  A plane with Inf/NaN, or with an exponent
 // outside the range the scaled result needs, sends all its points there.
 //
+// Where many values are small against their block's largest (a pulse or a front of a few
+// cells' width: a point below 1.7 % of the block fails its bound), every point would be
+// summed twice.  Each thread compares one value of the tile's middle rows with the block's
+// exponent (counted by the plane's barrier); when the count, decaying by a quarter a plane,
+// passes 5/4 of the threads -- two planes of small values, or a third of the values for
+// good -- the rest of the unit keeps the values themselves in the ring and evaluates each
+// point on the largest exponent of its own taps, a warp's four groups of 32 points in turn
+// three so and one in FP64, so that both pipes work; points that fail there too (far taps of
+// a small weight alone) are evaluated in FP64 at once.  256^3, a Gaussian of width 0.1 / 0.05
+// / 0.02 of the box, us: the per-point kernels before this one / as it was without this / now:
+// order 2 206 / 206 / 208 -> 291 / 518 / 512 -> 200 / 211 / 233; order 4 281 / 280 / 292 ->
+// 508 / 842 / 770 -> 264 / 293 / 333; order 6 610 / 610 / 676 -> 828 / 1236 / 1050 -> 448 /
+// 476 / 831; three bands (256 x 240 x 200), order 4, 506 / 506 / 507 -> 461 / 708 / 622 -> 268 /
+// 293 / 506.  The counting costs 1-2 % of a smooth field's time.  Evaluating the small units
+// inside the plane loop cost every field 40 % (registers); all groups on own exponents 305 at
+// width 0.05, order 4, half of them in FP64 361; limbs per tap, not per sum, 334.
+//
 // What bounds it (256^3, d2 a4, smooth field; start: the per-point fixed point,
 // 270 us beside its shell): 164 us for the interior, 139 us of them without the 2.8 %
 // of points in the reference's order.  139 instructions per point -- 20 32 x 32 ->
@@ -148,6 +165,8 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
 #pragma unroll
             for (int j = 0; j < C::NLD; ++j) raw[j] = __ldg(reinterpret_cast<const double*>(s + off[j]));
         };
+        unsigned probe = 0x7fffffffu;  // the key of this thread's value in the tile's middle rows, a plane ago
+        bool small = false;            // that is too small for the block's exponent
         // the loaded plane on exponent E into a slot; its largest key
         auto put = [&](Limbs* w, int E) {
             unsigned mx = 0;
@@ -155,6 +174,10 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
             for (int j = 0; j < C::NLD; ++j) {
                 const unsigned key = bfp_key(raw[j]);
                 mx = max(mx, key);
+                if (j == C::NLD / 2) {
+                    small = probe < (unsigned)(max(E - B.limit.gap, 1) << 20);
+                    probe = key;
+                }
                 if (j + 1 < C::NLD || tid + j * C::NTHR < C::PLANE) w[tid + j * C::NTHR] = bfp_convert(raw[j], key, E);
             }
             return mx;
@@ -165,19 +188,23 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
         int E = 64;
         int low = 0;           // planes since one last reached E
         int zeros = 0;         // planes since one last held anything but zeros
+        int crowd = 0;         // small values of the last planes
         int sl = 0;            // ring slot of plane p
-        for (int p = 0; p < npl; ++p) {
+        int p = 0;
+        for (; p < npl; ++p) {
             {
                 const unsigned mx = __reduce_max_sync(0xffffffffu, put(ring + sl * C::SLOT, E));
                 if (p + 1 < npl) load(p + 1);
                 if (tx == 0) atomicMax(&s_max[p & 15], mx);
                 if (tid == 0) s_max[(p + 2) & 15] = 0;
             }
-            __syncthreads();
+            const int nsmall = __syncthreads_count(small);
             const unsigned top = s_max[p & 15];
             const int ep = (int)(top >> 20);
             zeros = top == 0 ? zeros + 1 : 0;
             low = ep < E ? low + 1 : 0;
+            crowd = top == 0 ? 0 : nsmall + crowd - crowd / 4;
+            if (crowd > C::NTHR * 5 / 4) break;
             if (ep > E || low > NQ + 2) {
                 // a new exponent: the planes in use (this one included) again
                 int ew = 64;
@@ -281,6 +308,121 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                 }
                 __syncwarp();
                 if (nq > C::QCAP - 64 * RY) drain(31, x0, y0, z0);
+            }
+        }
+        int f64 = 0;  // groups of 32 points that this warp evaluates in FP64 alone
+        auto own_plane = [&](int p) {
+            constexpr int G = BFP_OWN[H];
+            const Limbs* pl[NQ];  // the tile's origin in the planes z - H .. z + H
+#pragma unroll
+            for (int m = 0; m < NQ; ++m) pl[m] = ring + (p - 2 * H + m) % S * C::SLOT + H * C::BX + C::HP;
+            double* dz = du + (int64_t)(z0 + p - 2 * H) * sxy;
+#pragma unroll 1
+            for (int i = 0; i < 2 * RY; ++i) {  // rows ty * RY + i / 2, lanes side by side in either half of the tile
+                const int cx = tx + 32 * (i & 1), cy = ty * RY + i / 2, at = cy * C::BX + cx;
+                auto word = [&](int a, int k) { return a == 0 ? pl[H][at + k - H] : (a == 1 ? pl[H][at + (k - H) * C::BX] : pl[k][at]); };
+                auto value = [&](int a, int k) {
+                    const Limbs b = word(a, k);
+                    return __hiloint2double(b.h, b.l);
+                };
+                // (19 taps are read once more for the sum; kept in registers they spill)
+                unsigned mx = 0;
+                auto taps = [&](auto f) {
+#pragma unroll
+                    for (int a = 0; a < 3; ++a)
+#pragma unroll
+                        for (int k = 0; k < NQ; ++k)
+                            if (a == 0 || k != H) f(word(a, k));
+                };
+                taps([&](Limbs b) { mx = max(mx, (unsigned)b.h & 0x7fffffffu); });
+                if constexpr (H == 3) asm volatile("" ::: "memory");
+                double r = 0.0;
+                bool ok = false;
+                if (__any_sync(0xffffffffu, mx == 0)) {  // zeros alone?
+                    unsigned lo = 0;
+                    taps([&](Limbs b) { lo |= (unsigned)b.l; });
+                    ok = (mx | lo) == 0;
+                }
+                if (f64 == 0 && i != ty) {
+                    const int e = (int)(mx >> 20), E = max(e, 64), kexp = B.kbase - 1 + E;
+                    long long sum;
+                    int cen = 0, near = 0;  // the centre and the neighbours at +1, in 2^30 units of limit's scale
+                    if constexpr (SH) {
+                        BfpOwn s{0, 0, 0, 0};
+                        const long long c = bfp_shift(word(0, H), E);
+                        bfp_mad(s, B.c0h, B.c0l, c);
+                        cen = (int)(c >> 30);
+#pragma unroll
+                        for (int k = 0; k < NQ; ++k) {
+                            if (k == H) continue;
+                            const long long n = bfp_shift(word(0, k), E) + bfp_shift(word(1, k), E) + bfp_shift(word(2, k), E);
+                            bfp_mad(s, B.wh[0][k], B.wl[0][k], n);
+                            if (k == H + 1) near = (int)(n >> 32);
+                        }
+                        sum = bfp_total(s);
+                    } else {
+                        const Limbs c = bfp_nearest<G>(value(0, H), E);
+                        BfpAcc s{0, 0, 0};
+                        bfp_mad(s, B.c0h, B.c0l, c.h, c.l);
+                        cen = c.h;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+#pragma unroll
+                            for (int k = 0; k < NQ; ++k) {
+                                if (k == H) continue;
+                                const Limbs x = bfp_nearest<G>(value(a, k), E);
+                                bfp_mad(s, B.wh[a][k], B.wl[a][k], x.h, x.l);
+                                if (a == 0 && k == H + 1) near = x.h;
+                            }
+                        sum = bfp_total_own<G>(s);
+                    }
+                    r = ok ? 0.0 : bfp_double(sum, kexp * (1 << 20));
+                    ok = ok || (e >= 64 && e < 2047 && bfp_range_ok(kexp) &&
+                                (B.own_any || max(abs(cen) >> B.limit.sh0, abs(near) >> B.limit.sh1) >= B.limit.t ||
+                                 abs((int)(sum >> 32)) >= (SH ? BFP_OWN_LIMIT : bfp_own_limit(G))));
+                    if (__popc(__ballot_sync(0xffffffffu, !ok)) > 8) f64 = 32;
+                } else {
+                    f64 = max(f64 - 1, 0);
+                }
+                if (__any_sync(0xffffffffu, !ok)) {  // the reference's order
+                    double v = 0.0;
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        double acc = 0.0;
+#pragma unroll
+                        for (int k = 0; k < NQ; ++k) acc = fma(U.t[a].w[k], value(a, k), acc);
+                        v = a == 0 ? acc : v + acc;
+                    }
+                    if (!ok) r = zero_fix(v);
+                }
+                const int x = x0 + cx, y = y0 + cy;
+                if (x >= B.lo[0] && x <= B.hi[0] && y >= B.lo[1] && y <= B.hi[1]) {
+                    double* d = dz + (int64_t)y * nx + x;
+                    *d = OW ? r : r + *d;
+                }
+            }
+        };
+        // The rest of a unit whose values are small against their block's, from plane p on: the
+        // ring holds the values themselves, and every point is evaluated on its own exponent.
+        if (p < npl) {
+            auto keep = [&](int q) {
+                Limbs* w = ring + q % S * C::SLOT;
+#pragma unroll
+                for (int j = 0; j < C::NLD; ++j)
+                    if (j + 1 < C::NLD || tid + j * C::NTHR < C::PLANE)
+                        w[tid + j * C::NTHR] = Limbs{__double2hiint(raw[j]), __double2loint(raw[j])};
+            };
+            for (int b = min(2 * H, p); b > 0; --b) {
+                load(p - b);
+                keep(p - b);
+            }
+            load(p);
+            for (; p < npl; ++p) {
+                keep(p);
+                if (p + 1 < npl) load(p + 1);
+                __syncthreads();
+                if (p < 2 * H) continue;
+                own_plane(p);
             }
         }
         // the queues, shared out over the CTA
