@@ -312,6 +312,7 @@ struct VcBfp {
     int ok;
     int wh[3][5], wl[3][5], wd[3][5];
     int t0;  // a derivative is accepted when the larger of its two nearest taps' high limbs reaches this
+    int gap;  // a value more than this many binades below the block's cannot
     int kbase[3];
     int zc;  // planes of a unit
 };

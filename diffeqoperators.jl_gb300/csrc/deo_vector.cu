@@ -251,6 +251,16 @@ __global__ void __launch_bounds__(256) k_vc_march(const VcDev V, const T* __rest
 // the threshold) are queued and evaluated by
 // vc_point at the end of the unit; points on boundary rows are units of their own.
 //
+// A unit whose values are small against their block's goes on with the values themselves, each
+// derivative on the largest exponent of its own taps and a quarter of the points in FP64 (see
+// deo_march.cu): a Gaussian of width 0.1 / 0.05 of the box, us: k_vc / as it was without
+// this / now: gradient 256^3, order 2 380 / 380 -> 411 / 619 -> 272 / 284, order 4 548 / 548 ->
+// 531 / 853 -> 372 / 409, order 6 724 / 722 -> 922 / 1261 -> 580 / 607; 192^3, divergence
+// order 4 242 / 243 -> 437 / 612 -> 263 / 276, order 6 316 / 316 -> 560 / 778 -> 338 / 356; curl
+// order 2 322 / 323 -> 459 / 595 -> 281 / 279, order 4 466 / 466 -> 795 / 1114 -> 496 / 521 (a
+// smooth field there 242 -> 191, 316 -> 254, 322 -> 207, 466 -> 353).  FP64 alone for these units:
+// gradient, order 4, width 0.05, 597.
+//
 // What bounds it: instruction issue, 253 a gradient point (39 multiply-adds, 45 to
 // load and convert 2.1 values, 39 to round and test three derivatives, the rest
 // addressing and control) at 48 %.  256^3, 4th order, against the per-point
@@ -378,6 +388,8 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
             const int i = C::has(c, 2) ? (r6 - back < 0 ? r6 - back + NK + 1 : r6 - back) : ((p - back) & 1);
             return ring + C::base(c) + i * C::plane(c);
         };
+        unsigned probe[NC];  // keys of a value in the tile's middle rows, a plane ago
+        bool small = false;  // one of them is too small for its block's exponent
         auto put = [&](auto cc, int p, int back, int E) {
             constexpr int c = decltype(cc)::value;
             Limbs* w = slot(cc, p, back);
@@ -386,6 +398,10 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
             for (int j = 0; j < C::nld(c); ++j) {
                 const unsigned key = bfp_key(raw[c][j]);
                 mx = max(mx, key);
+                if (j == C::nld(c) / 2) {
+                    small |= E > 64 && probe[c] < (unsigned)(max(E - B.gap, 1) << 20);  // (64: zeros)
+                    probe[c] = key;
+                }
                 if (j + 1 < C::nld(c) || tid + j * C::NTHR < C::plane(c))
                     w[tid + j * C::NTHR] = bfp_convert(raw[c][j], key, E);
             }
@@ -415,8 +431,11 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
         __syncthreads();
         int E[NC], low[NC], zeros[NC];
 #pragma unroll
-        for (int c = 0; c < NC; ++c) E[c] = 64, low[c] = 0, zeros[c] = 0;
-        for (int p = 0; p < npl; ++p, r6 = r6 == NK ? 0 : r6 + 1) {
+        for (int c = 0; c < NC; ++c) E[c] = 64, low[c] = 0, zeros[c] = 0, probe[c] = 0x7fffffffu;
+        int crowd = 0;  // threads with a small value, over the last planes
+        int p = 0;
+        for (; p < npl; ++p, r6 = r6 == NK ? 0 : r6 + 1) {
+            small = false;
             each([&](auto cc) {
                 constexpr int c = decltype(cc)::value;
                 if (C::has(c, 2) || p >= 2 * MID) {
@@ -426,7 +445,8 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
                 if (p + 1 < npl && (C::has(c, 2) || p + 1 >= 2 * MID)) load(cc, p + 1);
                 if (tid == 0) s_max[c][(p + 2) & 15] = 0;
             });
-            __syncthreads();
+            crowd += __syncthreads_count(small) - crowd / 4;
+            if (crowd > C::NTHR * 5 / 4) break;
             each([&](auto cc) {  // a new exponent: the planes in use again (as in deo_march.cu)
                 constexpr int c = decltype(cc)::value, W = C::has(c, 2) ? NK : 1;
                 if (!C::has(c, 2) && p < 2 * MID) return;
@@ -573,6 +593,126 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
                 }
                 __syncwarp();
                 if (nq > C::QCAP - 64 * RY) drain(31, x0, y0, z0);
+            }
+        }
+        // The rest of a unit whose values are small against their block's (as in deo_march.cu), from plane
+        // p on: the ring holds the values themselves, every derivative in the reference's order.
+        if (p < npl) {
+            auto keep = [&](auto cc, int back) {
+                constexpr int c = decltype(cc)::value;
+                Limbs* w = slot(cc, p, back);
+#pragma unroll
+                for (int j = 0; j < C::nld(c); ++j)
+                    if (j + 1 < C::nld(c) || tid + j * C::NTHR < C::plane(c))
+                        w[tid + j * C::NTHR] = Limbs{__double2hiint(raw[c][j]), __double2loint(raw[c][j])};
+            };
+            int f64 = 0;  // groups of 32 points that this warp evaluates in FP64 alone
+            auto own_plane = [&] {
+#pragma unroll 1
+                for (int i = 0; i < 2 * RY; ++i) {  // lanes side by side in either half of the tile
+                    const int cx = tx + 32 * (i & 1), cy = ty * RY + i / 2, x = x0 + cx, y = y0 + cy;
+                    const bool on = x >= bpc && x < n0 - bpc && y >= bpc && y < n1 - bpc;
+                    double* o = out + (int64_t)(z0 + p - 2 * MID) * osz + (int64_t)y * n0 + x;
+                    auto word = [&](auto cc, auto aa, int k) {  // tap k of component c along axis a
+                        constexpr int c = decltype(cc)::value, a = decltype(aa)::value, BX = C::bx(c);
+                        const int at = (cy + (C::has(c, 1) ? C::LH : 0)) * BX + (C::has(c, 0) ? C::PL : 0) + cx;
+                        if (a == 2) return slot(cc, p, 2 * MID - k)[at];
+                        return slot(cc, p, C::has(c, 2) ? MID + 1 : 0)[at + (1 - MID + k) * (a == 0 ? 1 : BX)];
+                    };
+                    // a derivative in the reference's order
+                    auto ref = [&](auto cc, auto aa) {
+                        double acc = 0.0;
+#pragma unroll
+                        for (int k = 0; k < NK; ++k) {
+                            const Limbs v = word(cc, aa, k);
+                            acc = fma(band_w<double>(V.t[decltype(aa)::value].tab[0], k), __hiloint2double(v.h, v.l), acc);
+                        }
+                        return acc;
+                    };
+                    // and on the exponent of its own taps
+                    const bool own_exp = f64 == 0 && i != ty;
+                    bool ok = own_exp;
+                    auto own = [&](auto cc, auto aa) {
+                        constexpr int a = decltype(aa)::value;
+                        Limbs t[NK];
+                        unsigned mx = 0, lo = 0;
+#pragma unroll
+                        for (int k = 0; k < NK; ++k) {
+                            t[k] = word(cc, aa, k);
+                            mx = max(mx, (unsigned)t[k].h & 0x7fffffffu);
+                            lo |= (unsigned)t[k].l;
+                        }
+                        const int e = (int)(mx >> 20), E = max(e, 64), kexp = B.kbase[a] - 1 + E;
+                        BfpOwn s{0, 0, 0, 0};
+                        s.lh = B.wd[a][0] * (bfp_shift(t[MID], E) >> 32);
+                        int near = 0;
+#pragma unroll
+                        for (int d = 1; d <= MID; ++d) {
+                            const long long r = bfp_shift(t[MID + d], E), l = bfp_shift(t[MID - d], E);
+                            bfp_mad(s, B.wh[a][d], B.wl[a][d], r - l);
+                            if (NK >= 7) s.lh += B.wd[a][d] * (l >> 32);
+                            if (d == 1) near = max(abs((int)(r >> 30)), abs((int)(l >> 30)));
+                        }
+                        const long long sum = bfp_total(s);
+                        const bool zero = (mx | lo) == 0;
+                        ok = ok && (zero || (e >= 64 && e < 2047 && bfp_range_ok(kexp) &&
+                                             (near >= B.t0 || abs((int)(sum >> 32)) >= BFP_OWN_LIMIT)));
+                        return zero ? 0.0 : bfp_double(sum, kexp * (1 << 20));
+                    };
+                    using X = Comp<0>;
+                    using Y = Comp<1>;
+                    using Z = Comp<2>;
+                    constexpr int ND = KIND == DEO_VC_CURL ? 6 : 3;
+                    double d[ND] = {};  // curl: the terms of x1, x2, x3 in order, without their signs
+                    auto all = [&](auto D) {
+                        if constexpr (KIND == DEO_VC_CURL) {
+                            d[0] = D(Z{}, Y{}), d[1] = D(Y{}, Z{}), d[2] = D(Z{}, X{});
+                            d[3] = D(X{}, Z{}), d[4] = D(Y{}, X{}), d[5] = D(X{}, Y{});
+                        } else if constexpr (KIND == DEO_VC_DIVERGENCE) {
+                            d[0] = D(X{}, X{}), d[1] = D(Y{}, Y{}), d[2] = D(Z{}, Z{});
+                        } else {
+                            d[0] = D(X{}, X{}), d[1] = D(X{}, Y{}), d[2] = D(X{}, Z{});
+                        }
+                    };
+                    if (own_exp) {
+                        all(own);
+                        if (__popc(__ballot_sync(0xffffffffu, !ok)) > 8) f64 = 33;
+                    }
+                    f64 = max(f64 - 1, 0);
+                    if (!ok) all(ref);
+                    if (!on) continue;
+                    if constexpr (KIND == DEO_VC_GRADIENT) {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) o[c * V.ovol] = OW ? zero_fix(d[c]) : o[c * V.ovol] + d[c];
+                    } else if constexpr (KIND == DEO_VC_DIVERGENCE) {
+                        *o = ((OW ? zero_fix(d[0]) : *o + d[0]) + d[1]) + d[2];
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            const double f = c == 1 ? -d[2] : d[2 * c], g = c == 1 ? d[3] : -d[2 * c + 1];
+                            o[c * V.ovol] = (OW ? zero_fix(f) : o[c * V.ovol] + f) + g;
+                        }
+                    }
+                }
+            };
+            auto in_use = [&](auto cc, int q) { return C::has(decltype(cc)::value, 2) || q >= 2 * MID; };
+            each([&](auto cc) {
+                if (in_use(cc, p))
+                    for (int b = min(C::has(decltype(cc)::value, 2) ? 2 * MID : 0, p); b >= 0; --b) {
+                        load(cc, p - b);
+                        keep(cc, b);
+                    }
+                if (p + 1 < npl && in_use(cc, p + 1)) load(cc, p + 1);
+            });
+            while (true) {
+                __syncthreads();
+                if (p >= 2 * MID) own_plane();
+                if (++p == npl) break;
+                r6 = r6 == NK ? 0 : r6 + 1;
+                each([&](auto cc) {
+                    if (in_use(cc, p)) keep(cc, 0);
+                    if (p + 1 < npl && in_use(cc, p + 1)) load(cc, p + 1);
+                });
             }
         }
         // the queues, shared out over the CTA
