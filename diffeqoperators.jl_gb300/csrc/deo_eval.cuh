@@ -345,7 +345,10 @@ __device__ __forceinline__ T straight(const T* w, int64_t ws, const T* __restric
 // 15.4 / 15.9 and 13.8 / 14.5).  2048^2 at 5 taps, general / straight, apply and
 // transposed: uniform Float64 97 -> 95 and 90 -> 86 us, Float32 49 -> 32 and 52 -> 35;
 // graded Float64 107 -> 89 and 114 -> 90, Float32 78 -> 36 and 99 -> 40.
-template <typename T, bool ADJ, bool LBC>
+// PLAIN (k_apply): Float64 bands of 9 taps and more stay in the general loop, which keeps
+// the FP64 pipe as busy there (2^22 points, order 8, 78.5 us against 82.6 straight; the
+// batched kernels lose by it, 256 mixed instances 468 -> 497).
+template <typename T, bool ADJ, bool LBC, bool PLAIN>
 __device__ __forceinline__ T term_at(const TermDev& t, const T* __restrict__ u, int64_t idx, int i) {
     const int64_t s = t.stride;
     if constexpr (ADJ) {
@@ -364,6 +367,7 @@ __device__ __forceinline__ T term_at(const TermDev& t, const T* __restrict__ u, 
             if (t.s_rows)
                 return straight<T, false, true, false>(reinterpret_cast<const T*>(t.tab[0].W) + (i + t.s_e0[0]),
                                                        t.tab[0].nexp, x, s, T(1), t.s_nk[0]);
+            if (PLAIN && sizeof(T) == 8 && t.s_nk[0] >= 9) return eval_term<T, LBC>(t, u, idx, i);
             return straight<T, false, false, false>(reinterpret_cast<const T*>(t.tab[0].wband), 0, x, s, T(1), t.s_nk[0]);
         }
         const T c = __ldg(reinterpret_cast<const T*>(t.field) + idx + t.s_cidx * s);
@@ -382,7 +386,7 @@ __device__ __forceinline__ T term_at(const TermDev& t, const T* __restrict__ u, 
     }
 }
 
-template <typename T, bool ADJ, bool LBC = false>
+template <typename T, bool ADJ, bool LBC = false, bool PLAIN = false>
 __device__ __forceinline__ T eval_point(const PlanDev& P, const T* __restrict__ u, int64_t idx) {
     if (!ADJ && P.star.n) {  // the merged star at points whose rows read no ghost along any axis
         bool in = true;
@@ -399,7 +403,7 @@ __device__ __forceinline__ T eval_point(const PlanDev& P, const T* __restrict__ 
     auto term = [&](int tt) {
         const TermDev& t = P.t[tt];
         const int i = term_row(P, t, idx);
-        return term_at<T, ADJ, LBC>(t, u, idx, i);
+        return term_at<T, ADJ, LBC, PLAIN>(t, u, idx, i);
     };
     T acc = term(0);  // the first term as is, then the others added left to right
     for (int tt = 1; tt < P.nterms; ++tt) acc = acc + term(tt);

@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256, !ADJ && !LBC ? 8 : 0)
     k_apply(const __grid_constant__ PlanDev P, const T* __restrict__ u, T* __restrict__ du, int overwrite) {
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= P.total) return;
-    const T r = eval_point<T, ADJ, LBC>(P, u, idx);
+    const T r = eval_point<T, ADJ, LBC, true>(P, u, idx);
     du[idx] = overwrite ? r : r + du[idx];
 }
 
