@@ -2512,17 +2512,17 @@ extern "C" deo_status deo_vector_calculus_plan(int kind, int ndims, const deo_op
             CUDA_TRY(V->claims.init(kSchedSlots), "cudaMalloc(claim counters)");
             CUDA_TRY((cudaError_t)deo_k_vector_chunk(&D, &V->bfp.zc), "marching kernel");
         }
-        // k_vc_fx from here on (units of 64 x 8 columns and their queues want a full chip):
-        // gradient, order 2 / 4, k_vc against k_vc_fx: 80^3 16 / 23 against 17 / 33 us, 100^3
-        // 31 / 45 against 22 / 38; curl 128^3 100 / 141 against 87 / 146, 160^3 187 / 270
-        // against 184 / 249; divergence 160^3 99 / 141 against 124 / 138, 200^3 207 / 299
-        // against 215 / 260, 256^3 385 / 556 against 346 / 433
-        // (order 6: gradient 256^3 724 against 391, divergence 192^3 316 against 251, but curl
-        // 614 against 812: never)
-        V->march_min = kind == DEO_VC_GRADIENT                     ? 1000000
-                       : kind == DEO_VC_DIVERGENCE && bnk == 3     ? 16000000
-                       : kind == DEO_VC_CURL && bnk >= 7           ? INT64_MAX
-                                                                   : 4000000;
+        // k_vc_fx from here on (units of 64 x 8 columns and their queues want a full chip; smooth
+        // fields, order 2 / 4 / 6, k_vc against k_vc_fx): gradient 80^3 23 / 29 / 35 against 23 /
+        // 52 / 70 us, 100^3 38 / 50 / 64 against 29 / 48 / 70, 128^3 56 / 76 / 99 against 38 / 64 /
+        // 85; divergence 160^3 103 / 146 / 187 against 130 / 148 / 179, 200^3 212 / 304 / 396 against
+        // 218 / 253 / 320, 256^3 388 / 560 / 730 against 337 / 414 / 478; curl 128^3 103 / 146 / 189
+        // against 99 / 156 / 389, 160^3 191 / 273 / 359 against 183 / 250 / 728, 200^3 404 / 586 / 773
+        // against 308 / 461 / 1311 (order 6: never).
+        const bool six = bnk >= 7;
+        if (kind == DEO_VC_GRADIENT) V->march_min = six ? 2000000 : 1000000;
+        else if (kind == DEO_VC_DIVERGENCE) V->march_min = bnk == 3 ? 16000000 : (six ? 4000000 : 5000000);
+        else V->march_min = six ? INT64_MAX : 4000000;
     }
     V->dtype = dtype;
     V->ncomp_in = kind == DEO_VC_GRADIENT ? 1 : (kind == DEO_VC_CURL ? 3 : ndims);

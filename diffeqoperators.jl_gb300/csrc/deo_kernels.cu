@@ -223,9 +223,8 @@ extern "C" int deo_k_scale(void* x, int64_t n, int dtype, double f, void* stream
 // log2 of the parts per work item: the persistent grid balances to within one part, so a
 // list with few items is claimed in parts until there are 8 for each resident
 // CTA, of 256 points (one per thread) at the least for the default 8192-point
-// items.  One 768 x 500 Float64 state (47 items) then runs on every SM instead
-// of 47: 97 -> 31 us per Runge-Kutta stage; 256 mixed instances (1100 items)
-// forward + transposed 705 -> 565 us (456 with the straight loops of deo_eval.cuh).
+// items.  256 mixed instances (1100 items), forward + transposed 705 -> 565 us (456 with
+// the straight loops of deo_eval.cuh).
 static int split_for(int64_t n_items, int64_t ctas) {
     int lsplit = 0;
     while (lsplit < 5 && (n_items << lsplit) < 8 * ctas) ++lsplit;

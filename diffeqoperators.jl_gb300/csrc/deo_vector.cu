@@ -2,13 +2,15 @@
 // (vector_calculus_operators.jl, vector_calculus_convolutions.jl) and the
 // pointwise vector algebra (vector_algebraic_operations.jl).
 //
-// One thread per output point.  Every derivative is one row of an axis
+// Every derivative is one row of an axis
 // operator's row table over the padded input (ghosts are the input's own
 // first/last planes, bc_kind 2), so boundary rows, non-uniform stencils and
 // coefficient vectors follow the same tables as the stencil-apply path; rows
 // of a uniform operator's interior band take an unrolled loop with the same
 // fused multiply-adds in the same order.  The reference's per-point additions
-// into the output are replayed in its order (see VcDev).
+// into the output are replayed in its order (see VcDev).  Three kernels: one thread per
+// output point (k_vc), per column (k_vc_march), and, for large Float64 arrays with a uniform
+// band, block fixed point on tiles (k_vc_fx).
 #include <cuda_runtime.h>
 #include <limits.h>
 #include <stdint.h>
