@@ -30,12 +30,15 @@
 // three so and one in FP64, so that both pipes work; points that fail there too (far taps of
 // a small weight alone) are evaluated in FP64 at once.  256^3, a Gaussian of width 0.1 / 0.05
 // / 0.02 of the box, us: the per-point kernels before this one / as it was without this / now:
-// order 2 206 / 206 / 208 -> 291 / 518 / 512 -> 200 / 211 / 233; order 4 281 / 280 / 292 ->
-// 508 / 842 / 770 -> 264 / 293 / 333; order 6 610 / 610 / 676 -> 828 / 1236 / 1050 -> 448 /
-// 476 / 831; three bands (256 x 240 x 200), order 4, 506 / 506 / 507 -> 461 / 708 / 622 -> 268 /
-// 293 / 506.  The counting costs 1-2 % of a smooth field's time.  Evaluating the small units
-// inside the plane loop cost every field 40 % (registers); all groups on own exponents 305 at
-// width 0.05, order 4, half of them in FP64 361; limbs per tap, not per sum, 334.
+// order 2 206 / 206 / 208 -> 291 / 518 / 512 -> 180 / 192 / 211; order 4 281 / 280 / 292 ->
+// 508 / 842 / 770 -> 269 / 293 / 332; order 6 610 / 610 / 676 -> 828 / 1236 / 1050 -> 445 /
+// 497 / 843; three bands (256 x 240 x 200), order 4, 506 / 506 / 507 -> 461 / 708 / 622 -> 262 /
+// 268 / 530.  The counting costs 2-3 % of a smooth field's time (order 4: 188 -> 194).  Evaluating
+// the small units inside the plane loop cost every field 40 % (registers); all groups on own exponents 305 at
+// width 0.05, order 4, half of them in FP64 361; limbs per tap, not per sum, 334; counted by
+// atomics beside the largest key the kernel spilled (order 4 smooth 5-20 % more).  Positions
+// outside the array are not counted: the copies of the edge filled half a narrow tile
+// (73 x 93 x 221 74 -> 57 us).  Five CTAs an SM at order 2 with one band: width 0.05 211 -> 192.
 //
 // What bounds it (256^3, d2 a4, smooth field; start: the per-point fixed point,
 // 270 us beside its shell): 164 us for the interior, 139 us of them without the 2.8 %
@@ -103,7 +106,7 @@ __device__ __forceinline__ double ref_point(const UniPlan& U, const double* __re
 }
 
 template <int H, bool SH, bool OW, int TYT, int RY>
-__global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __grid_constant__ UniPlan U,
+__global__ void __launch_bounds__(32 * TYT, H == 1 && SH ? 5 : 4) k_lap_fx(const __grid_constant__ UniPlan U,
                                                              const __grid_constant__ BfpMarch B, const LapGrid g,
                                                              const double* __restrict__ u, double* __restrict__ du, int pairs) {
     using C = Cfg<H, TYT, RY>;
@@ -166,6 +169,8 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
             for (int j = 0; j < C::NLD; ++j) raw[j] = __ldg(reinterpret_cast<const double*>(s + off[j]));
         };
         unsigned probe = 0x7fffffffu;  // the key of this thread's value in the tile's middle rows, a plane ago
+        const int pr = (tid + C::NLD / 2 * C::NTHR) / C::BX, pcol = x0 + tid + C::NLD / 2 * C::NTHR - pr * C::BX - C::HP;
+        const int gap = pcol < 0 || pcol >= nx || y0 + pr - H >= ny ? 4096 : B.limit.gap;  // (none outside the array)
         bool small = false;            // that is too small for the block's exponent
         // the loaded plane on exponent E into a slot; its largest key
         auto put = [&](Limbs* w, int E) {
@@ -175,7 +180,7 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                 const unsigned key = bfp_key(raw[j]);
                 mx = max(mx, key);
                 if (j == C::NLD / 2) {
-                    small = probe < (unsigned)(max(E - B.limit.gap, 1) << 20);
+                    small = probe < (unsigned)(max(E - gap, 0) << 20);
                     probe = key;
                 }
                 if (j + 1 < C::NLD || tid + j * C::NTHR < C::PLANE) w[tid + j * C::NTHR] = bfp_convert(raw[j], key, E);
@@ -198,12 +203,12 @@ __global__ void __launch_bounds__(32 * TYT, 512 / (32 * TYT)) k_lap_fx(const __g
                 if (tx == 0) atomicMax(&s_max[p & 15], mx);
                 if (tid == 0) s_max[(p + 2) & 15] = 0;
             }
-            const int nsmall = __syncthreads_count(small);
+            crowd += __syncthreads_count(small) - crowd / 4;
             const unsigned top = s_max[p & 15];
             const int ep = (int)(top >> 20);
             zeros = top == 0 ? zeros + 1 : 0;
             low = ep < E ? low + 1 : 0;
-            crowd = top == 0 ? 0 : nsmall + crowd - crowd / 4;
+            if (top == 0) crowd = 0;
             if (crowd > C::NTHR * 5 / 4) break;
             if (ep > E || low > NQ + 2) {
                 // a new exponent: the planes in use (this one included) again

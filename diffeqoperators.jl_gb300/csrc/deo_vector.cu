@@ -391,6 +391,7 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
             return ring + C::base(c) + i * C::plane(c);
         };
         unsigned probe[NC];  // keys of a value in the tile's middle rows, a plane ago
+        unsigned skip = 0;   // outside the array (bit c)
         bool small = false;  // one of them is too small for its block's exponent
         auto put = [&](auto cc, int p, int back, int E) {
             constexpr int c = decltype(cc)::value;
@@ -401,7 +402,7 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
                 const unsigned key = bfp_key(raw[c][j]);
                 mx = max(mx, key);
                 if (j == C::nld(c) / 2) {
-                    small |= E > 64 && probe[c] < (unsigned)(max(E - B.gap, 1) << 20);  // (64: zeros)
+                    small |= E > 64 && !((skip >> c) & 1u) && probe[c] < (unsigned)(max(E - B.gap, 1) << 20);  // (64: zeros)
                     probe[c] = key;
                 }
                 if (j + 1 < C::nld(c) || tid + j * C::NTHR < C::plane(c))
@@ -427,8 +428,11 @@ __global__ void __launch_bounds__(128, KIND == DEO_VC_GRADIENT ? 4 : 3)
 #pragma unroll
             for (int c = 0; c < NC; ++c) s_max[c][tid] = 0;
         each([&](auto cc) {
+            constexpr int c = decltype(cc)::value, BX = C::bx(c);
             offsets(cc);
-            if constexpr (C::has(decltype(cc)::value, 2)) load(cc, 0);
+            const int q = tid + C::nld(c) / 2 * C::NTHR, r = q / BX, x = x0 + (q - r * BX) - (C::has(c, 0) ? C::PL : 0);
+            if (x < 0 || x >= px || y0 + r - (C::has(c, 1) ? C::LH : 0) >= py) skip |= 1u << c;
+            if constexpr (C::has(c, 2)) load(cc, 0);
         });
         __syncthreads();
         int E[NC], low[NC], zeros[NC];
